@@ -1045,6 +1045,7 @@ static SceneDev scene_view(SceneSlot &S, const Scene *scene) {
     d.n_emissive = S.n_emissive;
     d.occluders = P<u32t>(S.occluders);
     d.n_occluders = S.n_occluders;
+    d.neg_zero = -0.0f;
     return d;
 }
 
@@ -1204,8 +1205,7 @@ int st_render_ex(st_ctx *ctx, int slot, const Scene *scene, const Viewport *view
             cudaStream_t ts = ctx->strip_trace[k];
             ST_CUDA(cudaStreamWaitEvent(ts, fork, 0));
             launch_trace(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), dev_float, dev_ids, P<unsigned>(ctx->status),
-                         P<unsigned long long>(ctx->counters), o->count_work != 0, ts, gx0 / 8, (gx1 - gx0 + 7) / 8,
-                         want_float);
+                         P<unsigned long long>(ctx->counters), o->count_work != 0, ts, gx0 / 8, (gx1 - gx0 + 7) / 8);
             ST_CUDA(cudaGetLastError());
             ST_CUDA(cudaEventRecord(done[k], ts));
         }

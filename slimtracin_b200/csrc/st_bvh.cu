@@ -598,9 +598,9 @@ __global__ void make_pairs_kernel(const BVHNode *nodes, u32t node_count, NodePai
     if (2 + 2 * k >= node_count) return;
     const BVHNode L = nodes[1 + 2 * k], R = nodes[2 + 2 * k];
     NodePair p;
-    p.a = make_float4(L.aabb.min.x, L.aabb.min.y, L.aabb.min.z, L.aabb.max.x);
-    p.b = make_float4(L.aabb.max.y, L.aabb.max.z, R.aabb.min.x, R.aabb.min.y);
-    p.c = make_float4(R.aabb.min.z, R.aabb.max.x, R.aabb.max.y, R.aabb.max.z);
+    p.a = make_float4(L.aabb.min.x, L.aabb.min.y, L.aabb.max.x, L.aabb.max.y);
+    p.b = make_float4(R.aabb.min.x, R.aabb.min.y, R.aabb.max.x, R.aabb.max.y);
+    p.c = make_float4(L.aabb.min.z, L.aabb.max.z, R.aabb.min.z, R.aabb.max.z);
     p.d = make_uint4(L.child_count ? L.first_child_id : (L.first_child_id - 1) >> 1, L.child_count,
                      R.child_count ? R.first_child_id : (R.first_child_id - 1) >> 1, R.child_count);
     pairs[k] = p;

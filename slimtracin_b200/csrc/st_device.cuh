@@ -28,9 +28,9 @@ enum Counter { C_PRIMARY = 0, C_SHADOW, C_BOUNCE, C_AABB, C_TRI, C_PRIM, C_LEAF,
 enum Status { S_STACK_OVERFLOW = 1 };
 
 struct __align__(16) NodePair {
-    float4 a;  // lmin.x lmin.y lmin.z lmax.x
-    float4 b;  // lmax.y lmax.z rmin.x rmin.y
-    float4 c;  // rmin.z rmax.x rmax.y rmax.z
+    float4 a;  // lmin.x lmin.y lmax.x lmax.y
+    float4 b;  // rmin.x rmin.y rmax.x rmax.y
+    float4 c;  // lmin.z lmax.z rmin.z rmax.z
     uint4 d;   // l.first l.count r.first r.count   (count==0: first = child pair index)
 };
 
@@ -94,6 +94,7 @@ struct SceneDev {
     u32t n_emissive;
     const u32t *occluders;         // primitive indices of spheres and quads, increasing
     u32t n_occluders;
+    float neg_zero;                // -0.0f, a value only the host knows (mul_add2)
 };
 
 // ---- float3 math in the reference's operation order ------------------------------------------

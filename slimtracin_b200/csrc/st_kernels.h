@@ -67,16 +67,15 @@ constexpr int kAuxStreams = ST_AUX_STREAMS;
 // A grid point of a batch parked at a bounce: the persistent kernel's warp-vote compaction moves the
 // bounce rays of a warp that few lanes still trace into a queue, and drain_kernel traces them to the
 // end.  The record holds the whole path state carried across shadeSurface's bounce loop
-// (surface.h:180-239): the bounce ray, colour, throughput, the ray-cone footprints, the glow limit,
-// the bounces left and the primary hit's distance and depth.
+// (surface.h:180-239): the bounce ray, colour, throughput, the primary hit's ray-cone footprint, the
+// glow limit, the bounces left and the primary hit's distance and depth.
 struct __align__(16) ParkedRay {
     float4 origin_r;               // bounce ray origin xyz, colour r
     float4 direction_g;            // bounce ray direction xyz, colour g
     float4 throughput_b;           // throughput xyz, colour b
-    float4 carry;                  // du, dv, max_distance, closest_distance
+    float4 carry;                  // dv, max_distance, closest_distance, z
     uint4 where;                   // x, y, view in the launch group (kEmptySlot: nothing parked there),
                                    // bounces << 2 | lights_shaded << 1 | hit_found
-    float4 depth;                  // z, unused x3
 };
 constexpr u32t kEmptySlot = 0xFFFFFFFFu;
 // The queue of one launch group: `threshold` is the warp-vote limit (a warp whose lanes still tracing
@@ -104,11 +103,10 @@ int batch_blocks_per_sm(int variant);
 void launch_ray_rows(const ViewDev &v, float *dirs, cudaStream_t st);
 inline size_t ray_rows_floats(const ViewDev &v) { return (size_t)v.grid_h * ((v.grid_w + kSegment - 1) / kSegment) * 3; }
 // Block columns [bx_first, bx_first + bx_count) of the grid (8 grid points wide each; bx_count 0:
-// to the last column).  overlapped: the grid is copied to the host while it is traced (the kernel
-// then runs with fewer blocks per SM).
+// to the last column).
 void launch_trace(const SceneDev &S, const ViewDev &v, const int4 *ssb, const float *dirs, FloatPixel *out,
                   u32t *prim_ids, unsigned *status, unsigned long long *counters, bool count, cudaStream_t st,
-                  u32t bx_first = 0, u32t bx_count = 0, bool overlapped = false);
+                  u32t bx_first = 0, u32t bx_count = 0);
 // The result of a pick (layout of st_pick_result)
 struct PickDev {
     int found, object_type;

@@ -6,215 +6,31 @@
 
 namespace st {
 
-// ---- triangles and the BLAS walk: intersection/mesh.h ----------------------------------------
-// hitTriangles (mesh.h:5) over the leaf's triangles: an accepted triangle (in front of the closest
-// so far, inside by its tangent-space UV) becomes the closest; only its distance and slot are kept
-// (finalize_hit rebuilds the rest of the record from them).
-template <bool CNT, int SHS>
-__device__ bool hit_triangles(TState<CNT, SHS> &t, const SceneDev &S, u32t base, u32t slot0, u32t n, bool any_hit) {
-    const RayD &ray = t.local;
-    bool found = false;
-    for (u32t i = 0; i < n; i++) {
-        TriHot T;
-        {
-            const float4 *f = reinterpret_cast<const float4 *>(S.tri_hot + base + i);
-            asm("ld.global.nc.L1::evict_first.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(T.p.x), "=f"(T.p.y), "=f"(T.p.z), "=f"(T.p.w) : "l"(f));
-            asm("ld.global.nc.L1::evict_first.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(T.q.x), "=f"(T.q.y), "=f"(T.q.z), "=f"(T.q.w) : "l"(f + 1));
-            asm("ld.global.nc.L1::evict_first.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(T.r.x), "=f"(T.r.y), "=f"(T.r.z), "=f"(T.r.w) : "l"(f + 2));
-            asm("ld.global.nc.L1::evict_first.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(T.s.x), "=f"(T.s.y), "=f"(T.s.z), "=f"(T.s.w) : "l"(f + 3));
-        }
-        t.count(C_TRI);
-        v3 pos = V(T.p.x, T.p.y, T.p.z), nrm = V(T.p.w, T.q.x, T.q.y);
-        Hit hit;
-        if (hit_plane(pos, nrm, ray.origin, ray.direction, hit) && hit.distance < t.mesh_distance) {
-            const float m[9] = {T.q.z, T.q.w, T.r.x, T.r.y, T.r.z, T.r.w, T.s.x, T.s.y, T.s.z};
-            v3 UV = vmat3(hit.position - pos, m);
-            if (UV.x < 0 || UV.y < 0 || (UV.x + UV.y) > 1) continue;
-            t.mesh_distance = hit.distance;
-            t.mesh_tri = slot0 + i;
-            found = true;
-            if (any_hit) break;
-        }
-    }
-    return found;
-}
-
-// Cache hints: node pairs are marked to stay in L1 (evict_last; the top of every BLAS is read by
-// every ray that enters an instance), triangle records to leave first (evict_first; a triangle is
-// tested by the few neighbouring rays that reach its leaf; the 128-byte record of the winning
-// triangle is read once per hit).  Hints change no value read.  Measured on the 1080p mesh frame:
-// 2.14 against 2.18 ms, the triangle hints making the difference.
+// Records of 64 bytes are read with two 256-bit loads (a warp's lanes read unrelated records, so
+// every load instruction costs a tag look-up per lane: four 128-bit loads made the traces 1 to 3 %
+// slower).  Cache hints: node pairs are marked to stay in L1 (evict_last; the top of every BLAS is
+// read by every ray that enters an instance), triangle records to leave first (evict_first; a
+// triangle is tested by the few neighbouring rays that reach its leaf; the 128-byte record of the
+// winning triangle is read once per hit).  Hints change no value read.
 __device__ __forceinline__ NodePair load_pair(const NodePair *p) {
     NodePair r;
-    const float4 *f = reinterpret_cast<const float4 *>(p);
-    asm("ld.global.nc.L1::evict_last.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w) : "l"(f));
-    asm("ld.global.nc.L1::evict_last.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w) : "l"(f + 1));
-    asm("ld.global.nc.L1::evict_last.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.c.x), "=f"(r.c.y), "=f"(r.c.z), "=f"(r.c.w) : "l"(f + 2));
-    asm("ld.global.nc.L1::evict_last.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.d.x), "=r"(r.d.y), "=r"(r.d.z), "=r"(r.d.w) : "l"(f + 3));
+    const float *f = reinterpret_cast<const float *>(p);
+    asm("ld.global.nc.L1::evict_last.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w) : "l"(f));
+    float d[4];
+    asm("ld.global.nc.L1::evict_last.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(r.c.x), "=f"(r.c.y), "=f"(r.c.z), "=f"(r.c.w), "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "l"(f + 8));
+    r.d = make_uint4(__float_as_uint(d[0]), __float_as_uint(d[1]), __float_as_uint(d[2]), __float_as_uint(d[3]));
     return r;
 }
-
-template <bool CNT, int SHS>
-__device__ __forceinline__ bool trace_mesh(TState<CNT, SHS> &t, const SceneDev &S, const MeshDev &M, bool any_hit) {   // mesh.h:38
-    const RayD &ray = t.local;
-    float ld, rd;
-    t.count(C_MESH);
-    t.count(C_AABB);
-    if (!hit_aabb(V(M.aabb[0], M.aabb[1], M.aabb[2]), V(M.aabb[3], M.aabb[4], M.aabb[5]), ray, t.mesh_distance, ld))
-        return false;
-    // Leaves met at a node are tested (left, then right) before the walk moves on, as in the
-    // reference; they are queued so that the triangle loop has a single call site.
-    // the queue is two named slots, not an indexed array, so that it stays in registers
-    u32t q0_first = 0, q0_count = 0, q1_first = 0, q1_count = 0;
-    int leaves = 0;
-    const NodePair *pairs = S.mesh_pairs + M.pair_offset;
-    u32t pair = kNoPair;
-    if (M.root_count) { q0_first = 0; q0_count = M.triangle_count; leaves = 1; }
-    else pair = (M.root_first - 1) >> 1;
-    u32t sp = 0;
-    bool found = false;
-    for (;;) {
-        // inner nodes until this lane has leaves queued ("while-while": lanes of a warp walk nodes
-        // together and test triangles together; each lane's own order of tests is unchanged)
-        while (leaves == 0 && pair != kNoPair) {
-            const NodePair P = load_pair(pairs + pair);
-            t.count(C_AABB, 2);
-            bool hl = hit_aabb(V(P.a.x, P.a.y, P.a.z), V(P.a.w, P.b.x, P.b.y), ray, t.mesh_distance, ld);
-            bool hr = hit_aabb(V(P.b.z, P.b.w, P.c.x), V(P.c.y, P.c.z, P.c.w), ray, t.mesh_distance, rd);
-            bool lgo = hl, rgo = hr;
-            if (hl && P.d.y) { q0_first = P.d.x; q0_count = P.d.y; leaves = 1; lgo = false; }
-            if (hr && P.d.w) {
-                if (leaves) { q1_first = P.d.z; q1_count = P.d.w; }
-                else { q0_first = P.d.z; q0_count = P.d.w; }
-                leaves++;
-                rgo = false;
-            }
-            if (lgo) {
-                u32t near_pair = P.d.x, far_pair = P.d.z;
-                if (rgo) {
-                    if (!any_hit && ld > rd) { near_pair = P.d.z; far_pair = P.d.x; }
-                    if (sp >= kStack) {           // the queued leaves still run, then the walk ends
-                        t.status |= S_STACK_OVERFLOW;
-                        pair = kNoPair;
-                        continue;
-                    }
-                    t.push(true, sp++, far_pair);
-                }
-                pair = near_pair;
-            } else if (rgo) {
-                pair = P.d.z;
-            } else {
-                pair = sp ? t.at(true, --sp) : kNoPair;
-            }
-        }
-        if (!leaves) break;
-#pragma unroll 1
-        for (;;) {                       // the queued leaves in order: q0, then q1
-            if (hit_triangles(t, S, M.tri_offset + q0_first, q0_first, q0_count, any_hit)) {
-                found = true;
-                if (any_hit) return true;
-            }
-            if (--leaves == 0) break;
-            q0_first = q1_first;
-            q0_count = q1_count;
-        }
-        if (pair == kNoPair) break;
-    }
-    return found;
-}
-
-// The primitive record again, by a load the compiler cannot merge with the first one: after a BLAS
-// walk the candidate's transform is reloaded (an L1 hit) instead of being held in registers, or
-// spilled, through the walk.
-__device__ __forceinline__ PrimDev load_prim_again(const PrimDev *p) {
-    PrimDev r;
-    asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(r.pos_bits.x), "=f"(r.pos_bits.y), "=f"(r.pos_bits.z), "=f"(r.pos_bits.w) : "l"(&p->pos_bits));
-    asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(r.rot.x), "=f"(r.rot.y), "=f"(r.rot.z), "=f"(r.rot.w) : "l"(&p->rot));
-    asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(r.scale_id.x), "=f"(r.scale_id.y), "=f"(r.scale_id.z), "=f"(r.scale_id.w) : "l"(&p->scale_id));
-    asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(r.inv_scale.x), "=f"(r.inv_scale.y), "=f"(r.inv_scale.z), "=f"(r.inv_scale.w) : "l"(&p->inv_scale));
-    return r;
-}
-
-// ---- hitPrimitives intersection/primitives.h:9 ----------------------------------------------------
-// ids == nullptr: the candidates are primitives first..first+count-1 in index order.
-// The candidate loop keeps the reference's order and comparisons; a winner updates t.best (the
-// hit test's distance, the world position and its squared distance, which the next candidates and
-// the walk read), and a call that found one ends with the world distance, as hitPrimitives' final
-// step leaves it (primitives.h:105).  The rest of that final step is finalize_hit's.
-template <bool CNT, int SHS>
-__device__ __forceinline__ bool hit_primitives(TState<CNT, SHS> &t, const SceneDev &S, const RayD &ray, const u32t *ids, u32t first,
-                               u32t count, bool any_hit, const int4 *ssb, int x, int y) {
-    Best &best = t.best;
-    bool found = false;
-    for (u32t i = 0; i < count; i++) {
-        t.count(C_LEAF);
-        const u32t pid = ids ? __ldg(ids + first + i) : first + i;
-        if (ssb) {  // primary rays: IS_VISIBLE and the screen-space rect, folded into one rect per view
-            const int4 b = __ldg(ssb + pid);
-            if (x < b.x || x >= b.z || y < b.y || y >= b.w) continue;
-        }
-        const PrimDev P = S.prims[pid];
-        const unsigned flags = prim_flags(P);
-        if (any_hit && !(flags & IS_SHADOWING)) continue;
-        t.count(C_PRIM);
-        to_object(ray.origin, ray.direction, P, t.local.origin, t.local.direction);
-        t.local.origin = vsfma(t.local.direction, kTraceOffset, t.local.origin);
-        bool cur;
-        float dist = 0.0f;
-        v3 pos = splat(0.0f);
-        u32t tri = 0;
-        const unsigned type = prim_type(P);
-        if (type == PrimitiveType_Mesh) {
-            t.local.rcp = rcp(t.local.direction);
-            t.mesh_distance = best.distance == INFINITY ? INFINITY :
-                len(pos_to_object(best.position, P) - t.local.origin);
-            pre_prep(t.local);
-            const u32t mesh = __float_as_uint(P.scale_id.w);
-            cur = trace_mesh(t, S, S.meshes[mesh], any_hit);
-            if (cur) {
-                // the accepted triangle's object-space hit point, recomputed exactly as
-                // hit_triangles computed it (same triangle, same ray, same operations)
-                const MeshDev &M = S.meshes[mesh];
-                tri = t.mesh_tri;
-                const float4 tp = __ldg(reinterpret_cast<const float4 *>(S.tri_hot + M.tri_offset + tri));
-                const float4 tq = __ldg(reinterpret_cast<const float4 *>(S.tri_hot + M.tri_offset + tri) + 1);
-                Hit h;
-                hit_plane(V(tp.x, tp.y, tp.z), V(tp.w, tq.x, tq.y), t.local.origin, t.local.direction, h);
-                pos = h.position;
-                dist = t.mesh_distance;
-            }
-        } else {
-            Hit hit;
-            switch (type) {
-                case PrimitiveType_Quad: cur = hit_quad(hit, t.local.origin, t.local.direction, flags); break;
-                case PrimitiveType_Box: cur = hit_box(hit, t.local.origin, t.local.direction, flags); break;
-                case PrimitiveType_Sphere: cur = hit_sphere(hit, t.local.origin, t.local.direction, flags); break;
-                case PrimitiveType_Tetrahedron: cur = hit_tetra(hit, t.local.origin, t.local.direction, flags); break;
-                default: continue;
-            }
-            pos = hit.position;
-            dist = hit.distance;
-        }
-        if (cur) {
-            pos = pos_to_world(pos, type == PrimitiveType_Mesh ? load_prim_again(S.prims + pid) : P);
-            const float dsq = sqlen(pos - ray.origin);
-            if (dsq < best.distance_squared) {
-                best.distance_squared = dsq;
-                best.distance = dist;
-                best.position = pos;
-                best.prim = pid;
-                best.tri = tri;
-                found = true;
-                if (any_hit) break;
-            }
-        }
-    }
-    if (found) best.distance = sqrtf(best.distance_squared);
-    return found;
+__device__ __forceinline__ TriHot load_tri(const TriHot *p) {
+    TriHot T;
+    const float *f = reinterpret_cast<const float *>(p);
+    asm("ld.global.nc.L1::evict_first.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(T.p.x), "=f"(T.p.y), "=f"(T.p.z), "=f"(T.p.w), "=f"(T.q.x), "=f"(T.q.y), "=f"(T.q.z), "=f"(T.q.w) : "l"(f));
+    asm("ld.global.nc.L1::evict_first.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(T.r.x), "=f"(T.r.y), "=f"(T.r.z), "=f"(T.r.w), "=f"(T.s.x), "=f"(T.s.y), "=f"(T.s.z), "=f"(T.s.w) : "l"(f + 8));
+    return T;
 }
 
 // The closest hit's full record (hitPrimitives' copy of the winner's RayHit and its final step,
@@ -224,7 +40,7 @@ __device__ __forceinline__ bool hit_primitives(TState<CNT, SHS> &t, const SceneD
 // uvs, the primitive id, the world normal, distance, cone width and area.
 template <bool CNT, int SHS>
 __device__ __forceinline__ void finalize_hit(TState<CNT, SHS> &t, const SceneDev &S, const RayD &ray, float cone_angle) {
-    Hit &closest = t.closest;
+    Hit closest = {};       // every field is written below: the last hit's record is not live through a walk
     const u32t hid = t.best.prim;
     const PrimDev HP = S.prims[hid];
     const unsigned flags = prim_flags(HP), type = prim_type(HP);
@@ -284,78 +100,225 @@ __device__ __forceinline__ void finalize_hit(TState<CNT, SHS> &t, const SceneDev
     closest.cone_width = 2.0f * cone_angle * closest.distance;
     v3 rs = qrot(V(HP.scale_id.x, HP.scale_id.y, HP.scale_id.z), prim_rot(HP));
     closest.area *= dot(one_minus(closest.normal), rs);
+    t.closest = closest;
 }
 
-// ---- traceScene shaders/trace.h:8 (TLAS walk); with ssb != null it also serves primary rays ----
-// The primitive loop, the BLAS walk and the triangle loop each have one call site here, so every
-// inlined copy of the walk carries one copy of them (the instruction footprint of the megakernel).
-// all_prims: test every primitive in leaf-id order without the root box (the primary-ray path of
-// scenes with few primitives, raytracer.h:100).
+// ---- traceScene shaders/trace.h:8, hitPrimitives primitives.h:9 and traceMesh mesh.h:38 --------------
+// One loop walks both levels.  A lane is either in the TLAS or, between enter_mesh and leave_mesh, in
+// the BLAS of one instance; both kinds of node are the same step on the same registers (node array,
+// reciprocal direction, scaled origin, limit), so that lanes of a warp that are in different
+// instances, or some in the TLAS, step together instead of waiting for one another's BLAS walk.  What
+// the TLAS level needs after the instance (its leaf queue, its next pair, its ray) is kept in the
+// stack's frame meanwhile.  (With the BLAS walk nested in the candidate loop, as in the reference, a
+// warp waited at every candidate for the longest BLAS walk among its lanes, and the outer walk's
+// state was spilled around the inner one: 1080p mesh frames 3.28-4.07 ms against 2.91-3.74, the
+// moving scene 1.32-1.57 against 0.92-1.09.  Leaving the node loop early by a warp vote once half
+// or a quarter of the lanes wait cost more in votes than it saved; keeping each pending pair's entry
+// distance on the stack to drop those beyond the closest hit saved as many steps as the wider stack
+// cost.)  Each lane's own sequence of tests is the reference's:
+// the leaves met at a node (left, then right) are tested before the walk moves on, the nearer child
+// is entered first, and candidates are tested in leaf order.
+// with ssb != null it serves primary rays (the screen-space cull); all_prims: every primitive in
+// leaf-id order without the root box (the primary-ray path of scenes with few primitives,
+// raytracer.h:100, and picking).
+// A winner updates t.best: the world distance (as hitPrimitives' final step leaves it,
+// primitives.h:105), its square, the world position and which primitive and triangle it is; the rest
+// of hitPrimitives' record is finalize_hit's.
 template <bool CNT, int SHS>
-__device__ __forceinline__ bool trace_scene(TState<CNT, SHS> &t, const SceneDev &S, RayD &ray, bool any_hit, const int4 *ssb,
-                                            int x, int y, bool prepped, bool all_prims) {
-    if (!prepped) {
-        ray.rcp = rcp(ray.direction);
-        pre_prep(ray);
-    }
-    float ld, rd;
-    u32t q0_first = 0, q0_count = 0, q1_first = 0, q1_count = 0;   // the leaf queue, as in trace_mesh
-    int leaves = 0;
-    u32t pair = kNoPair;
+__device__ __forceinline__ bool trace_scene(TState<CNT, SHS> &t, const SceneDev &S, const RayD &ray, bool any_hit,
+                                            const int4 *ssb, int x, int y, bool all_prims) {
+    Best &best = t.best;
+    Slabs slabs = prepare(ray.origin, ray.direction);
+    v3 lo = ray.origin, ld = ray.direction;            // the object-space ray while in a mesh
     if (!all_prims) {
         t.count(C_AABB);
-        if (!hit_aabb(V(S.tlas_root_aabb[0], S.tlas_root_aabb[1], S.tlas_root_aabb[2]),
-                      V(S.tlas_root_aabb[3], S.tlas_root_aabb[4], S.tlas_root_aabb[5]), ray, t.best.distance, ld))
-            return false;
+        if (!hit_box_slabs(S.tlas_root_aabb, slabs, best.distance)) return false;
     }
-    if (all_prims || S.tlas_root_count) { q0_first = 0; q0_count = S.n_prims; leaves = 1; }
+    const NodePair *nodes = S.tlas_pairs;
+    // the leaf queue: items [q0, q0_end) of the leaf being tested, then the q1_count items from q1
+    u32t q0 = 0, q0_end = 0, q1 = 0, q1_count = 0, pair = kNoPair;
+    if (all_prims || S.tlas_root_count) q0_end = S.n_prims;
     else pair = (S.tlas_root_first - 1) >> 1;
-    u32t sp = 0;
-    bool found = false;
+    u32t sp = 0, base = 0;                             // base: the stack's first entry of this level
+    float limit = best.distance;                       // the walk's closest hit at this level
+    bool in_mesh = false, found = false;
+    u32t tri_base = 0;
     for (;;) {
-        while (leaves == 0 && pair != kNoPair) {      // inner nodes until leaves are queued
-            const NodePair P = load_pair(S.tlas_pairs + pair);
+        // inner nodes until this lane has leaves queued ("while-while": lanes of a warp walk nodes
+        // together and test leaves together)
+        while (q0 == q0_end && pair != kNoPair) {
+            const NodePair P = load_pair(nodes + pair);
             t.count(C_AABB, 2);
-            bool hl = hit_aabb(V(P.a.x, P.a.y, P.a.z), V(P.a.w, P.b.x, P.b.y), ray, t.best.distance, ld);
-            bool hr = hit_aabb(V(P.b.z, P.b.w, P.c.x), V(P.c.y, P.c.z, P.c.w), ray, t.best.distance, rd);
-            bool lgo = hl, rgo = hr;
-            if (hl && P.d.y) { q0_first = P.d.x; q0_count = P.d.y; leaves = 1; lgo = false; }
-            if (hr && P.d.w) {
-                if (leaves) { q1_first = P.d.z; q1_count = P.d.w; }
-                else { q0_first = P.d.z; q0_count = P.d.w; }
-                leaves++;
+            float ldist, rdist;
+            bool lgo, rgo;
+            hit_pair(P, slabs, S.neg_zero, limit, lgo, rgo, ldist, rdist);
+            if (lgo && P.d.y) { q0 = P.d.x; q0_end = P.d.x + P.d.y; lgo = false; }
+            if (rgo && P.d.w) {
+                if (q0 != q0_end) { q1 = P.d.z; q1_count = P.d.w; }
+                else { q0 = P.d.z; q0_end = P.d.z + P.d.w; }
                 rgo = false;
             }
-            if (lgo) {
-                u32t near_pair = P.d.x, far_pair = P.d.z;
-                if (rgo) {
-                    if (!any_hit && ld > rd) { near_pair = P.d.z; far_pair = P.d.x; }
-                    if (sp >= kStack) {           // the queued leaves still run, then the walk ends
-                        t.status |= S_STACK_OVERFLOW;
-                        pair = kNoPair;
-                        continue;
-                    }
-                    t.push(false, sp++, far_pair);
+            if (lgo && rgo) {
+                const bool swap = !any_hit && ldist > rdist;
+                if (sp - base >= (u32t)kStack) {       // the queued leaves still run, then the level ends
+                    t.status |= S_STACK_OVERFLOW;
+                    pair = kNoPair;
+                    sp = base;
+                    continue;
                 }
-                pair = near_pair;
-            } else if (rgo) {
-                pair = P.d.z;
+                t.push(sp++, swap ? P.d.x : P.d.z);
+                pair = swap ? P.d.z : P.d.x;
+            } else if (lgo | rgo) {
+                pair = lgo ? P.d.x : P.d.z;
             } else {
-                pair = sp ? t.at(false, --sp) : kNoPair;
+                pair = sp != base ? t.at(--sp) : kNoPair;
             }
         }
-        if (!leaves) break;
-#pragma unroll 1
-        for (;;) {
-            if (hit_primitives(t, S, ray, S.tlas_leaf_ids, q0_first, q0_count, any_hit, ssb, x, y)) {
-                found = true;
-                if (any_hit) return true;
+        bool leave = false;
+        if (in_mesh) {
+            // hitTriangles (mesh.h:5) over the queued leaves: an accepted triangle (in front of the
+            // closest so far, inside by its tangent-space UV) becomes the closest
+            leave = q0 == q0_end;
+            while (q0 != q0_end) {
+                const TriHot T = load_tri(S.tri_hot + tri_base + q0);
+                t.count(C_TRI);
+                const v3 pos = V(T.p.x, T.p.y, T.p.z), nrm = V(T.p.w, T.q.x, T.q.y);
+                Hit hit;
+                if (hit_plane(pos, nrm, lo, ld, hit) && hit.distance < limit) {
+                    const float m[9] = {T.q.z, T.q.w, T.r.x, T.r.y, T.r.z, T.r.w, T.s.x, T.s.y, T.s.z};
+                    const v3 UV = vmat3(hit.position - pos, m);
+                    if (!(UV.x < 0 || UV.y < 0 || (UV.x + UV.y) > 1)) {
+                        limit = hit.distance;
+                        t.mesh_tri = q0;
+                        if (any_hit) { leave = true; break; }
+                    }
+                }
+                if (++q0 == q0_end && q1_count) {
+                    q0 = q1;
+                    q0_end = q1 + q1_count;
+                    q1_count = 0;
+                }
             }
-            if (--leaves == 0) break;
-            q0_first = q1_first;
-            q0_count = q1_count;
         }
-        if (pair == kNoPair) break;
+        if (in_mesh) {
+            if (!leave) continue;
+            // leave the instance: its ray's hit, if any, is a candidate (hitPrimitives after traceMesh)
+            sp = base;
+            const u32t pid = t.at(sp - 1), tri = t.mesh_tri;
+            in_mesh = false;
+            if (tri != kNoTriangle) {
+                // the accepted triangle's object-space hit point, recomputed exactly as it was
+                // computed above (same triangle, same ray, same operations)
+                const PrimDev Pm = S.prims[pid];
+                const float4 tp = __ldg(reinterpret_cast<const float4 *>(S.tri_hot + tri_base + tri));
+                const float4 tq = __ldg(reinterpret_cast<const float4 *>(S.tri_hot + tri_base + tri) + 1);
+                Hit h;
+                hit_plane(V(tp.x, tp.y, tp.z), V(tp.w, tq.x, tq.y), lo, ld, h);
+                const v3 pos = pos_to_world(h.position, Pm);
+                const float dsq = sqlen(pos - ray.origin);
+                if (dsq < best.distance_squared) {
+                    best.distance_squared = dsq;
+                    best.distance = sqrtf(dsq);
+                    best.position = pos;
+                    best.prim = pid;
+                    best.tri = tri;
+                    found = true;
+                    if (any_hit) return true;
+                }
+            }
+            pair = t.at(sp - 2);
+            q0 = t.at(sp - 3);
+            q0_end = t.at(sp - 4);
+            q1 = t.at(sp - 5);
+            q1_count = t.at(sp - 6);
+            sp -= kFrame;
+            base = 0;
+            nodes = S.tlas_pairs;
+            limit = best.distance;
+            slabs = prepare(ray.origin, ray.direction);
+            if (q0 == q0_end && q1_count) {
+                q0 = q1;
+                q0_end = q1 + q1_count;
+                q1_count = 0;
+            }
+        }
+        // candidates of the queued TLAS leaves, up to the next instance whose BLAS is to be walked
+        if (q0 == q0_end && pair == kNoPair) break;
+        while (q0 != q0_end) {
+            t.count(C_LEAF);
+            const u32t pid = __ldg(S.tlas_leaf_ids + q0);
+            q0++;
+            bool cull = false;
+            if (ssb) {      // primary rays: IS_VISIBLE and the screen-space rect, folded into one rect per view
+                const int4 b = __ldg(ssb + pid);
+                cull = x < b.x || x >= b.z || y < b.y || y >= b.w;
+            }
+            if (!cull) {
+                const PrimDev P = S.prims[pid];
+                const unsigned flags = prim_flags(P);
+                if (!any_hit || (flags & IS_SHADOWING)) {
+                    t.count(C_PRIM);
+                    to_object(ray.origin, ray.direction, P, lo, ld);
+                    lo = vsfma(ld, kTraceOffset, lo);
+                    const unsigned type = prim_type(P);
+                    if (type == PrimitiveType_Mesh) {
+                        const MeshDev &M = S.meshes[__float_as_uint(P.scale_id.w)];
+                        const Slabs ms = prepare(lo, ld);
+                        const float md = best.distance == INFINITY ? INFINITY : len(pos_to_object(best.position, P) - lo);
+                        t.count(C_MESH);
+                        t.count(C_AABB);
+                        if (hit_box_slabs(M.aabb, ms, md)) {
+                            t.push(sp, q1_count);
+                            t.push(sp + 1, q1);
+                            t.push(sp + 2, q0_end);
+                            t.push(sp + 3, q0);
+                            t.push(sp + 4, pair);
+                            t.push(sp + 5, pid);
+                            sp += kFrame;
+                            base = sp;
+                            in_mesh = true;
+                            slabs = ms;
+                            limit = md;
+                            t.mesh_tri = kNoTriangle;
+                            tri_base = M.tri_offset;
+                            nodes = S.mesh_pairs + M.pair_offset;
+                            q0 = q0_end = q1_count = 0;
+                            pair = kNoPair;
+                            if (M.root_count) q0_end = M.triangle_count;
+                            else pair = (M.root_first - 1) >> 1;
+                            break;
+                        }
+                    } else {
+                        Hit hit;
+                        bool cur = false;
+                        switch (type) {
+                            case PrimitiveType_Quad: cur = hit_quad(hit, lo, ld, flags); break;
+                            case PrimitiveType_Box: cur = hit_box(hit, lo, ld, flags); break;
+                            case PrimitiveType_Sphere: cur = hit_sphere(hit, lo, ld, flags); break;
+                            case PrimitiveType_Tetrahedron: cur = hit_tetra(hit, lo, ld, flags); break;
+                        }
+                        if (cur) {
+                            const v3 pos = pos_to_world(hit.position, P);
+                            const float dsq = sqlen(pos - ray.origin);
+                            if (dsq < best.distance_squared) {
+                                best.distance_squared = dsq;
+                                limit = best.distance = sqrtf(dsq);
+                                best.position = pos;
+                                best.prim = pid;
+                                best.tri = 0;
+                                found = true;
+                                if (any_hit) return true;
+                            }
+                        }
+                    }
+                }
+            }
+            if (q0 == q0_end && q1_count) {
+                q0 = q1;
+                q0_end = q1 + q1_count;
+                q1_count = 0;
+            }
+        }
     }
     return found;
 }
@@ -381,7 +344,7 @@ __device__ v3 shade_from_lights(TState<CNT, SHS> &t, const SceneDev &S, Shaded &
         ray.origin = s.position;
         ray.direction = s.light_direction;
         t.count(C_SHADOW);
-        if (trace_scene(t, S, ray, true, nullptr, 0, 0, false, false)) continue;       // inShadow trace.h:85
+        if (trace_scene(t, S, ray, true, nullptr, 0, 0, false)) continue;       // inShadow trace.h:85
         color = vvfma(shade_point(s, NdotL), vscale(from(light.color), li), color);
     }
     if (S.n_lights) {
@@ -418,11 +381,12 @@ __device__ bool shade_from_emissive_quads(TState<CNT, SHS> &t, const SceneDev &S
         v3 qpos = V(Q.pos_bits.x, Q.pos_bits.y, Q.pos_bits.z);
         s.light_direction = ray.direction = qpos - s.position;
         if (dot(qn, s.light_direction) >= 0) continue;
-        float ei = dot(s.normal, area_light_vector(quad, s.position, s.quad_vertices));
+        v3 quad_vertices[4];
+        float ei = dot(s.normal, area_light_vector(quad, s.position, quad_vertices));
         if (ei > 0) {
             bool skip = true;
             for (int j = 0; j < 4; j++)
-                if (dot(s.normal, s.quad_vertices[j] - s.position) >= 0) { skip = false; break; }
+                if (dot(s.normal, quad_vertices[j] - s.position) >= 0) { skip = false; break; }
             if (skip) continue;
             float shaded_light = 1;
             if (qi != s.prim_index) {
@@ -493,16 +457,14 @@ __device__ bool shade_lights(TState<CNT, SHS> &t, const SceneDev &S, v3 Ro, v3 R
 
 template <bool CNT, int SHS>
 __device__ __forceinline__ void apply_textures(TState<CNT, SHS> &t, const SceneDev &S, Shaded &s, Hit &hit, const Material &M,
-                                               float &du, float &dv, bool first) {
-    s.u = hit.u * M.uv_repeat.x;
-    s.v = hit.v * M.uv_repeat.y;
+                                               float &dv, bool first) {
+    const float u = hit.u * M.uv_repeat.x, v = hit.v * M.uv_repeat.y;
     hit.uv_area /= M.uv_repeat.x / M.uv_repeat.y;
-    float d = duv_ray_cone(hit.NdotV, hit.cone_width, hit.area, hit.uv_area);
-    du = d;
-    if (first) dv = d;              // surface.h:162 sets u and v; the bounce path (:230) only u
-    if (M.use & ALBEDO_MAP) s.albedo = sample_texture(t, S, M.texture_ids[0], s.u, s.v, du, dv);
+    const float du = duv_ray_cone(hit.NdotV, hit.cone_width, hit.area, hit.uv_area);
+    if (first) dv = du;             // surface.h:162 sets u and v; the bounce path (:230) only u
+    if (M.use & ALBEDO_MAP) s.albedo = sample_texture(t, S, M.texture_ids[0], u, v, du, dv);
     if ((M.use & NORMAL_MAP) && M.texture_count > 1) {
-        q4 rot = normal_rotation(sample_normal(t, S, M.texture_ids[1], s.u, s.v, du, dv));
+        q4 rot = normal_rotation(sample_normal(t, S, M.texture_ids[1], u, v, du, dv));
         hit.normal = qrot(hit.normal, rot);
     }
 }
@@ -623,9 +585,174 @@ __device__ __forceinline__ v3 grid_direction(const ViewDev &v, const float *seg,
     return cur;
 }
 
-// rayTrace render/raytracer.h:81 for one QCAA grid point, writing the FloatPixel the reference's
-// setPixel leaves after beginDrawing's clear (viewport.h:88): hit -> (color, 1, z), miss ->
-// (black, 0, +inf).
+// What a path carries from one trace to the next: shadeSurface's state across its bounce loop
+// (surface.h:146-239) and what rayTrace keeps of the primary hit.
+struct Path {
+    v3 color, throughput;
+    float dv;                       // the ray-cone footprint the primary hit leaves (surface.h:162)
+    float max_distance;             // the lights' glow limit
+    float closest_distance, z;      // the primary hit's distance and depth
+    u32t bounces;                   // shadeSurface's `depth`
+    bool lights_shaded, hit_found;
+};
+
+// The primary ray of grid point (x, y), and the path and walk state rayTrace starts with.
+template <bool CNT, int SHS>
+__device__ __forceinline__ void start_path(TState<CNT, SHS> &t, const ViewDev &v, const float *dirs, u32t x, u32t y,
+                                           RayD &ray) {
+    t.closest.distance = t.closest.distance_squared = INFINITY;
+    t.closest.cone_width = 0;
+    t.best.distance = t.best.distance_squared = INFINITY;
+    ray.origin = v.cam_pos;
+    ray.direction = norm(grid_direction(v, dirs, x, y));
+    t.count(C_PRIMARY);
+}
+__device__ __forceinline__ void start_path(Path &p, u32t depth) {
+    p.color = splat(0);
+    p.throughput = splat(1);
+    p.dv = p.max_distance = 0;
+    p.closest_distance = p.z = INFINITY;
+    p.bounces = depth;
+    p.lights_shaded = p.hit_found = false;
+}
+
+// The steps of rayTrace and shadeSurface (surface.h:146) from one trace to the next: what the ray
+// that was just traced found (t.best, when `found`) is shaded into the path.  True: the path goes on
+// with the bounce ray left in `ray`, its walk state reset; false: the path is done.
+template <bool CNT, int SHS>
+__device__ __forceinline__ bool shade_step(TState<CNT, SHS> &t, const SceneDev &S, const ViewDev &v, RayD &ray, Path &p,
+                                           bool primary, bool found) {
+    Hit &hit = t.closest;
+    if (found) finalize_hit(t, S, ray, primary ? v.cone_angle : 0.0f);
+    Shaded s;
+    const Material *M;
+    if (primary) {                                          // rayTrace after the hit test (raytracer.h:89)
+        p.hit_found = found;
+        p.closest_distance = found ? hit.distance : INFINITY;
+        if (!found) return false;
+        p.z = qrot(hit.position - v.cam_pos, v.cam_rot_inv).z;
+        if (v.mode != RenderMode_Beauty) {
+            switch (v.mode) {
+                case RenderMode_Depth: p.color = splat(4 / hit.distance); break;
+                case RenderMode_Normals: {
+                    const Material &NM = S.materials[hit.material_id];
+                    if (NM.texture_count > 1 && (NM.use & NORMAL_MAP)) {
+                        float u = hit.u * NM.uv_repeat.x, vv = hit.v * NM.uv_repeat.y;
+                        hit.uv_area /= NM.uv_repeat.x / NM.uv_repeat.y;
+                        float ndu = duv_ray_cone(hit.NdotV, hit.cone_width, hit.area, hit.uv_area);
+                        q4 rot = normal_rotation(sample_normal(t, S, NM.texture_ids[1], u, vv, ndu, 0.0f));
+                        hit.normal = qrot(hit.normal, rot);
+                    }
+                    p.color = V(0.5f * (hit.normal.x + 1), 0.5f * (hit.normal.y + 1), 0.5f * (hit.normal.z + 1));
+                } break;
+                case RenderMode_UVs: p.color = V(0.5f * hit.u, 0.5f * hit.v, 0.5f); break;
+            }
+            return false;
+        }
+        // shadeSurface (surface.h:146) up to its bounce loop
+        M = S.materials + hit.material_id;
+        t.count(C_SHADE);
+        if (M->is & EMISSIVE) {
+            if (!hit.from_behind) p.color = from(M->emission);
+            return false;
+        }
+        s.albedo = from(M->albedo);
+        if (M->use && M->texture_count) apply_textures(t, S, s, hit, *M, p.dv, true);
+        p.max_distance = hit.distance;
+    } else {                                                // traceRay returned (surface.h:214-239)
+        if (!found) return false;
+        t.count(C_SHADE);
+        M = S.materials + hit.material_id;
+        s.albedo = from(M->albedo);
+        if (M->use && M->texture_count) apply_textures(t, S, s, hit, *M, p.dv, false);
+        if (hit.object_type == PrimitiveType_Quad && (M->is & EMISSIVE)) {
+            p.color = hit.from_behind ? splat(0) : from(M->emission);
+            return false;
+        }
+        if (M->brdf != BRDF_CookTorrance) p.throughput = vmul(p.throughput, from(M->reflectivity));
+    }
+    s.viewing_origin = ray.origin;
+    s.viewing_direction = ray.direction;
+    s.prim_index = hit.object_id;
+    s.material = M;
+    // one iteration of shadeSurface's bounce loop
+    if (!p.bounces) return false;
+    s.position = ray.origin = hit.position;
+    s.normal = hit.from_behind ? neg(hit.normal) : hit.normal;
+    const float ior = hit.from_behind ? M->n2_over_n1 : M->n1_over_n2;
+    const bool is_ref = (M->is & REFLECTIVE) || (M->is & REFRACTIVE);
+    float NdotRd = 0;
+    s.reflected_direction = splat(0);
+    if (is_ref || M->brdf == BRDF_Phong) {
+        NdotRd = -clamp01(-dot(s.normal, s.viewing_direction));      // invDotVec3 common.h:97
+        s.reflected_direction = vsfma(s.normal, -2.0f * NdotRd, s.viewing_direction);  // reflectWithDot :101
+    }
+    v3 cur = is_ref ? splat(0) : from(S.ambient);
+    if (S.lights) cur = shade_from_lights(t, S, s, ray, cur);
+    if (S.n_emissive)
+        if (shade_from_emissive_quads(t, S, s, ray, cur)) p.max_distance = hit.distance;
+    p.color = vvfma(cur, p.throughput, p.color);
+    if (S.lights && shade_lights(t, S, s.viewing_origin, s.viewing_direction, p.max_distance, p.color))
+        p.lights_shaded = true;
+    if (!(is_ref && --p.bounces)) return false;
+    if (M->is & REFLECTIVE) ray.direction = s.reflected_direction;
+    else {                                                         // refract common.h:105
+        v3 Vv = s.viewing_direction, N = s.normal;
+        float c = ior * ior * (1 - (NdotRd * NdotRd));
+        if (c > 1) ray.direction = splat(0);
+        else {
+            Vv = vscale(Vv, ior);
+            Vv = vsfma(N, ior * -NdotRd - sqrtf(1 - c), Vv);
+            ray.direction = norm(Vv);
+        }
+        if (ray.direction.x == 0 && ray.direction.y == 0 && ray.direction.z == 0)
+            ray.direction = s.reflected_direction;
+    }
+    t.count(C_BOUNCE);
+    t.closest.distance = t.closest.distance_squared = INFINITY;           // traceRay trace.h:89
+    t.best.distance = t.best.distance_squared = INFINITY;
+    return true;
+}
+
+// The end of rayTrace for a path that is done: the last glow, the tone map, and the FloatPixel the
+// reference's setPixel leaves after beginDrawing's clear (viewport.h:88): hit -> (color, 1, z), miss
+// -> (black, 0, +inf).
+template <bool CNT, int SHS>
+__device__ __forceinline__ void finish_path(TState<CNT, SHS> &t, const SceneDev &S, const ViewDev &v, const float *dirs,
+                                            u32t x, u32t y, Path &p, FloatPixel *out) {
+    if (v.mode == RenderMode_Beauty && S.lights && !p.lights_shaded) {
+        const v3 Rd = norm(grid_direction(v, dirs, x, y));
+        if (shade_lights(t, S, v.cam_pos, Rd, p.closest_distance, p.color)) {
+            p.hit_found = true;
+            p.z = t.sphere.closest_distance;
+        }
+    }
+    v3 color = p.color;
+    float4 c01;
+    double depth;
+    if (p.hit_found) {
+        if (v.mode == RenderMode_Beauty) {
+            color.x = tone_mapped(color.x);
+            color.y = tone_mapped(color.y);
+            color.z = tone_mapped(color.z);
+        }
+        color = vscale(color, 255.0f);
+        color = vmul(color, color);
+        c01 = make_float4(color.x, color.y, color.z, 1.0f);
+        depth = (double)p.z;
+    } else {
+        c01 = make_float4(0, 0, 0, 0);
+        depth = (double)INFINITY;
+    }
+    // streaming stores: the grid is written once and read back by a copy or the resolve, so its
+    // lines go first from L2 rather than the scene's nodes (0.5 % off the 1080p mesh frame)
+    float2 *o = reinterpret_cast<float2 *>(out + (size_t)y * v.grid_w + x);
+    __stcs(o, make_float2(c01.x, c01.y));
+    __stcs(o + 1, make_float2(c01.z, c01.w));
+    __stcs(reinterpret_cast<double *>(o) + 2, depth);
+}
+
+// rayTrace render/raytracer.h:81 for one QCAA grid point.
 // park (optional): at each bounce, a warp whose lanes still tracing number fewer than
 // park->threshold parks those lanes' paths in the queue (returns false: the point is not finished,
 // nothing is written); resume (optional): a parked path, continued from its bounce ray.  A path
@@ -635,142 +762,38 @@ __device__ __forceinline__ bool trace_point(TState<CNT, SHS> &t, const SceneDev 
                                             const float *dirs, u32t x, u32t y, FloatPixel *out, u32t *prim_ids,
                                             const ParkQueue *park = nullptr,
                                             u32t view_index = 0, const ParkedRay *resume = nullptr) {
-    const size_t idx = (size_t)y * v.grid_w + x;
-    const v3 Ro = v.cam_pos, Rd = norm(grid_direction(v, dirs, x, y));
     RayD ray;
-    t.depth = v.depth;
-    t.closest.distance = t.closest.distance_squared = INFINITY;
-    t.closest.cone_width = 0;
-    t.best.distance = t.best.distance_squared = INFINITY;
-    v3 color = splat(0);
-    bool lights_shaded = false, hit_found = false;
-    float closest_distance = INFINITY, z = INFINITY;
-    Hit &hit = t.closest;
-    // shadeSurface's state (surface.h:146)
-    Shaded s;
-    const Material *M = nullptr;
-    float du = 0, dv = 0, NdotRd = 0, ior = 0, max_distance = 0;
-    v3 throughput = splat(1);
-    u32t bounces = 0;                                       // shadeSurface's `depth`
+    Path p;
     bool primary = true;
     if (resume) {                                           // a parked path, at its bounce ray
         const ParkedRay &P = *resume;
+        t.closest.distance = t.closest.distance_squared = INFINITY;
+        t.best.distance = t.best.distance_squared = INFINITY;
         ray.origin = V(P.origin_r.x, P.origin_r.y, P.origin_r.z);
         ray.direction = V(P.direction_g.x, P.direction_g.y, P.direction_g.z);
-        color = V(P.origin_r.w, P.direction_g.w, P.throughput_b.w);
-        throughput = V(P.throughput_b.x, P.throughput_b.y, P.throughput_b.z);
-        du = P.carry.x;
-        dv = P.carry.y;
-        max_distance = P.carry.z;
-        closest_distance = P.carry.w;
-        z = P.depth.x;
-        bounces = P.where.w >> 2;
-        lights_shaded = (P.where.w >> 1) & 1u;
-        hit_found = P.where.w & 1u;
+        p.color = V(P.origin_r.w, P.direction_g.w, P.throughput_b.w);
+        p.throughput = V(P.throughput_b.x, P.throughput_b.y, P.throughput_b.z);
+        p.dv = P.carry.x;
+        p.max_distance = P.carry.y;
+        p.closest_distance = P.carry.z;
+        p.z = P.carry.w;
+        p.bounces = P.where.w >> 2;
+        p.lights_shaded = (P.where.w >> 1) & 1u;
+        p.hit_found = P.where.w & 1u;
         primary = false;
     } else {
-        ray.origin = Ro;
-        ray.direction = Rd;
-        ray.rcp = rcp(ray.direction);
-        pre_prep(ray);      // only the walk reads the prepared fields; every bounce ray prepares its own
-        t.count(C_PRIMARY);
+        start_path(t, v, dirs, x, y, ray);
+        start_path(p, v.depth);
     }
     // The primary ray and every bounce ray of shadeSurface's loop share this one trace site, so the
     // kernel carries one inlined copy of the walk for both (shadow rays keep theirs).
     for (;;) {
-        const bool found = trace_scene(t, S, ray, false, primary ? ssb : nullptr, (int)x, (int)y, primary,
+        const bool found = trace_scene(t, S, ray, false, primary ? ssb : nullptr, (int)x, (int)y,
                                        primary && !v.primary_tlas);
-        if (found) finalize_hit(t, S, ray, primary ? v.cone_angle : 0.0f);
-        if (primary) {                                      // rayTrace after the hit test (raytracer.h:89)
-            primary = false;
-            hit_found = found;
-            if (prim_ids) __stcs(prim_ids + idx, found ? hit.object_id : 0xFFFFFFFFu);
-            closest_distance = found ? hit.distance : INFINITY;
-            if (!found) break;
-            z = qrot(hit.position - v.cam_pos, v.cam_rot_inv).z;
-            if (v.mode != RenderMode_Beauty) {
-                switch (v.mode) {
-                    case RenderMode_Depth: color = splat(4 / hit.distance); break;
-                    case RenderMode_Normals: {
-                        const Material &NM = S.materials[hit.material_id];
-                        if (NM.texture_count > 1 && (NM.use & NORMAL_MAP)) {
-                            float u = hit.u * NM.uv_repeat.x, vv = hit.v * NM.uv_repeat.y;
-                            hit.uv_area /= NM.uv_repeat.x / NM.uv_repeat.y;
-                            float ndu = duv_ray_cone(hit.NdotV, hit.cone_width, hit.area, hit.uv_area);
-                            q4 rot = normal_rotation(sample_normal(t, S, NM.texture_ids[1], u, vv, ndu, 0.0f));
-                            hit.normal = qrot(hit.normal, rot);
-                        }
-                        color = V(0.5f * (hit.normal.x + 1), 0.5f * (hit.normal.y + 1), 0.5f * (hit.normal.z + 1));
-                    } break;
-                    case RenderMode_UVs: color = V(0.5f * hit.u, 0.5f * hit.v, 0.5f); break;
-                }
-                break;
-            }
-            // shadeSurface (surface.h:146) up to its bounce loop
-            M = S.materials + hit.material_id;
-            t.count(C_SHADE);
-            if (M->is & EMISSIVE) {
-                if (!hit.from_behind) color = from(M->emission);
-                break;
-            }
-            s.viewing_origin = ray.origin;
-            s.viewing_direction = ray.direction;
-            s.prim_index = hit.object_id;
-            s.material = M;
-            s.albedo = from(M->albedo);
-            s.reflected_direction = splat(0);
-            if (M->use && M->texture_count) apply_textures(t, S, s, hit, *M, du, dv, true);
-            max_distance = hit.distance;
-            bounces = t.depth;
-        } else {                                            // traceRay returned (surface.h:214-239)
-            if (!found) break;
-            t.count(C_SHADE);
-            s.prim_index = hit.object_id;
-            s.material = M = S.materials + hit.material_id;
-            s.albedo = from(M->albedo);
-            if (M->use && M->texture_count) apply_textures(t, S, s, hit, *M, du, dv, false);
-            if (hit.object_type == PrimitiveType_Quad && (M->is & EMISSIVE)) {
-                color = hit.from_behind ? splat(0) : from(M->emission);
-                break;
-            }
-            if (M->brdf != BRDF_CookTorrance) throughput = vmul(throughput, from(M->reflectivity));
-            s.viewing_origin = ray.origin;
-            s.viewing_direction = ray.direction;
-        }
-        // one iteration of shadeSurface's bounce loop
-        if (!bounces) break;
-        s.position = ray.origin = hit.position;
-        s.normal = hit.from_behind ? neg(hit.normal) : hit.normal;
-        ior = hit.from_behind ? s.material->n2_over_n1 : s.material->n1_over_n2;
-        const bool is_ref = (M->is & REFLECTIVE) || (M->is & REFRACTIVE);
-        if (is_ref || M->brdf == BRDF_Phong) {
-            NdotRd = -clamp01(-dot(s.normal, s.viewing_direction));      // invDotVec3 common.h:97
-            s.reflected_direction = vsfma(s.normal, -2.0f * NdotRd, s.viewing_direction);  // reflectWithDot :101
-        }
-        v3 cur = is_ref ? splat(0) : from(S.ambient);
-        if (S.lights) cur = shade_from_lights(t, S, s, ray, cur);
-        if (S.n_emissive)
-            if (shade_from_emissive_quads(t, S, s, ray, cur)) max_distance = hit.distance;
-        color = vvfma(cur, throughput, color);
-        if (S.lights && shade_lights(t, S, s.viewing_origin, s.viewing_direction, max_distance, color))
-            lights_shaded = true;
-        if (!(is_ref && --bounces)) break;
-        if (M->is & REFLECTIVE) ray.direction = s.reflected_direction;
-        else {                                                         // refract common.h:105
-            v3 Vv = s.viewing_direction, N = s.normal;
-            float c = ior * ior * (1 - (NdotRd * NdotRd));
-            if (c > 1) ray.direction = splat(0);
-            else {
-                Vv = vscale(Vv, ior);
-                Vv = vsfma(N, ior * -NdotRd - sqrtf(1 - c), Vv);
-                ray.direction = norm(Vv);
-            }
-            if (ray.direction.x == 0 && ray.direction.y == 0 && ray.direction.z == 0)
-                ray.direction = s.reflected_direction;
-        }
-        t.count(C_BOUNCE);
-        t.closest.distance = t.closest.distance_squared = INFINITY;           // traceRay trace.h:89
-        t.best.distance = t.best.distance_squared = INFINITY;
+        if (primary && prim_ids) __stcs(prim_ids + (size_t)y * v.grid_w + x, found ? t.best.prim : 0xFFFFFFFFu);
+        const bool more = shade_step(t, S, v, ray, p, primary, found);
+        primary = false;
+        if (!more) break;
         if (park && park->threshold) {
             // warp-vote compaction: the lanes at this bounce are the warp's lanes still tracing
             const unsigned mask = __activemask();
@@ -783,12 +806,12 @@ __device__ __forceinline__ bool trace_point(TState<CNT, SHS> &t, const SceneDev 
                 const u32t slot = base + __popc(mask & ((1u << lane) - 1u));
                 if (base + n <= park->capacity) {
                     ParkedRay &P = park->rays[slot];
-                    P.origin_r = make_float4(ray.origin.x, ray.origin.y, ray.origin.z, color.x);
-                    P.direction_g = make_float4(ray.direction.x, ray.direction.y, ray.direction.z, color.y);
-                    P.throughput_b = make_float4(throughput.x, throughput.y, throughput.z, color.z);
-                    P.carry = make_float4(du, dv, max_distance, closest_distance);
-                    P.where = make_uint4(x, y, view_index, (bounces << 2) | ((u32t)lights_shaded << 1) | (u32t)hit_found);
-                    P.depth = make_float4(z, 0.0f, 0.0f, 0.0f);
+                    P.origin_r = make_float4(ray.origin.x, ray.origin.y, ray.origin.z, p.color.x);
+                    P.direction_g = make_float4(ray.direction.x, ray.direction.y, ray.direction.z, p.color.y);
+                    P.throughput_b = make_float4(p.throughput.x, p.throughput.y, p.throughput.z, p.color.z);
+                    P.carry = make_float4(p.dv, p.max_distance, p.closest_distance, p.z);
+                    P.where = make_uint4(x, y, view_index,
+                                         (p.bounces << 2) | ((u32t)p.lights_shaded << 1) | (u32t)p.hit_found);
                     return false;
                 }
                 // the queue is full: these paths go on here; slots of the refused range that lie
@@ -797,34 +820,7 @@ __device__ __forceinline__ bool trace_point(TState<CNT, SHS> &t, const SceneDev 
             }
         }
     }
-    if (v.mode == RenderMode_Beauty && S.lights && !lights_shaded) {
-        if (shade_lights(t, S, Ro, Rd, closest_distance, color)) {
-            hit_found = true;
-            z = t.sphere.closest_distance;
-        }
-    }
-    float4 c01;
-    double depth;
-    if (hit_found) {
-        if (v.mode == RenderMode_Beauty) {
-            color.x = tone_mapped(color.x);
-            color.y = tone_mapped(color.y);
-            color.z = tone_mapped(color.z);
-        }
-        color = vscale(color, 255.0f);
-        color = vmul(color, color);
-        c01 = make_float4(color.x, color.y, color.z, 1.0f);
-        depth = (double)z;
-    } else {
-        c01 = make_float4(0, 0, 0, 0);
-        depth = (double)INFINITY;
-    }
-    // streaming stores: the grid is written once and read back by a copy or the resolve, so its
-    // lines go first from L2 rather than the scene's nodes (0.5 % off the 1080p mesh frame)
-    float2 *o = reinterpret_cast<float2 *>(out + idx);
-    __stcs(o, make_float2(c01.x, c01.y));
-    __stcs(o + 1, make_float2(c01.z, c01.w));
-    __stcs(reinterpret_cast<double *>(o) + 2, depth);
+    finish_path(t, S, v, dirs, x, y, p, out);
     return true;
 }
 
@@ -841,29 +837,19 @@ __device__ __forceinline__ void flush_counters(TState<CNT, SHS> &t, unsigned *st
     }
 }
 
-// Resident 128-thread blocks per SM the register allocation must allow.  Eight (64 registers, more
-// spills) beat the compiler's own choice of 128 registers (four blocks) on the 1080p mesh frame
-// (2.38 vs 2.62 ms), and six and seven blocks (2.42, 2.40 ms) there, on the 64-view mixed batch and
-// on the served stream; 5 blocks measured 2.52 ms, 2 blocks 5.6 ms.
-// The per-frame trace kernel with device outputs runs nine blocks (56 registers): 2.101 ms against
-// 2.110 at eight and 2.176 at ten on the 1080p mesh frame.  A frame whose float grid is copied to
-// the host while it is traced runs with fewer blocks (more registers, fewer spills): its spill
-// traffic and the copies slow each other, and on the 1080p mesh frame six blocks measured 2.19 ms
-// alone but 798-803 Mrays/s end to end against 776 at eight.
+// Resident 128-thread blocks per SM the register allocation must allow: seven (72 registers).  Over
+// three seeds each of the 1080p and 1001x563 mesh scenes, the moving scene and the 16-primitive scene
+// the traces sum to 14.97 ms at seven, 15.21 at eight, 15.46 at nine, 15.30 at six, 15.68 at five:
+// fewer registers spill more, more registers leave too few warps to cover the node loads.  Frames
+// whose grid is copied to the host while they are traced and batches have the same optimum.
 #ifndef ST_TRACE_MIN_BLOCKS
-#define ST_TRACE_MIN_BLOCKS 8
-#endif
-#ifndef ST_TRACE_DEVICE_MIN_BLOCKS
-#define ST_TRACE_DEVICE_MIN_BLOCKS 9
-#endif
-#ifndef ST_TRACE_OVERLAP_MIN_BLOCKS
-#define ST_TRACE_OVERLAP_MIN_BLOCKS 6
+#define ST_TRACE_MIN_BLOCKS 7
 #endif
 #define ST_TRACE_BOUNDS __launch_bounds__(128, ST_TRACE_MIN_BLOCKS)
-template <bool CNT, int MINB>
-__global__ void __launch_bounds__(128, MINB) trace_kernel(SceneDev S, ViewDev v, const int4 *ssb, const float *dirs,
-                                                          FloatPixel *out, u32t *prim_ids, unsigned *status,
-                                                          unsigned long long *counters, u32t bx_first) {
+template <bool CNT>
+__global__ void ST_TRACE_BOUNDS trace_kernel(SceneDev S, ViewDev v, const int4 *ssb, const float *dirs, FloatPixel *out,
+                                             u32t *prim_ids, unsigned *status, unsigned long long *counters,
+                                             u32t bx_first) {
     const u32t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // A block covers 8x16 grid points: four 8x4 warp tiles stacked vertically.  Blocks are numbered
     // down the columns, starting at block column bx_first: blocks start in launch order, so this
@@ -893,9 +879,7 @@ __global__ void pick_kernel(SceneDev S, ViewDev v, const int4 *ssb, int x, int y
     RayD ray;
     ray.origin = v.cam_pos;
     ray.direction = norm(vsfma(v.pp_down, (float)y, vsfma(v.pp_right, (float)x, v.pp_start)));
-    ray.rcp = rcp(ray.direction);
-    bool found = hit_primitives(t, S, ray, S.tlas_leaf_ids, 0, S.n_prims, false, ssb, (int)(uint16_t)x,
-                                (int)(uint16_t)y);
+    bool found = trace_scene(t, S, ray, false, ssb, (int)(uint16_t)x, (int)(uint16_t)y, true);
     if (found) finalize_hit(t, S, ray, 0.0f);
     Hit &hit = t.closest;
     for (u32t i = 0; S.lights && i < S.n_lights; i++) {
@@ -1057,20 +1041,13 @@ void launch_ray_rows(const ViewDev &v, float *dirs, cudaStream_t st) {
 }
 void launch_trace(const SceneDev &S, const ViewDev &v, const int4 *ssb, const float *dirs, FloatPixel *out,
                   u32t *prim_ids, unsigned *status, unsigned long long *counters, bool count, cudaStream_t st,
-                  u32t bx_first, u32t bx_count, bool overlapped) {
+                  u32t bx_first, u32t bx_count) {
     const u32t bw = (v.grid_w + 7) / 8, bh = (v.grid_h + 15) / 16;
     if (bx_first >= bw) return;
     if (!bx_count || bx_first + bx_count > bw) bx_count = bw - bx_first;
     const dim3 grid(bh, bx_count);
-    constexpr int A = ST_TRACE_DEVICE_MIN_BLOCKS, B = ST_TRACE_OVERLAP_MIN_BLOCKS;
-    if (count && overlapped)
-        trace_kernel<true, B><<<grid, 128, 0, st>>>(S, v, ssb, dirs, out, prim_ids, status, counters, bx_first);
-    else if (count)
-        trace_kernel<true, A><<<grid, 128, 0, st>>>(S, v, ssb, dirs, out, prim_ids, status, counters, bx_first);
-    else if (overlapped)
-        trace_kernel<false, B><<<grid, 128, 0, st>>>(S, v, ssb, dirs, out, prim_ids, status, counters, bx_first);
-    else
-        trace_kernel<false, A><<<grid, 128, 0, st>>>(S, v, ssb, dirs, out, prim_ids, status, counters, bx_first);
+    if (count) trace_kernel<true><<<grid, 128, 0, st>>>(S, v, ssb, dirs, out, prim_ids, status, counters, bx_first);
+    else trace_kernel<false><<<grid, 128, 0, st>>>(S, v, ssb, dirs, out, prim_ids, status, counters, bx_first);
 }
 int launch_batch(const BatchView *views, u32t n_views, u32t total_tiles, int variant, u32t chunk, u32t grid_blocks,
                  u32t *tile_counter, unsigned *status, unsigned long long *counters, bool count, cudaStream_t st,

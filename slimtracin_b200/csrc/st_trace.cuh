@@ -29,10 +29,7 @@ struct Hit {                                        // RayHit core/types.h:185
     bool from_behind;
 };
 
-struct RayD {                                       // Ray core/types.h:180
-    v3 origin, direction, rcp, scaled_origin;
-    bool ox, oy, oz;                                // octant == 3 per axis
-};
+struct RayD { v3 origin, direction; };              // Ray core/types.h:180 (its prepared fields: Slabs)
 
 struct SphereHitD { float b, c, t_near, t_far, furthest, closest_distance; };
 
@@ -52,32 +49,31 @@ struct Best {
     u32t tri;                         // meshes: the winning triangle's slot in the mesh's leaf order
 };
 
-// SHS: entries of each traversal stack kept in shared memory (the block's stack columns, one per
-// thread, entry-major so that a warp's pushes hit distinct banks); the rest live in local memory.
-// Where the entries live changes no traversal step.
+// The walk's stack: the pending TLAS pairs (the reference's trace->scene_stack, trace.h:22), one frame
+// of kFrame words while in an instance, and the pending BLAS pairs (trace->mesh_stack, mesh.h:42).
+constexpr u32t kFrame = 6, kStackWords = 2 * kStack + kFrame;
+constexpr u32t kNoTriangle = 0xFFFFFFFFu;
+// SHS: half the stack words kept in shared memory (the block's stack columns, one per thread,
+// word-major so that a warp's pushes hit distinct banks); the rest live in local memory.
+// Where the words live changes no traversal step.
 template <bool CNT, int SHS = 0>
 struct TState {
     Hit closest;                      // the finalized closest hit, as shading reads it
     Best best;                        // the walk's view of it (above)
-    float mesh_distance;              // the BLAS walk's closest triangle so far (trace->closest_mesh_hit):
-    u32t mesh_tri;                    //   its distance along the object-space ray, and its slot
+    u32t mesh_tri;                    // the BLAS walk's closest triangle so far (trace->closest_mesh_hit): its slot
     SphereHitD sphere;
-    RayD local;
-    u32t depth;
     unsigned status;
     unsigned cnt[CNT ? C_COUNT : 1];
-    u32t scene_local[kStack - SHS];   // the TLAS walk (the reference's trace->scene_stack, trace.h:22)
-    u32t mesh_local[kStack - SHS];    // the BLAS walk nested inside it (trace->mesh_stack, mesh.h:42)
-    u32t *sh;                         // SHS > 0: this thread's column, 2 * SHS entries kTraceBlock apart
+    u32t stack[kStackWords - 2 * SHS];
+    u32t *sh;                         // SHS > 0: this thread's column, 2 * SHS words kTraceBlock apart
     __device__ __forceinline__ void count(int k, unsigned n = 1) { if (CNT) cnt[k] += n; }
-    __device__ __forceinline__ void push(bool mesh, u32t i, u32t v) {
-        if (SHS > 0 && i < (u32t)SHS) sh[((mesh ? SHS : 0) + i) * kTraceBlock] = v;
-        else if (mesh) mesh_local[i - SHS] = v;
-        else scene_local[i - SHS] = v;
+    __device__ __forceinline__ void push(u32t i, u32t v) {
+        if (SHS > 0 && i < 2u * SHS) sh[i * kTraceBlock] = v;
+        else stack[i - 2 * SHS] = v;
     }
-    __device__ __forceinline__ u32t at(bool mesh, u32t i) const {
-        if (SHS > 0 && i < (u32t)SHS) return sh[((mesh ? SHS : 0) + i) * kTraceBlock];
-        return mesh ? mesh_local[i - SHS] : scene_local[i - SHS];
+    __device__ __forceinline__ u32t at(u32t i) const {
+        if (SHS > 0 && i < 2u * SHS) return sh[i * kTraceBlock];
+        return stack[i - 2 * SHS];
     }
 };
 
@@ -100,33 +96,71 @@ __device__ __forceinline__ void parallel_axis(float dir, float org, float &rcp, 
     }
 }
 
-// prePrepRay core/init.h:536
-__device__ __forceinline__ void pre_prep(RayD &r) {
-    r.ox = signbit(r.direction.x);
-    r.oy = signbit(r.direction.y);
-    r.oz = signbit(r.direction.z);
-    r.scaled_origin.x = -r.origin.x * r.rcp.x;
-    r.scaled_origin.y = -r.origin.y * r.rcp.y;
-    r.scaled_origin.z = -r.origin.z * r.rcp.z;
-    parallel_axis(r.direction.x, r.origin.x, r.rcp.x, r.scaled_origin.x);
-    parallel_axis(r.direction.y, r.origin.y, r.rcp.y, r.scaled_origin.y);
-    parallel_axis(r.direction.z, r.origin.z, r.rcp.z, r.scaled_origin.z);
+// prePrepRay core/init.h:536: the reciprocal direction and -origin * rcp
+struct Slabs { v3 rcp, so; };
+__device__ __forceinline__ Slabs prepare(v3 org, v3 dir) {
+    Slabs r;
+    r.rcp = rcp(dir);
+    r.so.x = -org.x * r.rcp.x;
+    r.so.y = -org.y * r.rcp.y;
+    r.so.z = -org.z * r.rcp.z;
+    parallel_axis(dir.x, org.x, r.rcp.x, r.so.x);
+    parallel_axis(dir.y, org.y, r.rcp.y, r.so.y);
+    parallel_axis(dir.z, org.z, r.rcp.z, r.so.z);
+    return r;
 }
 
-// hitAABB render/AABB.h:6 (the octant offset selects max for the entry plane when negative)
-__device__ __forceinline__ bool hit_aabb(v3 bmin, v3 bmax, const RayD &r, float closest, float &dist) {
-    v3 mn = V(r.ox ? bmax.x : bmin.x, r.oy ? bmax.y : bmin.y, r.oz ? bmax.z : bmin.z);
-    v3 mx = V(r.ox ? bmin.x : bmax.x, r.oy ? bmin.y : bmax.y, r.oz ? bmin.z : bmax.z);
-    mn = vvfma(mn, r.rcp, r.scaled_origin);
-    mx = vvfma(mx, r.rcp, r.scaled_origin);
-    float a = mx.x < mx.y ? mx.x : mx.y;
-    a = a < mx.z ? a : mx.z;
-    a = a < closest ? a : closest;
-    float b = mn.x > mn.y ? mn.x : mn.y;
-    b = b > mn.z ? b : mn.z;
-    b = b > 0 ? b : 0;
-    dist = b;
-    return b <= a;
+// hitAABB render/AABB.h:6, from the six plane distances of a box: the direction's sign picks each
+// axis' entry plane, as in the reference; the axes meet in three-operand minima and maxima instead of
+// its compare chain.  The values are the same unless a distance is NaN, which takes a NaN box bound (a
+// mesh with a NaN vertex): that axis is then left out, where the chain also drops a neighbouring one
+// and visits boxes that hold no point of the ray.  A walk step is bound by its dependent instructions, not by bandwidth: with the
+// planes of a pair multiplied and added two at a time (mul_add2) it takes about 65 instructions
+// against 100; without the pairing the 4096-primitive moving scene traces in 1.08 ms instead of
+// 1.05, the mesh frames in 1 to 2 % more.
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ bool hit_slabs(float x0, float x1, float y0, float y1, float z0, float z1, v3 rcp, float closest,
+                                          float &dist) {
+    const bool nx = rcp.x < 0, ny = rcp.y < 0, nz = rcp.z < 0;
+    const float far = fminf(min3(nx ? x0 : x1, ny ? y0 : y1, nz ? z0 : z1), closest);
+    dist = fmaxf(max3(nx ? x1 : x0, ny ? y1 : y0, nz ? z1 : z0), 0.0f);
+    return dist <= far;
+}
+__device__ __forceinline__ bool hit_box_slabs(const float *b, const Slabs &r, float closest) {
+    float dist;
+    return hit_slabs(b[0] * r.rcp.x + r.so.x, b[3] * r.rcp.x + r.so.x, b[1] * r.rcp.y + r.so.y, b[4] * r.rcp.y + r.so.y,
+                     b[2] * r.rcp.z + r.so.z, b[5] * r.rcp.z + r.so.z, r.rcp, closest, dist);
+}
+// v * m + a on two floats at once, each product and sum rounded by itself.  The product is a fused
+// v * m + -0, the same value, with a -0 that the compiler does not know (SceneDev::neg_zero): a packed
+// multiply and a packed add, both .rn, were contracted into one rounding on the way to machine code,
+// which moved entry distances by an ulp and changed the work of 54 of the 1080p frame's rays.
+__device__ __forceinline__ float2 mul_add2(float2 v, float2 m, float2 a, float nz) {
+    float2 r;
+    asm("{.reg .b64 v, m, a, z;\n\tmov.b64 v, {%2, %3};\n\tmov.b64 m, {%4, %5};\n\tmov.b64 a, {%6, %7};\n\t"
+        "mov.b64 z, {%8, %8};\n\tfma.rn.f32x2 v, v, m, z;\n\tadd.rn.f32x2 v, v, a;\n\tmov.b64 {%0, %1}, v;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(v.x), "f"(v.y), "f"(m.x), "f"(m.y), "f"(a.x), "f"(a.y), "f"(nz));
+    return r;
+}
+// Both boxes of a pair.
+__device__ __forceinline__ void hit_pair(const NodePair &P, const Slabs &r, float nz, float closest, bool &lhit, bool &rhit,
+                                         float &ldist, float &rdist) {
+    const float2 mxy = make_float2(r.rcp.x, r.rcp.y), sxy = make_float2(r.so.x, r.so.y);
+    const float2 mz = make_float2(r.rcp.z, r.rcp.z), sz = make_float2(r.so.z, r.so.z);
+    const float2 l0 = mul_add2(make_float2(P.a.x, P.a.y), mxy, sxy, nz), l1 = mul_add2(make_float2(P.a.z, P.a.w), mxy, sxy, nz);
+    const float2 r0 = mul_add2(make_float2(P.b.x, P.b.y), mxy, sxy, nz), r1 = mul_add2(make_float2(P.b.z, P.b.w), mxy, sxy, nz);
+    const float2 lz = mul_add2(make_float2(P.c.x, P.c.y), mz, sz, nz), rz = mul_add2(make_float2(P.c.z, P.c.w), mz, sz, nz);
+    lhit = hit_slabs(l0.x, l1.x, l0.y, l1.y, lz.x, lz.y, r.rcp, closest, ldist);
+    rhit = hit_slabs(r0.x, r1.x, r0.y, r1.y, rz.x, rz.y, r.rcp, closest, rdist);
 }
 
 // scene/primitive.h:8-51
@@ -241,8 +275,6 @@ struct Shaded {                                                      // core/typ
     u32t prim_index;
     const Material *material;
     v3 albedo, position, normal, viewing_direction, viewing_origin, reflected_direction, light_direction;
-    v3 quad_vertices[4];
-    float u, v;
 };
 
 __device__ __forceinline__ v3 shade_classic(v3 diffuse, float NdotL, v3 spec, float sf, float exponent, float roughness) {
