@@ -768,11 +768,11 @@ int st_update_scene_bvh(st_ctx *ctx, int slot, Scene *scene, int mode) {
     return status;
 }
 
-// An LBVH30 TLAS update waits once: the build's counts, its nodes (at most 2n - 1) and its leaf order
-// come back together into page-locked staging, are checked there and, when the host scene has BVH
-// arrays, copied into them from there (the other modes wait for the build, the check and the copy
-// one after another).
-static int update_scene_lbvh(st_ctx *ctx, SceneSlot *S, Scene *scene) {
+// An LBVH30 TLAS update, and a binned-SAH one that needs no host on the way, waits once: the build's counts, its
+// nodes (at most 2n - 1) and its leaf order come back together into page-locked staging, are checked
+// there and, when the host scene has BVH arrays, copied into them from there (the other modes wait for
+// the build, the check and the copy one after another).
+static int update_scene_once(st_ctx *ctx, SceneSlot *S, Scene *scene, bool sah) {
     const u32t n = S->n_prims;
     cudaStream_t st = ctx->stream;
     if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
@@ -788,9 +788,15 @@ static int update_scene_lbvh(st_ctx *ctx, SceneSlot *S, Scene *scene) {
     BVHNode *nodes = reinterpret_cast<BVHNode *>(ctx->bvh_pinned + 64);
     u32t *ids = reinterpret_cast<u32t *>(ctx->bvh_pinned + 64 + node_bytes);
     launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, st);
-    lbvh_enqueue(ctx->lbvh, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes), P<u32t>(S->tlas_leaf_ids),
-                 counts, st);
-    ST_CUDA(cudaGetLastError());
+    if (sah) {
+        ST_TRY(reserve(ctx, ctx->sah_scratch, sah_scratch_bytes(n)));
+        ST_CUDA(sah_enqueue(ctx->lbvh.aabbs, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes),
+                            P<u32t>(S->tlas_leaf_ids), ctx->sah_scratch.ptr, counts, st));
+    } else {
+        lbvh_enqueue(ctx->lbvh, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes), P<u32t>(S->tlas_leaf_ids),
+                     counts, st);
+        ST_CUDA(cudaGetLastError());
+    }
     ST_CUDA(cudaMemcpyAsync(nodes, S->tlas_nodes.ptr, node_bytes - sizeof(BVHNode), cudaMemcpyDeviceToHost, st));
     ST_CUDA(cudaMemcpyAsync(ids, S->tlas_leaf_ids.ptr, sizeof(u32t) * n, cudaMemcpyDeviceToHost, st));
     ST_TRY(ST_CUDA_SYNC(ctx));
@@ -820,7 +826,9 @@ static int update_scene_lbvh(st_ctx *ctx, SceneSlot *S, Scene *scene) {
 static int update_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode) {
     const u32t n = S->n_prims;
     if (mode == ST_BVH_LBVH30) {
-        return update_scene_lbvh(ctx, S, scene);
+        return update_scene_once(ctx, S, scene, false);
+    } else if (mode == ST_BVH_BINNED_SAH && sah_without_wait(n, MAX_OBJS_PER_SCENE_BVH_NODE)) {
+        return update_scene_once(ctx, S, scene, true);
     } else if (mode == ST_BVH_BINNED_SAH) {
         if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
         launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, ctx->stream);

@@ -167,6 +167,11 @@ void lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32
 cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t info[2],
                       cudaStream_t st, void *scratch = nullptr, size_t scratch_bytes = 0);
 size_t sah_scratch_bytes(u32t n);
+// Whether sah_enqueue makes the build without waiting for the device on the way.
+bool sah_without_wait(u32t n, u32t max_leaf);
+// The build with sah_scratch_bytes(n) bytes of scratch; counts as lbvh_enqueue's.
+cudaError_t sah_enqueue(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, void *scratch,
+                        u32t *counts, cudaStream_t st);
 // After lbvh_build: the Morton code of every item, by item index.
 void launch_codes_by_item(const LbvhScratch &s, u32t n, u32t *out, cudaStream_t st);
 // World boxes of primitives as updateSceneBVH computes them (builder_top_down.h:370-377).

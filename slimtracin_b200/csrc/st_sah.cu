@@ -1,32 +1,48 @@
 // st_sah.cu — device binned-SAH BVH build (TLAS "binned SAH" mode, and BLAS on request).
 //
-// Breadth-first, one level per step, the same specification as the CPU oracle's orc_binned_sah:
+// The same specification as the CPU oracle's orc_binned_sah:
 //   centroid (min+max)*0.5; a node's box and centroid box are unions under the IEEE total order;
 //   per axis with centroid extent e > 0, bin = clamp((c - lo) * (32 / e)) in [0, 31];
 //   a split after bin k costs halfArea(L)*nL + halfArea(R)*nR (AABB.h:39), empty sides skipped,
 //   the lowest cost wins with ties to the lower axis then the lower k; with no candidate the range
 //   is split at its middle; the partition is stable; the split nodes of a level get child pairs in
 //   level order (pair p -> slots 1+2p, 2+2p); depth = level; height = deepest leaf.
-// Large tasks (> kSmall items) are binned by many blocks into global bins; small tasks are done by
-// one block each in shared memory.  Bin counts are integers and boxes are min/max of ordered bits,
-// so the result does not depend on the order the atomics land in.
+// Every count is an integer and every box a min/max of ordered bits, so nothing depends on the order
+// in which threads meet.
+//
+// A range is split by as many threads as it is worth: above kCap items by many blocks (two launches a
+// level), above kSub by one block in shared memory, and from there a block of its own builds it to its
+// leaves, a warp for each range of a level, the smallest ranges (most of a tree) without bins.  The
+// numbering comes last: a level's split nodes are counted from left to right (the nodes of a level lie
+// in the order of their ranges), and the nodes are written to the slots this gives.  Nothing waits for
+// the host but the splitting of ranges above kCap.
+// Bound by latency (a split is a chain of reductions, a few microseconds whatever its size), so what
+// counts is how many ranges are split at once and how few launches there are.  One launch per step
+// and level with a block for each range, and the level's totals read back by the host, took 1.42 ms of
+// a 4096-box TLAS update and 8 ms for 327,680 triangles; one block for everything up to 4096 items
+// 0.5 ms.
 #include <cstdio>
 #include "st_kernels.h"
 
 namespace st {
 
 constexpr int kBins = 32;
-constexpr int kSmall = 2048;           // items a single block partitions in shared memory
-constexpr int kChunk = 2048;           // items per block when binning / partitioning a large task
-constexpr int kBinWords = 13;          // count + box(6) + centroid box(6)
+constexpr u32t kCap = 4096;            // items one block splits in shared memory
+constexpr u32t kSub = 512;             // items a block builds to the leaves (a warp splits them in about 8 us)
+constexpr u32t kTiny = 10;             // items up to which a range is split without bins (3 axes x 10 lanes)
+constexpr int kMidThreads = 1024, kMidWarps = kMidThreads / 32;
+constexpr int kThreads = 256, kWarps = kThreads / 32;
+constexpr u32t kPer = (kSub + kThreads - 1) / kThreads;
+constexpr u32t kChunk = 2048;          // items per block when binning / partitioning a large range
+constexpr int kBinWords = 13;          // large ranges: count + box(6) + centroid box(6)
+constexpr int kSweepWords = 7;         // in shared memory: count + box(6), [axis][word][bin]
+constexpr int kWarpBins = 3 * kSweepWords * kBins;
 
-struct SahTask {
-    u32t begin, end, slot, pad;
-    unsigned box[6], cbox[6];          // ordered bits
-};
-
+// The move is opaque on purpose: as plain integer code "set the sign bit" became a float negation, which
+// does not keep a NaN's bits.
 __device__ __forceinline__ unsigned ob(float f) {
-    unsigned u = __float_as_uint(f);
+    unsigned u;
+    asm("mov.b32 %0, %1;" : "=r"(u) : "f"(f));
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ float fo(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k); }
@@ -50,118 +66,562 @@ __device__ __forceinline__ void grow6(unsigned *b, const unsigned *c) {
 __device__ __forceinline__ void atomic_grow6(unsigned *b, const unsigned *c) {
     for (int q = 0; q < 3; q++) { atomicMin(b + q, c[q]); atomicMax(b + 3 + q, c[3 + q]); }
 }
+__device__ __forceinline__ void warp_grow6(unsigned *b) {
+    for (int q = 0; q < 3; q++) {
+        b[q] = __reduce_min_sync(0xFFFFFFFFu, b[q]);
+        b[3 + q] = __reduce_max_sync(0xFFFFFFFFu, b[3 + q]);
+    }
+}
+// The axes of a range with centroid box `c`: where its bins start and how wide they are.
+struct Axes { float lo[3], scale[3]; bool valid[3]; };
+__device__ __forceinline__ Axes axes_of(const unsigned *c) {
+    Axes A;
+    for (int a = 0; a < 3; a++) {
+        const float l = fo(c[a]), e = fo(c[3 + a]) - l;
+        A.valid[a] = e > 0.0f;
+        A.lo[a] = l;
+        A.scale[a] = A.valid[a] ? (float)kBins / e : 0.0f;
+    }
+    return A;
+}
+__device__ __forceinline__ void write_node(BVHNode &o, const unsigned *b, u32t first, u32t count, u32t level) {
+    o.aabb.min.x = fo(b[0]); o.aabb.min.y = fo(b[1]); o.aabb.min.z = fo(b[2]);
+    o.aabb.max.x = fo(b[3]); o.aabb.max.y = fo(b[4]); o.aabb.max.z = fo(b[5]);
+    o.first_child_id = first;
+    o.child_count = (uint16_t)count;
+    o.depth = (uint16_t)level;
+}
 
-// ---- set-up: centroids and the root task ----------------------------------------------------
-__global__ void sah_setup_kernel(const float *aabbs, u32t n, float *cent, u32t *ids, unsigned *root) {
-    unsigned b[6], c[6];
-    empty6(b);
+// A split: after which bin of which axis (key = axis * 32 + bin, kNoSplit: at the middle), and how
+// many items go left.
+constexpr u32t kNoSplit = 0xFFFFFFFFu;
+struct Split { float cost; u32t key, nleft; };
+__device__ __forceinline__ Split better(Split a, Split b) {
+    return b.cost < a.cost || (b.cost == a.cost && b.key < a.key) ? b : a;
+}
+__device__ __forceinline__ Split warp_best(Split s) {
+    for (int off = 16; off; off >>= 1) {
+        Split o;
+        o.cost = __shfl_xor_sync(0xFFFFFFFFu, s.cost, off);
+        o.key = __shfl_xor_sync(0xFFFFFFFFu, s.key, off);
+        o.nleft = __shfl_xor_sync(0xFFFFFFFFu, s.nleft, off);
+        s = better(s, o);
+    }
+    return s;
+}
+// One axis' bins, a lane each: its box and count; the best split of the axis (all lanes agree).
+__device__ __forceinline__ Split sweep_axis(const unsigned *mine, u32t n, int axis, int lane) {
+    unsigned L[6], R[6];
+    u32t nl = n;
+    for (int q = 0; q < 6; q++) L[q] = R[q] = mine[q];
+    for (int off = 1; off < 32; off <<= 1) {
+        unsigned u[6], d[6];
+        const u32t c = __shfl_up_sync(0xFFFFFFFFu, nl, off);
+        for (int q = 0; q < 6; q++) {
+            u[q] = __shfl_up_sync(0xFFFFFFFFu, L[q], off);
+            d[q] = __shfl_down_sync(0xFFFFFFFFu, R[q], off);
+        }
+        if (lane >= off) { nl += c; grow6(L, u); }
+        if (lane + off < 32) grow6(R, d);
+    }
+    const u32t total = __shfl_sync(0xFFFFFFFFu, nl, 31), nr = total - nl;
+    for (int q = 0; q < 6; q++) R[q] = __shfl_down_sync(0xFFFFFFFFu, R[q], 1);
+    Split s{INFINITY, kNoSplit, 0};
+    if (lane < 31 && nl && nr) {
+        const float cost = half_area_bits(L) * (float)nl + half_area_bits(R) * (float)nr;
+        if (cost < INFINITY) s = Split{cost, (u32t)(axis * kBins + lane), nl};
+    }
+    return warp_best(s);
+}
+
+// ---- a range built to its leaves by one block ---------------------------------------------------
+// A range of the ids, what made it, and its first level; `source`: which of the two id buffers holds it.
+struct SahTask {
+    u32t begin, end, level, source;
+    u32t parent, side;                 // the large node it is a child of (kNoSplit: the root), and which child
+};
+// A node as a block leaves it when the numbering is not known yet.
+struct SahRecord {
+    unsigned box[6];
+    u32t first, count;                 // leaf: first item and count; inner (count 0): its split's rank in the level
+    u32t level, index;                 // level of the tree, index in the range's level
+};
+// A split range above kSub items, as the numbering needs it.
+struct LargeNode {
+    unsigned box[6];
+    u32t begin, level, parent, side;
+};
+// Counters of a build, in device memory.
+struct SahCounts {
+    u32t large[2], chunks[2];          // ranges above kCap and their chunks: this level's, the next level's
+    u32t mids, nodes, subtrees;        // ranges above kSub left to a block, large nodes so far, ranges up to kSub
+    u32t info[4];                      // -, height, pairs
+    unsigned root[6];                  // the root's centroid box
+};
+struct SubtreeShared {
+    unsigned box[6][kSub];             // the items' boxes as ordered bits, by place in the range at its start
+    unsigned bins[kWarps][kWarpBins];
+    uint16_t order[2][kSub];           // the items in their present order (two buffers, a level apart)
+    uint16_t task[2][kSub][2];         // this level's and the next level's ranges: begin, end
+    unsigned red[6];
+    u32t warp_sum[kWarps];
+};
+constexpr u32t kMidTasks = kCap / kSub;    // ranges above kSub items of one block: fewer than this
+struct MidShared {
+    unsigned box[6][kCap];
+    unsigned bins[kWarpBins];
+    uint16_t order[2][kCap];
+    SahTask task[2][kMidTasks];        // begin and end within the block's range
+    u32t tasks[2];
+    unsigned red[12];
+    Split axis_split[3];
+    u32t warp_sum[kMidWarps], child[2], self;
+};
+
+template <class Shared>
+__device__ __forceinline__ void item_bits(const Shared &S, u32t it, unsigned *b) {
+    for (int q = 0; q < 6; q++) b[q] = S.box[q][it];
+}
+template <class Shared>
+__device__ __forceinline__ float item_centroid(const Shared &S, u32t it, int a) {
+    return (fo(S.box[a][it]) + fo(S.box[3 + a][it])) * 0.5f;
+}
+__device__ __forceinline__ void clear_bins(unsigned *bins, u32t at, u32t step) {
+    for (u32t k = at; k < (u32t)kWarpBins; k += step) {
+        const u32t w = (k / kBins) % kSweepWords;
+        bins[k] = w >= 1 && w <= 3 ? 0xFFFFFFFFu : 0u;
+    }
+}
+template <class Shared>
+__device__ __forceinline__ void bin_item(unsigned *bins, const Axes &A, const Shared &S, u32t it) {
+    unsigned b[6];
+    item_bits(S, it, b);
+    for (int a = 0; a < 3; a++) {
+        if (!A.valid[a]) continue;
+        unsigned *d = bins + a * kSweepWords * kBins + bin_of((fo(b[a]) + fo(b[3 + a])) * 0.5f, A.lo[a], A.scale[a]);
+        atomicAdd(d, 1u);
+        for (int q = 0; q < 3; q++) { atomicMin(d + (1 + q) * kBins, b[q]); atomicMax(d + (4 + q) * kBins, b[3 + q]); }
+    }
+}
+__device__ __forceinline__ Split sweep_bins(const unsigned *bins, const Axes &A, int a, int lane) {
+    if (!A.valid[a]) return Split{INFINITY, kNoSplit, 0};
+    const unsigned *d = bins + a * kSweepWords * kBins + lane;
+    unsigned b[6];
+    for (int q = 0; q < 6; q++) b[q] = d[(1 + q) * kBins];
+    return sweep_axis(b, d[0], a, lane);
+}
+template <class Shared>
+__device__ __forceinline__ bool goes_left(const Shared &S, const Axes &A, const Split &s, u32t it, u32t place) {
+    if (s.key == kNoSplit) return place < s.nleft;
+    const int a = s.key / kBins;
+    return bin_of(item_centroid(S, it, a), A.lo[a], A.scale[a]) <= s.key % kBins;
+}
+// Every candidate split of a tiny range, a lane each: after the bin of item i on axis a (a split after
+// a bin that holds no item parts the items as the next lower bin that holds some, and ties go to it).
+__device__ __forceinline__ Split tiny_split(const SubtreeShared &S, const Axes &A, const uint16_t *ord, u32t cnt, int lane) {
+    const int a = lane / (int)kTiny;
+    const u32t i = lane % kTiny;
+    const bool on = a < 3 && i < cnt && A.valid[a];
+    u32t bin = kBins;
+    if (on) bin = bin_of(item_centroid(S, ord[i], a), A.lo[a], A.scale[a]);
+    unsigned L[6], R[6];
+    empty6(L);
+    empty6(R);
+    u32t nl = 0;
+    for (u32t j = 0; j < cnt; j++) {
+        const u32t other = __shfl_sync(0xFFFFFFFFu, bin, (a < 3 ? a : 2) * (int)kTiny + (int)j);
+        unsigned b[6];
+        item_bits(S, ord[j], b);
+        if (other <= bin) { grow6(L, b); nl++; }
+        else grow6(R, b);
+    }
+    Split s{INFINITY, kNoSplit, 0};
+    if (on && nl < cnt) {
+        const float cost = half_area_bits(L) * (float)nl + half_area_bits(R) * (float)(cnt - nl);
+        if (cost < INFINITY) s = Split{cost, a * kBins + bin, nl};
+    }
+    return warp_best(s);
+}
+
+// A range's items into shared memory.
+template <class Shared>
+__device__ __forceinline__ void load_items(Shared &S, const float *aabbs, const u32t *ids, u32t base, u32t cnt) {
+    for (u32t k = threadIdx.x; k < cnt; k += blockDim.x) {
+        const u32t it = ids ? ids[base + k] : base + k;
+        const float2 *f = reinterpret_cast<const float2 *>(aabbs + 6 * (size_t)it);
+        const float2 p = f[0], q = f[1], r = f[2];
+        S.box[0][k] = ob(p.x); S.box[1][k] = ob(p.y); S.box[2][k] = ob(q.x);
+        S.box[3][k] = ob(q.y); S.box[4][k] = ob(r.x); S.box[5][k] = ob(r.y);
+        S.order[0][k] = (uint16_t)k;
+    }
+}
+// The left items before each thread's, over a block of WARPS warps (all threads call; `sums` is
+// reused: the caller syncs before the next use).
+template <int WARPS>
+__device__ __forceinline__ u32t block_exclusive(u32t v, u32t *sums, u32t &total) {
+    const u32t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u32t x = v;
+    for (int off = 1; off < 32; off <<= 1) {
+        const u32t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+        if (lane >= (u32t)off) x += y;
+    }
+    if (lane == 31) sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        u32t w = lane < WARPS ? sums[lane] : 0;
+        for (int off = 1; off < 32; off <<= 1) {
+            const u32t y = __shfl_up_sync(0xFFFFFFFFu, w, off);
+            if (lane >= (u32t)off) w += y;
+        }
+        if (lane < WARPS) sums[lane] = w;
+    }
+    __syncthreads();
+    total = sums[WARPS - 1];
+    return (warp ? sums[warp - 1] : 0) + x - v;
+}
+
+// Ranges of kSub to kCap items, a block each: split level after level by the whole block; children of
+// at most kSub items (or a leaf's) are left to sah_subtree_kernel.  The ranges are mids[0, C->mids), or
+// with mids == null the whole build, [0, n).
+__global__ void __launch_bounds__(kMidThreads, 1) sah_mid_kernel(const float *aabbs, SahCounts *C, const SahTask *mids, u32t n,
+                                                                 u32t max_leaf, u32t *ids0, u32t *ids1, LargeNode *nodes,
+                                                                 SahTask *subtrees) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    MidShared &S = *reinterpret_cast<MidShared *>(raw);
+    const u32t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const u32t ranges = mids ? C->mids : 1;
+    for (u32t range = blockIdx.x; range < ranges; range += gridDim.x) {
+        SahTask T{0, n, 0, 0, kNoSplit, 0};
+        if (mids) T = mids[range];
+        const u32t *ids = !mids ? nullptr : T.source ? ids1 : ids0;      // null: the identity
+        u32t *parted = T.source ? ids0 : ids1;                // the children's items go to the other buffer
+        const u32t base = T.begin;
+        __syncthreads();
+        load_items(S, aabbs, ids, base, T.end - T.begin);
+        if (tid == 0) {
+            S.task[0][0] = SahTask{0, T.end - T.begin, T.level, 0, T.parent, T.side};
+            S.tasks[0] = 1;
+            S.tasks[1] = 0;
+        }
+        __syncthreads();
+        for (int cur = 0; S.tasks[cur]; cur ^= 1) {
+            const uint16_t *ord = S.order[cur];
+            uint16_t *ord_next = S.order[cur ^ 1];
+            for (u32t t = 0; t < S.tasks[cur]; t++) {
+                const SahTask K = S.task[cur][t];
+                const u32t b = K.begin, e = K.end, c = e - b;
+                unsigned bx[6], cb[6];
+                empty6(bx);
+                empty6(cb);
+                if (tid < 12) S.red[tid] = tid % 6 < 3 ? 0xFFFFFFFFu : 0u;
+                clear_bins(S.bins, tid, kMidThreads);
+                __syncthreads();
+                for (u32t k = b + tid; k < e; k += kMidThreads) {
+                    unsigned it[6], ct[6];
+                    item_bits(S, ord[k], it);
+                    for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob((fo(it[q]) + fo(it[3 + q])) * 0.5f);
+                    grow6(bx, it);
+                    grow6(cb, ct);
+                }
+                warp_grow6(bx);
+                warp_grow6(cb);
+                if (lane == 0) { atomic_grow6(S.red, bx); atomic_grow6(S.red + 6, cb); }
+                __syncthreads();
+                const Axes A = axes_of(S.red + 6);
+                for (u32t k = b + tid; k < e; k += kMidThreads) bin_item(S.bins, A, S, ord[k]);
+                __syncthreads();
+                if (warp < 3) {
+                    const Split s = sweep_bins(S.bins, A, (int)warp, (int)lane);
+                    if (lane == 0) S.axis_split[warp] = s;
+                }
+                __syncthreads();
+                Split s = better(better(S.axis_split[0], S.axis_split[1]), S.axis_split[2]);
+                if (s.key == kNoSplit) s.nleft = c / 2;
+                // stable partition: a thread takes consecutive places
+                const u32t per = (c + kMidThreads - 1) / kMidThreads;
+                const u32t k0 = b + min(tid * per, c), k1 = b + min((tid + 1) * per, c);
+                u32t left = 0, total;
+                for (u32t k = k0; k < k1; k++) left += goes_left(S, A, s, ord[k], k - b);
+                u32t before = block_exclusive<kMidWarps>(left, S.warp_sum, total);
+                for (u32t k = k0; k < k1; k++) {
+                    const uint16_t it = ord[k];
+                    const bool l = goes_left(S, A, s, it, k - b);
+                    ord_next[l ? b + before : b + s.nleft + (k - b - before)] = it;
+                    before += l;
+                }
+                if (tid == 0) {
+                    const u32t self = atomicAdd(&C->nodes, 1u);
+                    LargeNode &o = nodes[self];
+                    for (int q = 0; q < 6; q++) o.box[q] = S.red[q];
+                    o.begin = base + b; o.level = K.level; o.parent = K.parent; o.side = K.side;
+                    for (u32t side = 0; side < 2; side++) {
+                        SahTask N{side ? b + s.nleft : b, side ? e : b + s.nleft, K.level + 1, T.source ? 0u : 1u, self, side};
+                        const u32t nc = N.end - N.begin;
+                        S.child[side] = nc <= kSub || nc <= max_leaf;
+                        if (S.child[side]) {
+                            N.begin += base;
+                            N.end += base;
+                            subtrees[atomicAdd(&C->subtrees, 1u)] = N;
+                        } else {
+                            S.task[cur ^ 1][S.tasks[cur ^ 1]++] = N;
+                        }
+                    }
+                }
+                __syncthreads();
+                // a child that leaves takes its items, in their order, with it
+                for (u32t k = b + tid; k < e; k += kMidThreads) {
+                    if (!S.child[k - b < s.nleft ? 0 : 1]) continue;
+                    const u32t it = base + ord_next[k];
+                    parted[base + k] = ids ? ids[it] : it;
+                }
+                __syncthreads();
+            }
+            if (tid == 0) S.tasks[cur] = 0;
+            __syncthreads();
+        }
+    }
+}
+
+// Ranges of at most kSub items, and leaves of any size, a block each, to the leaves: records at
+// 2 * begin, the splits of the range's level l counted in splits[begin + l], the number of its levels
+// in levels[range].  With subtrees == null the range is the whole build, [0, n), and the nodes are
+// written to their slots as they come, info = {-, height, pairs}.
+__global__ void __launch_bounds__(kThreads) sah_subtree_kernel(const float *aabbs, SahCounts *C, const SahTask *subtrees, u32t n,
+                                                               u32t max_leaf, const u32t *ids0, const u32t *ids1,
+                                                               u32t *out_order, BVHNode *nodes, u32t *info,
+                                                               SahRecord *records, u32t *splits, u32t *levels) {
+    __shared__ SubtreeShared S;
+    const u32t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const u32t ranges = subtrees ? C->subtrees : 1;
+    for (u32t range = blockIdx.x; range < ranges; range += gridDim.x) {
+        SahTask T{0, n, 0, 0, kNoSplit, 0};
+        if (subtrees) T = subtrees[range];
+        const u32t *ids = T.source ? ids1 : ids0;             // null: the identity
+        const u32t cnt = T.end - T.begin, base = T.begin;
+        SahRecord *rec = subtrees ? records + 2 * (size_t)base : nullptr;
+        __syncthreads();
+        if (cnt <= max_leaf) {                                // one leaf, of any size
+            unsigned b[6];
+            empty6(b);
+            if (tid < 6) S.red[tid] = tid < 3 ? 0xFFFFFFFFu : 0u;
+            __syncthreads();
+            for (u32t k = tid; k < cnt; k += kThreads) {
+                const u32t it = ids ? ids[base + k] : base + k;
+                out_order[base + k] = it;
+                for (int q = 0; q < 6; q++) {
+                    const unsigned w = ob(aabbs[6 * (size_t)it + q]);
+                    b[q] = q < 3 ? min(b[q], w) : max(b[q], w);
+                }
+            }
+            warp_grow6(b);
+            if (lane == 0) atomic_grow6(S.red, b);
+            __syncthreads();
+            if (tid == 0) {
+                if (!rec) {
+                    write_node(nodes[0], S.red, 0, cnt, 0);
+                    info[0] = 0; info[1] = 1; info[2] = 0;
+                } else {
+                    for (int q = 0; q < 6; q++) rec[0].box[q] = S.red[q];
+                    rec[0].first = base; rec[0].count = cnt; rec[0].level = T.level; rec[0].index = 0;
+                    splits[base] = 0;
+                    levels[range] = 1;
+                    atomicMax(info + 1, T.level);
+                }
+            }
+            continue;
+        }
+        load_items(S, aabbs, ids, base, cnt);
+        if (tid == 0) { S.task[0][0][0] = 0; S.task[0][0][1] = (uint16_t)cnt; }
+        __syncthreads();
+        u32t nt = 1, pairs = 0, written = 0, level = 0, height = 0;
+        for (int cur = 0; nt; cur ^= 1, level++) {
+            const uint16_t *ord = S.order[cur];
+            uint16_t *ord_next = S.order[cur ^ 1];
+            // the ranks of the level's splits, left to right
+            u32t mine = 0, level_splits;
+            for (u32t k = kPer * tid; k < min(kPer * tid + kPer, nt); k++)
+                mine += (u32t)(S.task[cur][k][1] - S.task[cur][k][0]) > max_leaf;
+            u32t rank = block_exclusive<kWarps>(mine, S.warp_sum, level_splits);
+            for (u32t k = kPer * tid; k < min(kPer * tid + kPer, nt); k++) {
+                const u32t b = S.task[cur][k][0], e = S.task[cur][k][1];
+                if (e - b > max_leaf) {
+                    S.task[cur ^ 1][2 * rank][0] = (uint16_t)b;      // (the middle is filled in by the split)
+                    S.task[cur ^ 1][2 * rank + 1][1] = (uint16_t)e;
+                    // the split finds its rank in its range's first place of the next order, which is
+                    // free until the range is parted into it
+                    ord_next[b] = (uint16_t)rank;
+                    rank++;
+                }
+            }
+            __syncthreads();
+            for (u32t t = warp; t < nt; t += kWarps) {
+                const u32t b = S.task[cur][t][0], e = S.task[cur][t][1], c = e - b;
+                const bool leaf = c <= max_leaf;
+                unsigned bx[6], cb[6];
+                empty6(bx);
+                empty6(cb);
+                for (u32t k = b + lane; k < e; k += 32) {
+                    unsigned it[6], ct[6];
+                    item_bits(S, ord[k], it);
+                    for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob((fo(it[q]) + fo(it[3 + q])) * 0.5f);
+                    grow6(bx, it);
+                    grow6(cb, ct);
+                }
+                warp_grow6(bx);
+                u32t first = base + b;
+                if (leaf) {
+                    for (u32t k = b + lane; k < e; k += 32) {
+                        const u32t it = base + ord[k];
+                        out_order[base + k] = ids ? ids[it] : it;
+                    }
+                } else {
+                    warp_grow6(cb);
+                    const Axes A = axes_of(cb);
+                    const u32t r = ord_next[b];
+                    __syncwarp();
+                    Split s;
+                    if (c <= kTiny) {
+                        s = tiny_split(S, A, ord + b, c, (int)lane);
+                    } else {
+                        unsigned *bins = S.bins[warp];
+                        clear_bins(bins, lane, 32);
+                        __syncwarp();
+                        for (u32t k = b + lane; k < e; k += 32) bin_item(bins, A, S, ord[k]);
+                        __syncwarp();
+                        s = sweep_bins(bins, A, 0, (int)lane);
+                        s = better(s, sweep_bins(bins, A, 1, (int)lane));
+                        s = better(s, sweep_bins(bins, A, 2, (int)lane));
+                        __syncwarp();
+                    }
+                    if (s.key == kNoSplit) s.nleft = c / 2;
+                    u32t before = 0;
+                    for (u32t k0 = b; k0 < e; k0 += 32) {
+                        const u32t k = k0 + lane;
+                        const uint16_t it = k < e ? ord[k] : 0;
+                        const bool l = k < e && goes_left(S, A, s, it, k - b);
+                        const unsigned m = __ballot_sync(0xFFFFFFFFu, l);
+                        const u32t lb = before + __popc(m & ((1u << lane) - 1u));
+                        if (k < e) ord_next[l ? b + lb : b + s.nleft + (k - b - lb)] = it;
+                        before += __popc(m);
+                    }
+                    if (lane == 0) S.task[cur ^ 1][2 * r][1] = S.task[cur ^ 1][2 * r + 1][0] = (uint16_t)(b + s.nleft);
+                    first = rec ? r : 1 + 2 * (pairs + r);
+                }
+                if (lane == 0) {
+                    if (!rec) {
+                        write_node(nodes[written + t], bx, first, leaf ? c : 0, level);
+                    } else {
+                        SahRecord &o = rec[written + t];
+                        for (int q = 0; q < 6; q++) o.box[q] = bx[q];
+                        o.first = first; o.count = leaf ? c : 0; o.level = T.level + level; o.index = t;
+                    }
+                }
+            }
+            if (rec && tid == 0) splits[base + level] = level_splits;
+            if (level_splits < nt) height = level;             // some range of the level is a leaf
+            written += nt;
+            pairs += level_splits;
+            nt = 2 * level_splits;
+            __syncthreads();
+        }
+        if (tid == 0) {
+            if (!rec) {
+                info[0] = 0;
+                info[1] = height < 1 ? 1 : height;
+                info[2] = pairs;
+            } else {
+                levels[range] = level;
+                atomicMax(info + 1, T.level + height);
+            }
+        }
+    }
+}
+
+// ---- ranges above kCap items: many blocks each, a level at a time ------------------------------------
+struct LargeTask {
+    SahTask t;
+    u32t chunk0;                       // its first chunk of this level
+    unsigned cbox[6];
+};
+__global__ void sah_init_kernel(SahCounts *C) {
+    if (threadIdx.x < 6) C->root[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    if (threadIdx.x == 0) {
+        C->large[0] = C->large[1] = C->chunks[0] = C->chunks[1] = C->mids = C->nodes = C->subtrees = 0;
+        C->info[1] = 1;
+        C->info[2] = 0;
+    }
+}
+__global__ void sah_root_kernel(const float *aabbs, u32t n, SahCounts *C) {
+    unsigned c[6];
     empty6(c);
     for (u32t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float *a = aabbs + 6 * (size_t)i;
-        unsigned it[6], ct[6];
-        for (int q = 0; q < 3; q++) {
-            float cc = (a[q] + a[3 + q]) * 0.5f;
-            cent[3 * (size_t)i + q] = cc;
-            ct[q] = ct[3 + q] = ob(cc);
-        }
-        for (int q = 0; q < 6; q++) it[q] = ob(a[q]);
-        grow6(b, it);
+        unsigned ct[6];
+        for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob((a[q] + a[3 + q]) * 0.5f);
         grow6(c, ct);
-        ids[i] = i;
     }
-    for (int q = 0; q < 3; q++)
-        for (int off = 16; off; off >>= 1) {
-            b[q] = min(b[q], __shfl_down_sync(0xFFFFFFFFu, b[q], off));
-            b[3 + q] = max(b[3 + q], __shfl_down_sync(0xFFFFFFFFu, b[3 + q], off));
-            c[q] = min(c[q], __shfl_down_sync(0xFFFFFFFFu, c[q], off));
-            c[3 + q] = max(c[3 + q], __shfl_down_sync(0xFFFFFFFFu, c[3 + q], off));
-        }
-    if ((threadIdx.x & 31) == 0) {
-        atomic_grow6(root, b);
-        atomic_grow6(root + 6, c);
+    warp_grow6(c);
+    if ((threadIdx.x & 31) == 0) atomic_grow6(C->root, c);
+}
+__device__ __forceinline__ u32t chunks_of(const SahTask &t) { return (t.end - t.begin + kChunk - 1) / kChunk; }
+__device__ void clear_large_bins(unsigned *g, u32t at, u32t step) {
+    for (u32t k = at; k < 3u * kBins; k += step) {
+        g[k * kBinWords] = 0;
+        empty6(g + k * kBinWords + 1);
+        empty6(g + k * kBinWords + 7);
     }
 }
-__global__ void sah_root_init_kernel(unsigned *root) {
-    if (threadIdx.x == 0) { empty6(root); empty6(root + 6); }
-}
-__global__ void sah_root_task_kernel(const unsigned *root, u32t n, SahTask *tasks) {
-    SahTask t;
-    t.begin = 0;
-    t.end = n;
-    t.slot = 0;
-    t.pad = 0;
-    for (int q = 0; q < 6; q++) { t.box[q] = root[q]; t.cbox[q] = root[6 + q]; }
-    tasks[0] = t;
-}
-
-// ---- per level: classification -------------------------------------------------------------
-// flags: [0,nt) split, [nt,2nt) large, [2nt,3nt) chunks of large tasks
-__global__ void sah_classify_kernel(const SahTask *tasks, u32t nt, u32t max_leaf, u32t *flags) {
-    u32t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt) return;
-    u32t cnt = tasks[t].end - tasks[t].begin;
-    bool split = cnt > max_leaf;
-    bool large = cnt > (u32t)kSmall;
-    flags[t] = split;
-    flags[nt + t] = large;
-    flags[2 * nt + t] = large ? (cnt + kChunk - 1) / kChunk : 0;
-}
-// scanned: [0,nt) pair index within the level, [nt,2nt) large rank, [2nt,3nt) chunk offset
-__global__ void sah_large_list_kernel(const SahTask *tasks, u32t nt, const u32t *flags, const u32t *scanned,
-                                      u32t *large_tasks, u32t *chunk_task) {
-    u32t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt || !flags[nt + t]) return;
-    u32t r = scanned[nt + t];
-    large_tasks[r] = t;
-    u32t off = scanned[2 * nt + t], c = flags[2 * nt + t];
-    for (u32t k = 0; k < c; k++) chunk_task[off + k] = r;
-}
-
-// ---- large tasks: global binning ------------------------------------------------------------
-__device__ __forceinline__ void task_axes(const SahTask &T, float lo[3], float scale[3], bool valid[3]) {
-    for (int a = 0; a < 3; a++) {
-        float l = fo(T.cbox[a]), h = fo(T.cbox[3 + a]);
-        float e = h - l;
-        valid[a] = e > 0.0f;
-        lo[a] = l;
-        scale[a] = valid[a] ? (float)kBins / e : 0.0f;
+__global__ void sah_first_kernel(u32t n, SahCounts *C, LargeTask *tasks, u32t *chunk_task, unsigned *bins) {
+    const SahTask t{0, n, 0, 2, kNoSplit, 0};
+    if (threadIdx.x == 0) {
+        LargeTask L;
+        L.t = t;
+        L.chunk0 = 0;
+        for (int q = 0; q < 6; q++) L.cbox[q] = C->root[q];
+        tasks[0] = L;
+        C->large[0] = 1;
+        C->chunks[0] = chunks_of(t);
     }
+    for (u32t k = threadIdx.x; k < chunks_of(t); k += blockDim.x) chunk_task[k] = 0;
+    clear_large_bins(bins, threadIdx.x, blockDim.x);
 }
-__global__ void sah_bin_large_kernel(const SahTask *tasks, const u32t *large_tasks, const u32t *chunk_task,
-                                     const u32t *chunk_offsets, const u32t *ids, const float *aabbs, const float *cent,
-                                     unsigned *gbins) {
+// source 2: the identity (the root's level)
+__device__ __forceinline__ u32t item_at(const u32t *ids0, const u32t *ids1, u32t source, u32t k) {
+    return source == 2 ? k : source ? ids1[k] : ids0[k];
+}
+// One chunk of a large range: its items binned in shared memory, then added to the range's bins; the
+// chunk's own counts are kept for the partition.
+__global__ void sah_bin_kernel(const float *aabbs, const SahCounts *C, int now, const LargeTask *tasks, const u32t *chunk_task,
+                               const u32t *ids0, const u32t *ids1, unsigned *bins, uint16_t *chunk_counts) {
     __shared__ unsigned sb[3 * kBins * kBinWords];
+    if (blockIdx.x >= C->chunks[now]) return;
     const u32t r = chunk_task[blockIdx.x];
-    const SahTask T = tasks[large_tasks[r]];
-    const u32t chunk = blockIdx.x - chunk_offsets[large_tasks[r]];
-    for (int k = threadIdx.x; k < 3 * kBins; k += blockDim.x) {
-        unsigned *b = sb + k * kBinWords;
-        b[0] = 0;
-        empty6(b + 1);
-        empty6(b + 7);
-    }
+    const LargeTask L = tasks[r];
+    clear_large_bins(sb, threadIdx.x, blockDim.x);
     __syncthreads();
-    float lo[3], scale[3];
-    bool valid[3];
-    task_axes(T, lo, scale, valid);
-    const u32t first = T.begin + chunk * kChunk, last = min(T.end, first + kChunk);
+    const Axes A = axes_of(L.cbox);
+    const bool none = !(A.valid[0] | A.valid[1] | A.valid[2]);      // the box is still wanted: bin 0 of axis 0
+    const u32t first = L.t.begin + (blockIdx.x - L.chunk0) * kChunk, last = min(L.t.end, first + kChunk);
     for (u32t k = first + threadIdx.x; k < last; k += blockDim.x) {
-        const u32t i = ids[k];
+        const u32t i = item_at(ids0, ids1, L.t.source, k);
+        float f[6];
         unsigned it[6], ct[6];
-        for (int q = 0; q < 6; q++) it[q] = ob(aabbs[6 * (size_t)i + q]);
-        for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob(cent[3 * (size_t)i + q]);
+        for (int q = 0; q < 6; q++) { f[q] = aabbs[6 * (size_t)i + q]; it[q] = ob(f[q]); }
+        float c[3];
+        for (int q = 0; q < 3; q++) { c[q] = (f[q] + f[3 + q]) * 0.5f; ct[q] = ct[3 + q] = ob(c[q]); }
         for (int a = 0; a < 3; a++) {
-            if (!valid[a]) continue;
-            unsigned *b = sb + (a * kBins + bin_of(cent[3 * (size_t)i + a], lo[a], scale[a])) * kBinWords;
+            if (!A.valid[a] && !(none && a == 0)) continue;
+            unsigned *b = sb + (a * kBins + (none ? 0 : bin_of(c[a], A.lo[a], A.scale[a]))) * kBinWords;
             atomicAdd(b, 1u);
             atomic_grow6(b + 1, it);
             atomic_grow6(b + 7, ct);
         }
     }
     __syncthreads();
-    unsigned *g = gbins + (size_t)r * 3 * kBins * kBinWords;
+    unsigned *g = bins + (size_t)r * 3 * kBins * kBinWords;
     for (int k = threadIdx.x; k < 3 * kBins; k += blockDim.x) {
         const unsigned *b = sb + k * kBinWords;
+        chunk_counts[(size_t)blockIdx.x * 3 * kBins + k] = (uint16_t)b[0];
         if (!b[0]) continue;
         unsigned *d = g + k * kBinWords;
         atomicAdd(d, b[0]);
@@ -169,417 +629,354 @@ __global__ void sah_bin_large_kernel(const SahTask *tasks, const u32t *large_tas
         atomic_grow6(d + 7, b + 7);
     }
 }
-__global__ void sah_clear_bins_kernel(unsigned *gbins, u32t nlarge) {
-    u32t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nlarge * 3 * kBins) return;
-    unsigned *b = gbins + (size_t)k * kBinWords;
-    b[0] = 0;
-    empty6(b + 1);
-    empty6(b + 7);
-}
-
-// Sweep the bins of one task (one warp; lanes 0..2 take one axis each).  Writes the decision
-// (axis, k; axis -1 = middle split) and, for a binned split, the children's boxes and left count.
-__device__ void sweep(const unsigned *bins, const bool valid[3], int lane, int &best_axis, int &best_k, float &best_cost) {
-    float cost_a = INFINITY;
-    int k_a = -1;
-    if (lane < 3 && valid[lane]) {
-        const unsigned *B = bins + lane * kBins * kBinWords;
-        unsigned R[kBins][6];
-        u32t nR[kBins];
-        unsigned acc[6];
-        empty6(acc);
-        u32t an = 0;
-        for (int b = kBins - 1; b >= 1; b--) {
-            grow6(acc, B + b * kBinWords + 1);
-            an += B[b * kBinWords];
-            for (int q = 0; q < 6; q++) R[b][q] = acc[q];
-            nR[b] = an;
-        }
-        empty6(acc);
-        an = 0;
-        for (int k = 0; k < kBins - 1; k++) {
-            grow6(acc, B + k * kBinWords + 1);
-            an += B[k * kBinWords];
-            if (!an || !nR[k + 1]) continue;
-            float cost = half_area_bits(acc) * (float)an + half_area_bits(R[k + 1]) * (float)nR[k + 1];
-            if (cost < cost_a) { cost_a = cost; k_a = k; }
-        }
-    }
-    float c0 = __shfl_sync(0xFFFFFFFFu, cost_a, 0), c1 = __shfl_sync(0xFFFFFFFFu, cost_a, 1), c2 = __shfl_sync(0xFFFFFFFFu, cost_a, 2);
-    int k0 = __shfl_sync(0xFFFFFFFFu, k_a, 0), k1 = __shfl_sync(0xFFFFFFFFu, k_a, 1), k2 = __shfl_sync(0xFFFFFFFFu, k_a, 2);
-    best_axis = -1;
-    best_k = -1;
-    best_cost = INFINITY;
-    if (k0 >= 0 && c0 < best_cost) { best_cost = c0; best_axis = 0; best_k = k0; }
-    if (k1 >= 0 && c1 < best_cost) { best_cost = c1; best_axis = 1; best_k = k1; }
-    if (k2 >= 0 && c2 < best_cost) { best_cost = c2; best_axis = 2; best_k = k2; }
-}
-
-struct SahDecision { int axis, k; u32t nleft; unsigned lbox[6], lcbox[6], rbox[6], rcbox[6]; };
-
-__device__ void side_boxes(const unsigned *bins, int axis, int k, SahDecision &d) {
-    empty6(d.lbox); empty6(d.lcbox); empty6(d.rbox); empty6(d.rcbox);
-    d.nleft = 0;
-    const unsigned *B = bins + axis * kBins * kBinWords;
-    for (int b = 0; b < kBins; b++) {
-        if (b <= k) { grow6(d.lbox, B + b * kBinWords + 1); grow6(d.lcbox, B + b * kBinWords + 7); d.nleft += B[b * kBinWords]; }
-        else { grow6(d.rbox, B + b * kBinWords + 1); grow6(d.rcbox, B + b * kBinWords + 7); }
-    }
-}
-
-// one warp per large task
-__global__ void sah_split_large_kernel(const SahTask *tasks, const u32t *large_tasks, u32t nlarge, const unsigned *gbins,
-                                       SahDecision *dec) {
-    const u32t r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    if (r >= nlarge) return;
-    const int lane = threadIdx.x & 31;
-    const SahTask T = tasks[large_tasks[r]];
-    float lo[3], scale[3];
-    bool valid[3];
-    task_axes(T, lo, scale, valid);
-    const unsigned *bins = gbins + (size_t)r * 3 * kBins * kBinWords;
-    int axis, k;
-    float cost;
-    sweep(bins, valid, lane, axis, k, cost);
-    if (lane == 0) {
-        SahDecision d;
-        d.axis = axis;
-        d.k = k;
-        if (axis >= 0) side_boxes(bins, axis, k, d);
-        else {
-            d.nleft = (T.end - T.begin) / 2;
-            empty6(d.lbox); empty6(d.lcbox); empty6(d.rbox); empty6(d.rcbox);
-        }
-        dec[r] = d;
-    }
-}
-
-// middle split of a large task: children's boxes from the items (rare: all centroids equal)
-__global__ void sah_middle_boxes_kernel(const SahTask *tasks, const u32t *large_tasks, const u32t *chunk_task,
-                                        const u32t *chunk_offsets, const u32t *ids, const float *aabbs,
-                                        const float *cent, SahDecision *dec) {
+// One large range: its split is found (every block finds it, a warp for each axis), its items are
+// parted into the other id buffer, and the first chunk's block writes its node and its children.
+__global__ void sah_part_kernel(const float *aabbs, SahCounts *C, int now, u32t max_leaf, const LargeTask *tasks,
+                                const u32t *chunk_task, u32t *ids0, u32t *ids1, const unsigned *bins,
+                                const uint16_t *chunk_counts, LargeTask *next, u32t *next_chunk_task, unsigned *next_bins,
+                                LargeNode *nodes, SahTask *mids, SahTask *subtrees) {
+    __shared__ Split axis_split[3];
+    __shared__ u32t warp_sums[8], left_before, child[2], place[2];
+    __shared__ unsigned cb[2][6];
+    if (blockIdx.x >= C->chunks[now]) return;
+    const u32t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const u32t r = chunk_task[blockIdx.x];
-    SahDecision &d = dec[r];
-    if (d.axis >= 0) return;
-    const SahTask T = tasks[large_tasks[r]];
-    const u32t chunk = blockIdx.x - chunk_offsets[large_tasks[r]];
-    const u32t mid = T.begin + d.nleft;
-    const u32t first = T.begin + chunk * kChunk, last = min(T.end, first + kChunk);
-    for (u32t k = first + threadIdx.x; k < last; k += blockDim.x) {
-        const u32t i = ids[k];
-        unsigned it[6], ct[6];
-        for (int q = 0; q < 6; q++) it[q] = ob(aabbs[6 * (size_t)i + q]);
-        for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob(cent[3 * (size_t)i + q]);
-        if (k < mid) { atomic_grow6(d.lbox, it); atomic_grow6(d.lcbox, ct); }
-        else { atomic_grow6(d.rbox, it); atomic_grow6(d.rcbox, ct); }
+    const LargeTask L = tasks[r];
+    const u32t chunk = blockIdx.x - L.chunk0, cnt = L.t.end - L.t.begin;
+    const Axes A = axes_of(L.cbox);
+    const unsigned *g = bins + (size_t)r * 3 * kBins * kBinWords;
+    if (tid == 0) left_before = 0;
+    if (warp < 3) {
+        Split s{INFINITY, kNoSplit, 0};
+        if (A.valid[warp]) {
+            const unsigned *b = g + (warp * kBins + lane) * kBinWords;
+            s = sweep_axis(b + 1, b[0], (int)warp, (int)lane);
+        }
+        if (lane == 0) axis_split[warp] = s;
     }
-}
-
-// stable partition of large tasks: per-chunk left counts, a per-task scan over its chunks, scatter
-__device__ __forceinline__ bool goes_left(const SahDecision &d, const float lo[3], const float scale[3], const float *cent,
-                                          u32t i, u32t pos, u32t mid) {
-    if (d.axis < 0) return pos < mid;
-    return bin_of(cent[3 * (size_t)i + d.axis], lo[d.axis], scale[d.axis]) <= (u32t)d.k;
-}
-__global__ void sah_count_left_kernel(const SahTask *tasks, const u32t *large_tasks, const u32t *chunk_task,
-                                      const u32t *chunk_offsets, const u32t *ids, const float *cent,
-                                      const SahDecision *dec, u32t *chunk_left) {
-    __shared__ u32t total;
-    const u32t r = chunk_task[blockIdx.x];
-    const SahTask T = tasks[large_tasks[r]];
-    const SahDecision d = dec[r];
-    const u32t chunk = blockIdx.x - chunk_offsets[large_tasks[r]];
-    float lo[3], scale[3];
-    bool valid[3];
-    task_axes(T, lo, scale, valid);
-    if (threadIdx.x == 0) total = 0;
     __syncthreads();
-    const u32t first = T.begin + chunk * kChunk, last = min(T.end, first + kChunk);
-    u32t c = 0;
-    for (u32t k = first + threadIdx.x; k < last; k += blockDim.x)
-        c += goes_left(d, lo, scale, cent, ids[k], k, T.begin + d.nleft);
-    for (int off = 16; off; off >>= 1) c += __shfl_down_sync(0xFFFFFFFFu, c, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&total, c);
+    Split s = better(better(axis_split[0], axis_split[1]), axis_split[2]);
+    const bool middle = s.key == kNoSplit;
+    if (middle) s.nleft = cnt / 2;
+    const int axis = middle ? 0 : (int)(s.key / kBins);
+    const u32t kbin = s.key % kBins;
+    // the left items in the chunks before this one
+    if (!middle) {
+        u32t c = 0;
+        for (u32t k = tid; k < chunk * kBins; k += blockDim.x)
+            if (k % kBins <= kbin) c += chunk_counts[((size_t)(L.chunk0 + k / kBins) * 3 + axis) * kBins + k % kBins];
+        c = __reduce_add_sync(0xFFFFFFFFu, c);
+        if (lane == 0) atomicAdd(&left_before, c);
+    }
     __syncthreads();
-    if (threadIdx.x == 0) chunk_left[blockIdx.x] = total;
-}
-__global__ void sah_chunk_scan_kernel(const u32t *large_tasks, u32t nlarge, const u32t *chunk_offsets, const u32t *flags,
-                                      u32t nt, u32t *chunk_left) {
-    u32t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nlarge) return;
-    u32t t = large_tasks[r];
-    u32t off = chunk_offsets[t], c = flags[2 * nt + t], run = 0;
-    for (u32t k = 0; k < c; k++) { u32t v = chunk_left[off + k]; chunk_left[off + k] = run; run += v; }
-}
-__global__ void sah_scatter_kernel(const SahTask *tasks, const u32t *large_tasks, const u32t *chunk_task,
-                                   const u32t *chunk_offsets, const u32t *ids, const float *cent, const SahDecision *dec,
-                                   const u32t *chunk_left, u32t *tmp) {
-    __shared__ u32t warp_sums[8];
-    __shared__ u32t carry;
-    const u32t r = chunk_task[blockIdx.x];
-    const SahTask T = tasks[large_tasks[r]];
-    const SahDecision d = dec[r];
-    const u32t chunk = blockIdx.x - chunk_offsets[large_tasks[r]];
-    float lo[3], scale[3];
-    bool valid[3];
-    task_axes(T, lo, scale, valid);
-    const u32t first = T.begin + chunk * kChunk, last = min(T.end, first + kChunk);
-    const u32t left_before = chunk_left[blockIdx.x];
-    const u32t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (u32t base = first; base < last; base += blockDim.x) {
-        const u32t k = base + threadIdx.x;
+    const u32t first = L.t.begin + chunk * kChunk, last = min(L.t.end, first + kChunk);
+    const u32t target = L.t.source == 0 ? 1u : 0u;
+    u32t *out = target ? ids1 : ids0;
+    u32t carry = middle ? min(chunk * kChunk, s.nleft) : left_before;
+    for (u32t b0 = first; b0 < last; b0 += blockDim.x) {
+        const u32t k = b0 + tid;
         const bool in = k < last;
-        const u32t i = in ? ids[k] : 0;
-        const bool l = in && goes_left(d, lo, scale, cent, i, k, T.begin + d.nleft);
+        const u32t i = in ? item_at(ids0, ids1, L.t.source, k) : 0;
+        bool l = false;
+        if (in) {
+            if (middle) l = k - L.t.begin < s.nleft;
+            else l = bin_of((aabbs[6 * (size_t)i + axis] + aabbs[6 * (size_t)i + 3 + axis]) * 0.5f, A.lo[axis], A.scale[axis]) <= kbin;
+        }
         const unsigned ball = __ballot_sync(0xFFFFFFFFu, l);
         if (lane == 0) warp_sums[warp] = __popc(ball);
         __syncthreads();
-        u32t before = carry;
-        for (u32t w = 0; w < warp; w++) before += warp_sums[w];
+        u32t before = carry, sum = 0;
+        for (u32t w = 0; w < blockDim.x / 32; w++) {
+            if (w < warp) before += warp_sums[w];
+            sum += warp_sums[w];
+        }
         before += __popc(ball & ((1u << lane) - 1u));
-        if (in) {
-            const u32t lrank = left_before + before;                   // left items before k in the task
-            const u32t pos_in_task = k - T.begin;
-            const u32t dst = l ? T.begin + lrank : T.begin + d.nleft + (pos_in_task - lrank);
-            tmp[dst] = i;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) { u32t s = 0; for (u32t w = 0; w < blockDim.x / 32; w++) s += warp_sums[w]; carry += s; }
+        if (in) out[l ? L.t.begin + before : L.t.begin + s.nleft + (k - L.t.begin - before)] = i;
+        carry += sum;
         __syncthreads();
     }
-}
-__global__ void sah_copy_back_kernel(const SahTask *tasks, const u32t *large_tasks, const u32t *chunk_task,
-                                     const u32t *chunk_offsets, const u32t *tmp, u32t *ids) {
-    const u32t r = chunk_task[blockIdx.x];
-    const SahTask T = tasks[large_tasks[r]];
-    const u32t chunk = blockIdx.x - chunk_offsets[large_tasks[r]];
-    const u32t first = T.begin + chunk * kChunk, last = min(T.end, first + kChunk);
-    for (u32t k = first + threadIdx.x; k < last; k += blockDim.x) ids[k] = tmp[k];
-}
-
-// ---- small tasks: one block does binning, sweep and the stable partition in shared memory ----
-__global__ void sah_small_kernel(const SahTask *tasks, u32t nt, const u32t *flags, u32t *ids, const float *aabbs,
-                                 const float *cent, SahDecision *small_dec) {
-    const u32t t = blockIdx.x;
-    if (t >= nt) return;
-    const SahTask T = tasks[t];
-    const u32t cnt = T.end - T.begin;
-    if (!flags[t] || flags[nt + t]) return;                  // leaves and large tasks are elsewhere
-    __shared__ unsigned sb[3 * kBins * kBinWords];
-    __shared__ u32t sids[kSmall], stmp[kSmall];
-    __shared__ SahDecision sd;
-    __shared__ u32t warp_sums[8];
-    for (int k = threadIdx.x; k < 3 * kBins; k += blockDim.x) {
-        unsigned *b = sb + k * kBinWords;
-        b[0] = 0;
-        empty6(b + 1);
-        empty6(b + 7);
-    }
-    for (u32t k = threadIdx.x; k < cnt; k += blockDim.x) sids[k] = ids[T.begin + k];
+    if (chunk) return;
+    // the range's node and its children, by the block of its first chunk
+    if (tid < 2) child[tid] = kNoSplit;
+    if (tid < 12) cb[tid / 6][tid % 6] = tid % 6 < 3 ? 0xFFFFFFFFu : 0u;
+    __shared__ u32t self;
+    if (tid == 0) self = atomicAdd(&C->nodes, 1u);
     __syncthreads();
-    float lo[3], scale[3];
-    bool valid[3];
-    task_axes(T, lo, scale, valid);
-    for (u32t k = threadIdx.x; k < cnt; k += blockDim.x) {
-        const u32t i = sids[k];
-        unsigned it[6], ct[6];
-        for (int q = 0; q < 6; q++) it[q] = ob(aabbs[6 * (size_t)i + q]);
-        for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob(cent[3 * (size_t)i + q]);
-        for (int a = 0; a < 3; a++) {
-            if (!valid[a]) continue;
-            unsigned *b = sb + (a * kBins + bin_of(cent[3 * (size_t)i + a], lo[a], scale[a])) * kBinWords;
-            atomicAdd(b, 1u);
-            atomic_grow6(b + 1, it);
-            atomic_grow6(b + 7, ct);
+    if (middle)       // the children's centroid boxes from the items (rare: all centroids equal)
+        for (u32t k = L.t.begin + tid; k < L.t.end; k += blockDim.x) {
+            const u32t i = item_at(ids0, ids1, L.t.source, k);
+            unsigned ct[6];
+            for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob((aabbs[6 * (size_t)i + q] + aabbs[6 * (size_t)i + 3 + q]) * 0.5f);
+            atomic_grow6(cb[k - L.t.begin < s.nleft ? 0 : 1], ct);
         }
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        int axis, k;
-        float cost;
-        sweep(sb, valid, threadIdx.x, axis, k, cost);
-        if (threadIdx.x == 0) {
-            sd.axis = axis;
-            sd.k = k;
-            if (axis >= 0) side_boxes(sb, axis, k, sd);
-            else {
-                sd.nleft = cnt / 2;
-                empty6(sd.lbox); empty6(sd.lcbox); empty6(sd.rbox); empty6(sd.rcbox);
+    if (warp == 0) {
+        const int va = A.valid[0] ? 0 : A.valid[1] ? 1 : A.valid[2] ? 2 : 0;
+        unsigned b[6];
+        for (int q = 0; q < 6; q++) b[q] = g[(va * kBins + lane) * kBinWords + 1 + q];
+        warp_grow6(b);
+        if (lane == 0) {
+            LargeNode &o = nodes[self];
+            for (int q = 0; q < 6; q++) o.box[q] = b[q];
+            o.begin = L.t.begin; o.level = L.t.level; o.parent = L.t.parent; o.side = L.t.side;
+        }
+        if (!middle) {
+            for (int side = 0; side < 2; side++) {
+                empty6(b);
+                if ((lane <= kbin) == (side == 0))
+                    for (int q = 0; q < 6; q++) b[q] = g[(axis * kBins + lane) * kBinWords + 7 + q];
+                warp_grow6(b);
+                if (lane == 0) for (int q = 0; q < 6; q++) cb[side][q] = b[q];
             }
         }
     }
     __syncthreads();
-    if (sd.axis < 0) {  // middle split: boxes from the items
-        for (u32t k = threadIdx.x; k < cnt; k += blockDim.x) {
-            const u32t i = sids[k];
-            unsigned it[6], ct[6];
-            for (int q = 0; q < 6; q++) it[q] = ob(aabbs[6 * (size_t)i + q]);
-            for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob(cent[3 * (size_t)i + q]);
-            if (k < sd.nleft) { atomic_grow6(sd.lbox, it); atomic_grow6(sd.lcbox, ct); }
-            else { atomic_grow6(sd.rbox, it); atomic_grow6(sd.rcbox, ct); }
+    if (tid < 2) {
+        SahTask t{tid ? L.t.begin + s.nleft : L.t.begin, tid ? L.t.end : L.t.begin + s.nleft, L.t.level + 1, target, self, tid};
+        const u32t c = t.end - t.begin;
+        if (c > kCap && c > max_leaf) {
+            LargeTask N;
+            N.t = t;
+            for (int q = 0; q < 6; q++) N.cbox[q] = cb[tid][q];
+            child[tid] = atomicAdd(&C->large[now ^ 1], 1u);
+            N.chunk0 = place[tid] = atomicAdd(&C->chunks[now ^ 1], chunks_of(t));
+            next[child[tid]] = N;
+        } else if (c > kSub && c > max_leaf) {
+            mids[atomicAdd(&C->mids, 1u)] = t;
+        } else {
+            subtrees[atomicAdd(&C->subtrees, 1u)] = t;
         }
     }
-    // stable partition through shared memory
-    const u32t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    u32t carry = 0;
-    for (u32t base = 0; base < cnt; base += blockDim.x) {
-        const u32t k = base + threadIdx.x;
-        const bool in = k < cnt;
-        const u32t i = in ? sids[k] : 0;
-        const bool l = in && (sd.axis < 0 ? k < sd.nleft
-                                          : bin_of(cent[3 * (size_t)i + sd.axis], lo[sd.axis], scale[sd.axis]) <= (u32t)sd.k);
-        const unsigned ball = __ballot_sync(0xFFFFFFFFu, l);
-        if (lane == 0) warp_sums[warp] = __popc(ball);
-        __syncthreads();
-        u32t before = carry;
-        for (u32t w = 0; w < warp; w++) before += warp_sums[w];
-        before += __popc(ball & ((1u << lane) - 1u));
-        if (in) stmp[l ? before : sd.nleft + (k - before)] = i;
-        u32t s = 0;
-        for (u32t w = 0; w < blockDim.x / 32; w++) s += warp_sums[w];
-        __syncthreads();
-        carry += s;
-    }
     __syncthreads();
-    for (u32t k = threadIdx.x; k < cnt; k += blockDim.x) ids[T.begin + k] = stmp[k];
-    if (threadIdx.x == 0) small_dec[t] = sd;
-}
-
-// ---- per level: write nodes and the next level's tasks -------------------------------------------
-__global__ void sah_emit_kernel(const SahTask *tasks, u32t nt, const u32t *flags, const u32t *scanned,
-                                const SahDecision *large_dec, const SahDecision *small_dec, u32t pairs_before,
-                                u32t level, BVHNode *nodes, SahTask *next, u32t *height) {
-    u32t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt) return;
-    const SahTask T = tasks[t];
-    BVHNode &o = nodes[T.slot];
-    o.aabb.min.x = fo(T.box[0]); o.aabb.min.y = fo(T.box[1]); o.aabb.min.z = fo(T.box[2]);
-    o.aabb.max.x = fo(T.box[3]); o.aabb.max.y = fo(T.box[4]); o.aabb.max.z = fo(T.box[5]);
-    o.depth = (uint16_t)level;
-    if (!flags[t]) {
-        o.first_child_id = T.begin;
-        o.child_count = (uint16_t)(T.end - T.begin);
-        atomicMax(height, level);
-        return;
+    for (int side = 0; side < 2; side++) {
+        if (child[side] == kNoSplit) continue;
+        const u32t c = side ? cnt - s.nleft : s.nleft;
+        for (u32t k = tid; k < (c + kChunk - 1) / kChunk; k += blockDim.x) next_chunk_task[place[side] + k] = child[side];
+        clear_large_bins(next_bins + (size_t)child[side] * 3 * kBins * kBinWords, tid, blockDim.x);
     }
-    const SahDecision &d = flags[nt + t] ? large_dec[scanned[nt + t]] : small_dec[t];
-    const u32t p = scanned[t];
-    o.first_child_id = 1 + 2 * (pairs_before + p);
-    o.child_count = 0;
-    SahTask L, R;
-    L.begin = T.begin; L.end = T.begin + d.nleft; L.slot = 1 + 2 * (pairs_before + p); L.pad = 0;
-    R.begin = L.end; R.end = T.end; R.slot = L.slot + 1; R.pad = 0;
-    for (int q = 0; q < 6; q++) { L.box[q] = d.lbox[q]; L.cbox[q] = d.lcbox[q]; R.box[q] = d.rbox[q]; R.cbox[q] = d.rcbox[q]; }
-    next[2 * p] = L;
-    next[2 * p + 1] = R;
+}
+__global__ void sah_next_level_kernel(SahCounts *C, int now) { C->large[now] = C->chunks[now] = 0; }
+
+// ---- numbering --------------------------------------------------------------------------------------
+// The parts of the tree are its large nodes, one split each, and its subtrees, splits[begin + l] at
+// their level l, in order.  Sorted by where they begin, the parts of a level lie from left to right.
+__device__ __forceinline__ u32t part_begin(const LargeNode *nodes, const SahTask *subtrees, u32t nl, u32t j) {
+    return j < nl ? nodes[j].begin : subtrees[j - nl].begin;
+}
+__global__ void sah_sort_kernel(const SahCounts *C, const LargeNode *nodes, const SahTask *subtrees, u32t *sorted) {
+    __shared__ u32t begins[256];
+    const u32t nl = C->nodes, n = nl + C->subtrees;
+    for (u32t j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x) {
+        const u32t j = j0 + threadIdx.x, mine = j < n ? part_begin(nodes, subtrees, nl, j) : 0;
+        u32t before = 0;
+        for (u32t i0 = 0; i0 < n; i0 += blockDim.x) {
+            __syncthreads();
+            if (i0 + threadIdx.x < n) begins[threadIdx.x] = part_begin(nodes, subtrees, nl, i0 + threadIdx.x);
+            __syncthreads();
+            for (u32t k = 0; k < min(blockDim.x, n - i0); k++) before += begins[k] < mine || (begins[k] == mine && i0 + k < j);
+        }
+        if (j < n) sorted[before] = j;
+    }
+}
+// A block per level: rank[begin + l] (subtrees) and large_rank (large nodes) = how many of the level's
+// split nodes lie left of the part's; totals[level] = all of the level.
+__global__ void sah_rank_kernel(const SahCounts *C, const LargeNode *nodes, const SahTask *subtrees, const u32t *levels,
+                                const u32t *splits, const u32t *sorted, u32t *rank, u32t *large_rank, u32t *totals) {
+    __shared__ u32t sums[kWarps];
+    const u32t nl = C->nodes, n = nl + C->subtrees, height = C->info[1];
+    for (u32t level = blockIdx.x; level <= height; level += gridDim.x) {
+        u32t carry = 0;
+        for (u32t p0 = 0; p0 < n; p0 += kThreads) {
+            const u32t p = p0 + threadIdx.x;
+            u32t count = 0, total;
+            u32t *out = nullptr;
+            if (p < n) {
+                const u32t j = sorted[p];
+                if (j < nl) {
+                    if (nodes[j].level == level) { count = 1; out = large_rank + j; }
+                } else {
+                    const SahTask t = subtrees[j - nl];
+                    if (level >= t.level && level - t.level < levels[j - nl]) {
+                        const u32t at = t.begin + level - t.level;
+                        count = splits[at];
+                        out = rank + at;
+                    }
+                }
+            }
+            const u32t before = block_exclusive<kWarps>(count, sums, total);
+            if (out) *out = carry + before;
+            carry += total;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) totals[level] = carry;
+    }
+}
+// totals -> the pairs of the levels before; one warp
+__global__ void sah_base_kernel(SahCounts *C, u32t *totals) {
+    u32t run = 0;
+    for (u32t l0 = 0; l0 <= C->info[1]; l0 += 32) {
+        const u32t l = l0 + threadIdx.x, v = l <= C->info[1] ? totals[l] : 0;
+        u32t x = v;
+        for (int off = 1; off < 32; off <<= 1) {
+            const u32t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+            if (threadIdx.x >= (u32t)off) x += y;
+        }
+        if (l <= C->info[1]) totals[l] = run + x - v;
+        run += __shfl_sync(0xFFFFFFFFu, x, 31);
+    }
+    if (threadIdx.x == 0) C->info[2] = run;
+}
+__global__ void sah_emit_kernel(const SahCounts *C, const LargeNode *nodes, const SahTask *subtrees, const u32t *levels,
+                                const u32t *rank, const u32t *large_rank, const u32t *base, const SahRecord *records,
+                                const u32t *splits, BVHNode *out) {
+    const u32t nl = C->nodes, ns = C->subtrees;
+    auto child_slot = [&](u32t parent, u32t side) {
+        return parent == kNoSplit ? 0u : 1 + 2 * (base[nodes[parent].level] + large_rank[parent]) + side;
+    };
+    for (u32t s = blockIdx.x; s < ns; s += gridDim.x) {
+        const SahTask t = subtrees[s];
+        u32t count = 1;                                            // its nodes: the root and two per split
+        for (u32t l = 0; l < levels[s]; l++) count += 2 * splits[t.begin + l];
+        for (u32t k = threadIdx.x; k < count; k += blockDim.x) {
+            const SahRecord R = records[2 * (size_t)t.begin + k];
+            const u32t l = R.level - t.level;
+            const u32t slot = l ? 1 + 2 * (base[R.level - 1] + rank[t.begin + l - 1]) + R.index : child_slot(t.parent, t.side);
+            write_node(out[slot], R.box, R.count ? R.first : 1 + 2 * (base[R.level] + rank[t.begin + l] + R.first), R.count, R.level);
+        }
+    }
+    for (u32t j = blockIdx.x * blockDim.x + threadIdx.x; j < nl; j += gridDim.x * blockDim.x) {
+        const LargeNode N = nodes[j];
+        write_node(out[child_slot(N.parent, N.side)], N.box, 1 + 2 * (base[N.level] + large_rank[j]), 0, N.level);
+    }
 }
 
 // ---- host driver ------------------------------------------------------------------------------
-struct SahScratch {
-    size_t n = 0;
-    char *base = nullptr;
-};
-
-void scan_exclusive_u32(const u32t *in, u32t *out, u32t n, u32t *sums, u32t *total, cudaStream_t st);
-
 namespace {
 struct SahLayout {
-    size_t o_cent, o_tmp, o_ta, o_tb, o_flags, o_scan, o_sums, o_large, o_ctask, o_cleft, o_bins, o_ldec, o_sdec, o_misc;
+    size_t ids0, ids1, records, splits, rank, large_rank, totals, sorted, subtrees, levels, mids, task_a, task_b, chunk_a,
+        chunk_b, bins_a, bins_b, counts, nodes, chunk_counts;
+    u32t max_large, max_chunks;
     size_t bytes = 0;
 };
-// scratch: centroids, tmp ids, two task lists, flags/scans (3n each), large lists, bins, decisions
+// Ranges above kCap items at one level: fewer than n / kCap.  Large nodes and subtrees: a split may part
+// as little as one item from the rest, so fewer than n of either.
 SahLayout sah_layout(u32t n) {
     SahLayout L;
-    const size_t nb = n;
-    const u32t max_large = (u32t)(n / kSmall + 2);
-    const size_t max_chunks = n / kChunk + max_large + 2;
+    L.max_large = n / kCap + 2;
+    L.max_chunks = n / kChunk + L.max_large + 2;
     auto add = [&](size_t b) { size_t off = L.bytes; L.bytes += (b + 255) & ~(size_t)255; return off; };
-    L.o_cent = add(sizeof(float) * 3 * nb); L.o_tmp = add(sizeof(u32t) * nb);
-    L.o_ta = add(sizeof(SahTask) * nb); L.o_tb = add(sizeof(SahTask) * nb);
-    L.o_flags = add(sizeof(u32t) * 3 * nb + 64); L.o_scan = add(sizeof(u32t) * 3 * nb + 64);
-    L.o_sums = add(sizeof(u32t) * (3 * nb / 1024 + 64));
-    L.o_large = add(sizeof(u32t) * max_large); L.o_ctask = add(sizeof(u32t) * max_chunks);
-    L.o_cleft = add(sizeof(u32t) * max_chunks);
-    L.o_bins = add(sizeof(unsigned) * (size_t)max_large * 3 * kBins * kBinWords);
-    L.o_ldec = add(sizeof(SahDecision) * max_large); L.o_sdec = add(sizeof(SahDecision) * nb);
-    L.o_misc = add(sizeof(u32t) * 64);
+    L.counts = add(sizeof(SahCounts));
+    L.ids0 = add(sizeof(u32t) * (size_t)n);
+    L.ids1 = add(sizeof(u32t) * (size_t)n);
+    L.records = add(sizeof(SahRecord) * 2 * (size_t)n);
+    L.splits = add(sizeof(u32t) * (size_t)n);
+    L.rank = add(sizeof(u32t) * (size_t)n);
+    L.large_rank = add(sizeof(u32t) * (size_t)n);
+    L.totals = add(sizeof(u32t) * ((size_t)n + 2));
+    L.sorted = add(sizeof(u32t) * 2 * (size_t)n);
+    L.subtrees = add(sizeof(SahTask) * (size_t)n);
+    L.levels = add(sizeof(u32t) * (size_t)n);
+    L.nodes = add(sizeof(LargeNode) * (size_t)n);
+    L.mids = add(sizeof(SahTask) * (size_t)(n / kSub + 1));
+    L.task_a = add(sizeof(LargeTask) * L.max_large);
+    L.task_b = add(sizeof(LargeTask) * L.max_large);
+    L.chunk_a = add(sizeof(u32t) * L.max_chunks);
+    L.chunk_b = add(sizeof(u32t) * L.max_chunks);
+    L.bins_a = add(sizeof(unsigned) * (size_t)L.max_large * 3 * kBins * kBinWords);
+    L.bins_b = add(sizeof(unsigned) * (size_t)L.max_large * 3 * kBins * kBinWords);
+    L.chunk_counts = add(sizeof(uint16_t) * (size_t)L.max_chunks * 3 * kBins);
     return L;
 }
 }  // namespace
 
 size_t sah_scratch_bytes(u32t n) { return sah_layout(n).bytes; }
 
+bool sah_without_wait(u32t n, u32t max_leaf) { return n <= kCap || n <= max_leaf; }
+
+// The build on `st`; scratch: sah_scratch_bytes(n) bytes; *info: where the device leaves {-, height, pairs}.
+static cudaError_t sah_launch(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, char *base,
+                              u32t **info, cudaStream_t st) {
+    const SahLayout Lo = sah_layout(n);
+    SahCounts *C = (SahCounts *)(base + Lo.counts);
+    *info = C->info;
+    cudaError_t e = cudaFuncSetAttribute(sah_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MidShared));
+    if (e != cudaSuccess) return e;
+    if (n <= kSub || n <= max_leaf) {
+        sah_subtree_kernel<<<1, kThreads, 0, st>>>(aabbs, nullptr, nullptr, n, max_leaf, nullptr, nullptr, out_order, out_nodes,
+                                                   C->info, nullptr, nullptr, nullptr);
+        return cudaGetLastError();
+    }
+    u32t *ids0 = (u32t *)(base + Lo.ids0), *ids1 = (u32t *)(base + Lo.ids1);
+    SahRecord *records = (SahRecord *)(base + Lo.records);
+    u32t *splits = (u32t *)(base + Lo.splits), *rank = (u32t *)(base + Lo.rank), *totals = (u32t *)(base + Lo.totals);
+    u32t *large_rank = (u32t *)(base + Lo.large_rank), *levels = (u32t *)(base + Lo.levels), *sorted = (u32t *)(base + Lo.sorted);
+    SahTask *subtrees = (SahTask *)(base + Lo.subtrees), *mids = (SahTask *)(base + Lo.mids);
+    LargeNode *nodes = (LargeNode *)(base + Lo.nodes);
+    sah_init_kernel<<<1, 32, 0, st>>>(C);
+    if (n <= kCap) {
+        sah_mid_kernel<<<1, kMidThreads, sizeof(MidShared), st>>>(aabbs, C, nullptr, n, max_leaf, ids0, ids1, nodes,
+                                                                  subtrees);
+    } else {
+        LargeTask *task[2] = {(LargeTask *)(base + Lo.task_a), (LargeTask *)(base + Lo.task_b)};
+        u32t *chunk[2] = {(u32t *)(base + Lo.chunk_a), (u32t *)(base + Lo.chunk_b)};
+        unsigned *bins[2] = {(unsigned *)(base + Lo.bins_a), (unsigned *)(base + Lo.bins_b)};
+        uint16_t *chunk_counts = (uint16_t *)(base + Lo.chunk_counts);
+        sah_root_kernel<<<min((n + 255) / 256, 1184u), 256, 0, st>>>(aabbs, n, C);
+        sah_first_kernel<<<1, 256, 0, st>>>(n, C, task[0], chunk[0], bins[0]);
+        // the levels of the ranges above kCap: a few are enqueued between looks at how many are left
+        // (launches for a level that is not there end at once)
+        SahCounts now;
+        now.large[0] = 1;
+        for (u32t level = 0; now.large[level & 1];) {
+            for (int k = 0; k < 4; k++, level++) {
+                const int c = level & 1;
+                sah_bin_kernel<<<Lo.max_chunks, 256, 0, st>>>(aabbs, C, c, task[c], chunk[c], ids0, ids1, bins[c], chunk_counts);
+                sah_part_kernel<<<Lo.max_chunks, 256, 0, st>>>(aabbs, C, c, max_leaf, task[c], chunk[c], ids0, ids1, bins[c],
+                                                               chunk_counts, task[c ^ 1], chunk[c ^ 1], bins[c ^ 1], nodes,
+                                                               mids, subtrees);
+                sah_next_level_kernel<<<1, 1, 0, st>>>(C, c);
+            }
+            e = cudaMemcpyAsync(&now, C, sizeof(now), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) return e;
+        }
+        if (now.mids)
+            sah_mid_kernel<<<min(now.mids, 1184u), kMidThreads, sizeof(MidShared), st>>>(aabbs, C, mids, n, max_leaf, ids0, ids1,
+                                                                                      nodes, subtrees);
+    }
+    // few subtrees for every block of these grids to have one, or more than one for each: both are loops
+    const u32t grid = min(max(n / 128, 1u), 1184u);
+    sah_subtree_kernel<<<grid, kThreads, 0, st>>>(aabbs, C, subtrees, n, max_leaf, ids0, ids1, out_order, nullptr, C->info,
+                                                  records, splits, levels);
+    sah_sort_kernel<<<min(max(n / 4096, 1u), 148u), 256, 0, st>>>(C, nodes, subtrees, sorted);
+    sah_rank_kernel<<<64, kThreads, 0, st>>>(C, nodes, subtrees, levels, splits, sorted, rank, large_rank, totals);
+    sah_base_kernel<<<1, 32, 0, st>>>(C, totals);
+    sah_emit_kernel<<<grid, 128, 0, st>>>(C, nodes, subtrees, levels, rank, large_rank, totals, records, splits, out_nodes);
+    return cudaGetLastError();
+}
+
+cudaError_t sah_enqueue(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, void *scratch,
+                        u32t *counts, cudaStream_t st) {
+    u32t *info;
+    const cudaError_t e = sah_launch(aabbs, n, max_leaf, out_nodes, out_order, static_cast<char *>(scratch), &info, st);
+    return e != cudaSuccess ? e : cudaMemcpyAsync(counts, info, sizeof(u32t) * 3, cudaMemcpyDeviceToHost, st);
+}
+
 cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t info[2],
                       cudaStream_t st, void *scratch, size_t scratch_bytes) {
     if (n == 0) { info[0] = info[1] = 0; return cudaSuccess; }
-    const SahLayout Lo = sah_layout(n);
-    const size_t o_cent = Lo.o_cent, o_tmp = Lo.o_tmp, o_ta = Lo.o_ta, o_tb = Lo.o_tb, o_flags = Lo.o_flags,
-                 o_scan = Lo.o_scan, o_sums = Lo.o_sums, o_large = Lo.o_large, o_ctask = Lo.o_ctask,
-                 o_cleft = Lo.o_cleft, o_bins = Lo.o_bins, o_ldec = Lo.o_ldec, o_sdec = Lo.o_sdec, o_misc = Lo.o_misc;
+    const size_t bytes = sah_scratch_bytes(n);
     // the caller's scratch when it is large enough, else a stream-ordered allocation
-    char *base = nullptr;
-    const bool own = !(scratch && scratch_bytes >= Lo.bytes);
+    void *base = scratch;
+    const bool own = !(scratch && scratch_bytes >= bytes);
     cudaError_t e = cudaSuccess;
-    if (own) e = cudaMallocAsync((void **)&base, Lo.bytes, st);
-    else base = static_cast<char *>(scratch);
+    if (own) e = cudaMallocAsync(&base, bytes, st);
     if (e != cudaSuccess) return e;
-    float *cent = (float *)(base + o_cent);
-    u32t *tmp = (u32t *)(base + o_tmp);
-    SahTask *cur = (SahTask *)(base + o_ta), *next = (SahTask *)(base + o_tb);
-    u32t *flags = (u32t *)(base + o_flags), *scanned = (u32t *)(base + o_scan), *sums = (u32t *)(base + o_sums);
-    u32t *large = (u32t *)(base + o_large), *ctask = (u32t *)(base + o_ctask), *cleft = (u32t *)(base + o_cleft);
-    unsigned *bins = (unsigned *)(base + o_bins);
-    SahDecision *ldec = (SahDecision *)(base + o_ldec), *sdec = (SahDecision *)(base + o_sdec);
-    u32t *misc = (u32t *)(base + o_misc);   // [0..12) root bits, [16..20) totals, [20] height
-    u32t *ids = out_order;
-
-    sah_root_init_kernel<<<1, 32, 0, st>>>(misc);
-    sah_setup_kernel<<<min((n + 255) / 256, 1184u), 256, 0, st>>>(aabbs, n, cent, ids, misc);
-    sah_root_task_kernel<<<1, 1, 0, st>>>(misc, n, cur);
-    cudaMemsetAsync(misc + 20, 0, sizeof(u32t), st);
-    u32t nt = 1, pairs = 0, level = 0;
-    while (nt) {
-        const u32t T = 256;
-        sah_classify_kernel<<<(nt + T - 1) / T, T, 0, st>>>(cur, nt, max_leaf, flags);
-        scan_exclusive_u32(flags, scanned, nt, sums, misc + 16, st);
-        scan_exclusive_u32(flags + nt, scanned + nt, nt, sums, misc + 17, st);
-        scan_exclusive_u32(flags + 2 * nt, scanned + 2 * nt, nt, sums, misc + 18, st);
-        u32t tot[3];
-        cudaMemcpyAsync(tot, misc + 16, sizeof(tot), cudaMemcpyDeviceToHost, st);
-        e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) break;
-        const u32t nsplit = tot[0], nlarge = tot[1], nchunks = tot[2];
-        if (nlarge) {
-            sah_large_list_kernel<<<(nt + T - 1) / T, T, 0, st>>>(cur, nt, flags, scanned, large, ctask);
-            sah_clear_bins_kernel<<<(nlarge * 3 * kBins + T - 1) / T, T, 0, st>>>(bins, nlarge);
-            sah_bin_large_kernel<<<nchunks, 256, 0, st>>>(cur, large, ctask, scanned + 2 * nt, ids, aabbs, cent, bins);
-            sah_split_large_kernel<<<(nlarge + 3) / 4, 128, 0, st>>>(cur, large, nlarge, bins, ldec);
-            sah_middle_boxes_kernel<<<nchunks, 256, 0, st>>>(cur, large, ctask, scanned + 2 * nt, ids, aabbs, cent, ldec);
-            sah_count_left_kernel<<<nchunks, 256, 0, st>>>(cur, large, ctask, scanned + 2 * nt, ids, cent, ldec, cleft);
-            sah_chunk_scan_kernel<<<(nlarge + T - 1) / T, T, 0, st>>>(large, nlarge, scanned + 2 * nt, flags, nt, cleft);
-            sah_scatter_kernel<<<nchunks, 256, 0, st>>>(cur, large, ctask, scanned + 2 * nt, ids, cent, ldec, cleft, tmp);
-            sah_copy_back_kernel<<<nchunks, 256, 0, st>>>(cur, large, ctask, scanned + 2 * nt, tmp, ids);
-        }
-        sah_small_kernel<<<nt, 256, 0, st>>>(cur, nt, flags, ids, aabbs, cent, sdec);
-        sah_emit_kernel<<<(nt + T - 1) / T, T, 0, st>>>(cur, nt, flags, scanned, ldec, sdec, pairs, level, out_nodes, next,
-                                                       misc + 20);
-        pairs += nsplit;
-        nt = 2 * nsplit;
-        SahTask *sw = cur; cur = next; next = sw;
-        level++;
-    }
-    u32t h = 0;
-    if (e == cudaSuccess) {
-        cudaMemcpyAsync(&h, misc + 20, sizeof(u32t), cudaMemcpyDeviceToHost, st);
-        e = cudaStreamSynchronize(st);
-    }
+    u32t got[3] = {0, 0, 0};
+    e = sah_enqueue(aabbs, n, max_leaf, out_nodes, out_order, base, got, st);
     if (own) cudaFreeAsync(base, st);
-    cudaError_t e2 = cudaStreamSynchronize(st);
-    info[0] = 1 + 2 * pairs;
-    info[1] = h < 1 ? 1 : h;
+    const cudaError_t e2 = cudaStreamSynchronize(st);
+    info[0] = 1 + 2 * got[2];
+    info[1] = got[1] < 1 ? 1 : got[1];
     return e != cudaSuccess ? e : e2;
 }
 
