@@ -32,7 +32,7 @@ struct DevBuf {
 // The arrays a transform update rewrites: primitive records and the TLAS.  The serving loop gives a
 // scene a fresh copy of them when batches still in flight read the current one (scene versions).
 struct MotionBufs {
-    DevBuf prims_raw, prims, tlas_nodes, tlas_leaf_ids, tlas_pairs, tlas_aabbs, tlas_scratch;
+    DevBuf prims_raw, prims, tlas_nodes, tlas_leaf_ids, tlas_pairs, tlas_scratch;
 };
 
 struct SceneSlot {
@@ -41,7 +41,7 @@ struct SceneSlot {
     u32t cap_prims = 0, cap_materials = 0, cap_lights = 0, cap_tris = 0, cap_meshes = 0, cap_mips = 0;
     size_t cap_quads = 0;
     DevBuf prims_raw, prims, materials, lights;
-    DevBuf tlas_nodes, tlas_leaf_ids, tlas_pairs, tlas_aabbs, tlas_scratch;
+    DevBuf tlas_nodes, tlas_leaf_ids, tlas_pairs, tlas_scratch;
     u32t tlas_node_count = 0, tlas_height = 0;
     u32t moved_since_build = 0;            // primitives moved since the TLAS was last built in full
     bool tlas_valid = false;
@@ -62,8 +62,8 @@ struct SceneSlot {
 };
 
 DevBuf *motion_field(SceneSlot &S, MotionBufs &m, int k, DevBuf **mine) {
-    DevBuf *a[7] = {&S.prims_raw, &S.prims, &S.tlas_nodes, &S.tlas_leaf_ids, &S.tlas_pairs, &S.tlas_aabbs, &S.tlas_scratch};
-    DevBuf *b[7] = {&m.prims_raw, &m.prims, &m.tlas_nodes, &m.tlas_leaf_ids, &m.tlas_pairs, &m.tlas_aabbs, &m.tlas_scratch};
+    DevBuf *a[6] = {&S.prims_raw, &S.prims, &S.tlas_nodes, &S.tlas_leaf_ids, &S.tlas_pairs, &S.tlas_scratch};
+    DevBuf *b[6] = {&m.prims_raw, &m.prims, &m.tlas_nodes, &m.tlas_leaf_ids, &m.tlas_pairs, &m.tlas_scratch};
     *mine = a[k];
     return b[k];
 }
@@ -284,7 +284,6 @@ int allocate(st_ctx *ctx, SceneSlot &S, const Scene *scene) {
     ST_TRY(reserve(ctx, S.tlas_nodes, sizeof(BVHNode) * 2 * std::max(np, 1u)));
     ST_TRY(reserve(ctx, S.tlas_leaf_ids, sizeof(u32t) * std::max(np, 1u)));
     ST_TRY(reserve(ctx, S.tlas_pairs, sizeof(NodePair) * std::max(np, 1u)));
-    ST_TRY(reserve(ctx, S.tlas_aabbs, sizeof(float) * 6 * std::max(np, 1u)));
     ST_TRY(reserve(ctx, S.tlas_scratch, (sizeof(u32t) * 2 + sizeof(unsigned) * 6) * 2 * std::max(np, 1u)));
     ST_TRY(reserve(ctx, S.meshes, sizeof(MeshDev) * std::max(nmesh, 1u)));
     ST_TRY(reserve(ctx, S.mesh_pairs, sizeof(NodePair) * std::max(nt, 1u)));
@@ -459,12 +458,12 @@ int st_free_scene(st_ctx *ctx, int slot) {
     SceneSlot *S = slot_of(ctx, slot);
     if (!S) return ST_ERR_INVALID_ARG;
     for (DevBuf *b : {&S->prims_raw, &S->prims, &S->materials, &S->lights, &S->tlas_nodes, &S->tlas_leaf_ids,
-                      &S->tlas_pairs, &S->tlas_aabbs, &S->tlas_scratch, &S->meshes, &S->mesh_pairs, &S->tri_hot,
+                      &S->tlas_pairs, &S->tlas_scratch, &S->meshes, &S->mesh_pairs, &S->tri_hot,
                       &S->tri_full, &S->textures, &S->mips, &S->quads, &S->emissive, &S->occluders, &S->outlines,
                       &S->outline_ranges})
         release(ctx, *b);
     for (MotionBufs &m : S->spare)
-        for (int k = 0; k < 7; k++) {
+        for (int k = 0; k < 6; k++) {
             DevBuf *mine;
             release(ctx, *motion_field(*S, m, k, &mine));
         }
@@ -768,14 +767,19 @@ int st_update_scene_bvh(st_ctx *ctx, int slot, Scene *scene, int mode) {
     return status;
 }
 
-// An LBVH30 TLAS update, and a binned-SAH one that needs no host on the way, waits once: the build's counts, its
-// nodes (at most 2n - 1) and its leaf order come back together into page-locked staging, are checked
-// there and, when the host scene has BVH arrays, copied into them from there (the other modes wait for
-// the build, the check and the copy one after another).
-static int update_scene_once(st_ctx *ctx, SceneSlot *S, Scene *scene, bool sah) {
-    const u32t n = S->n_prims;
-    cudaStream_t st = ctx->stream;
-    if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
+// The device address of a page-locked (pinned or registered) host buffer, or null for pageable
+// memory, which the device cannot write.
+static void *device_view_of_host(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+}
+
+// Page-locked staging of a TLAS update: counts and root, and the nodes and leaf ids of n primitives.
+static int tlas_staging(st_ctx *ctx, u32t n, TlasStaging &t) {
     const size_t node_bytes = sizeof(BVHNode) * 2 * (size_t)n, need = 64 + node_bytes + sizeof(u32t) * (size_t)n;
     if (need > ctx->bvh_pinned_cap) {
         if (ctx->bvh_pinned) cudaFreeHost(ctx->bvh_pinned);
@@ -784,52 +788,76 @@ static int update_scene_once(st_ctx *ctx, SceneSlot *S, Scene *scene, bool sah) 
         ST_CUDA(cudaHostAlloc((void **)&ctx->bvh_pinned, need, cudaHostAllocDefault));
         ctx->bvh_pinned_cap = need;
     }
-    u32t *counts = reinterpret_cast<u32t *>(ctx->bvh_pinned);
-    BVHNode *nodes = reinterpret_cast<BVHNode *>(ctx->bvh_pinned + 64);
-    u32t *ids = reinterpret_cast<u32t *>(ctx->bvh_pinned + 64 + node_bytes);
-    launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, st);
-    if (sah) {
-        ST_TRY(reserve(ctx, ctx->sah_scratch, sah_scratch_bytes(n)));
-        ST_CUDA(sah_enqueue(ctx->lbvh.aabbs, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes),
-                            P<u32t>(S->tlas_leaf_ids), ctx->sah_scratch.ptr, counts, st));
+    char *dev = static_cast<char *>(device_view_of_host(ctx->bvh_pinned));
+    if (!dev) return ST_ERR_CUDA;
+    t.counts = reinterpret_cast<u32t *>(dev);
+    t.root = reinterpret_cast<BVHNode *>(dev + 32);
+    t.nodes = reinterpret_cast<BVHNode *>(dev + 64);
+    t.ids = reinterpret_cast<u32t *>(dev + 64 + node_bytes);
+    return ST_OK;
+}
+
+// A TLAS update that needs no host on the way (LBVH30, a binned SAH of few primitives, a refit) waits
+// once: the last kernels make the node pairs, check a new tree, and write what the host reads - the
+// counts, the root and, for a host scene with BVH arrays, nodes and leaf order - into page-locked
+// staging.  The other builds wait for the build, the check and the copies one after another.
+static int update_scene_once(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode) {
+    const u32t n = S->n_prims;
+    cudaStream_t st = ctx->stream;
+    const bool refit = mode == ST_BVH_REFIT, host = scene && scene->bvh.nodes && scene->bvh.leaf_ids;
+    if (!refit && lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
+    TlasStaging t;
+    ST_TRY(tlas_staging(ctx, n, t));
+    if (!host) {
+        t.nodes = nullptr;
+        t.ids = nullptr;
+    }
+    u32t *counts = reinterpret_cast<u32t *>(ctx->bvh_pinned), *info = nullptr;
+    counts[3] = 0;
+    BVHNode *dev_nodes = P<BVHNode>(S->tlas_nodes);
+    u32t *dev_ids = P<u32t>(S->tlas_leaf_ids), *words = P<u32t>(S->tlas_scratch);
+    if (refit) {
+        ST_CUDA(refit_bvh(dev_nodes, S->tlas_node_count, dev_ids, P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), words,
+                          words + 2 * n, words + 4 * n, st));
     } else {
-        lbvh_enqueue(ctx->lbvh, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes), P<u32t>(S->tlas_leaf_ids),
-                     counts, st);
-        ST_CUDA(cudaGetLastError());
+        launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, st);
+        if (mode == ST_BVH_BINNED_SAH) {
+            ST_TRY(reserve(ctx, ctx->sah_scratch, sah_scratch_bytes(n)));
+            ST_CUDA(sah_enqueue(ctx->lbvh.aabbs, n, MAX_OBJS_PER_SCENE_BVH_NODE, dev_nodes, dev_ids, ctx->sah_scratch.ptr, &info, st));
+        } else {
+            info = ctx->lbvh.info;
+            ST_CUDA(lbvh_enqueue(ctx->lbvh, n, MAX_OBJS_PER_SCENE_BVH_NODE, dev_nodes, dev_ids, st));
+        }
     }
-    ST_CUDA(cudaMemcpyAsync(nodes, S->tlas_nodes.ptr, node_bytes - sizeof(BVHNode), cudaMemcpyDeviceToHost, st));
-    ST_CUDA(cudaMemcpyAsync(ids, S->tlas_leaf_ids.ptr, sizeof(u32t) * n, cudaMemcpyDeviceToHost, st));
+    launch_tlas_finish(dev_nodes, info, S->tlas_node_count, dev_ids, n, P<NodePair>(S->tlas_pairs), refit ? nullptr : words, t, st);
+    ST_CUDA(cudaGetLastError());
     ST_TRY(ST_CUDA_SYNC(ctx));
-    const u32t count = 1 + 2 * counts[2], height = counts[1];
-    // the walk trusts every index it reads: check the new arrays before first use
-    if (count > 2 * n - 1 || height + 2 > (u32t)kStack) return ST_ERR_BAD_SCENE;
-    if (!check_bvh(nodes, count, n, height)) return ST_ERR_BAD_SCENE;
-    for (u32t i = 0; i < n; i++) if (ids[i] >= n) return ST_ERR_BAD_SCENE;
-    S->tlas_node_count = count;
-    S->tlas_height = height;
-    if (count > 1) {
-        launch_make_pairs(P<BVHNode>(S->tlas_nodes), count, P<NodePair>(S->tlas_pairs), st);
-        ST_CUDA(cudaGetLastError());
+    if (!refit) {
+        // the walk trusts every index it reads: a new tree is used only if it was found to be one
+        const u32t count = 1 + 2 * counts[2], height = counts[1];
+        if (counts[3] || count > 2 * n - 1 || height + 2 > (u32t)kStack) return ST_ERR_BAD_SCENE;
+        S->tlas_node_count = count;
+        S->tlas_height = height;
+        S->moved_since_build = 0;
     }
-    S->tlas_root = nodes[0];
+    memcpy(&S->tlas_root, ctx->bvh_pinned + 32, sizeof(BVHNode));
     S->tlas_valid = true;
-    S->moved_since_build = 0;
-    if (scene && scene->bvh.nodes && scene->bvh.leaf_ids) {
-        memcpy(scene->bvh.nodes, nodes, sizeof(BVHNode) * count);
-        memcpy(scene->bvh.leaf_ids, ids, sizeof(u32t) * n);
-        scene->bvh.node_count = count;
-        scene->bvh.height = height;
+    if (host) {
+        memcpy(scene->bvh.nodes, ctx->bvh_pinned + 64, sizeof(BVHNode) * S->tlas_node_count);
+        memcpy(scene->bvh.leaf_ids, ctx->bvh_pinned + 64 + sizeof(BVHNode) * 2 * (size_t)n, sizeof(u32t) * n);
+        scene->bvh.node_count = S->tlas_node_count;
+        scene->bvh.height = S->tlas_height;
     }
     return ST_OK;
 }
 
 static int update_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode) {
     const u32t n = S->n_prims;
-    if (mode == ST_BVH_LBVH30) {
-        return update_scene_once(ctx, S, scene, false);
-    } else if (mode == ST_BVH_BINNED_SAH && sah_without_wait(n, MAX_OBJS_PER_SCENE_BVH_NODE)) {
-        return update_scene_once(ctx, S, scene, true);
-    } else if (mode == ST_BVH_BINNED_SAH) {
+    if (mode == ST_BVH_REFIT && !S->tlas_valid) return ST_ERR_NOT_RESIDENT;
+    if (mode == ST_BVH_LBVH30 || mode == ST_BVH_REFIT ||
+        (mode == ST_BVH_BINNED_SAH && sah_without_wait(n, MAX_OBJS_PER_SCENE_BVH_NODE)))
+        return update_scene_once(ctx, S, scene, mode);
+    if (mode == ST_BVH_BINNED_SAH) {
         if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
         launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, ctx->stream);
         u32t info[2];
@@ -849,21 +877,11 @@ static int update_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode) {
         if (e != cudaSuccess) return fail_cuda(ctx, e);
         S->tlas_node_count = info[0];
         S->tlas_height = info[1];
-    } else if (mode == ST_BVH_REFIT) {
-        if (!S->tlas_valid) return ST_ERR_NOT_RESIDENT;
-        launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, P<float>(S->tlas_aabbs), ctx->stream);
-        u32t *par = P<u32t>(S->tlas_scratch);
-        u32t *arr = par + 2 * n;
-        unsigned *box = reinterpret_cast<unsigned *>(arr + 2 * n);
-        cudaError_t e = refit_bvh(P<BVHNode>(S->tlas_nodes), S->tlas_node_count, P<u32t>(S->tlas_leaf_ids),
-                                  P<float>(S->tlas_aabbs), par, arr, box, ctx->stream);
-        if (e != cudaSuccess) return fail_cuda(ctx, e);
     } else {
         return ST_ERR_INVALID_ARG;
     }
-    // the walk trusts every index it reads: check a newly built array before first use (a refit
-    // rewrites boxes only, so the topology checked when it was built still holds)
-    if (mode != ST_BVH_REFIT) {
+    // the walk trusts every index it reads: check a newly built array before first use
+    {
         std::vector<BVHNode> host(S->tlas_node_count);
         std::vector<u32t> ids(n);
         ST_CUDA(cudaMemcpyAsync(host.data(), S->tlas_nodes.ptr, sizeof(BVHNode) * host.size(), cudaMemcpyDeviceToHost, ctx->stream));
@@ -873,7 +891,7 @@ static int update_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode) {
         for (u32t i = 0; i < n; i++) if (ids[i] >= n) return ST_ERR_BAD_SCENE;
     }
     ST_TRY(finish_tlas(ctx, *S));
-    if (mode != ST_BVH_REFIT) S->moved_since_build = 0;
+    S->moved_since_build = 0;
     if (scene && scene->bvh.nodes && scene->bvh.leaf_ids) {
         ST_CUDA(cudaMemcpyAsync(scene->bvh.nodes, S->tlas_nodes.ptr, sizeof(BVHNode) * S->tlas_node_count, cudaMemcpyDeviceToHost, ctx->stream));
         ST_CUDA(cudaMemcpyAsync(scene->bvh.leaf_ids, S->tlas_leaf_ids.ptr, sizeof(u32t) * n, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1014,17 +1032,6 @@ static int make_view(const Viewport *vp, ViewDev &v) {
     v.depth = vp->trace.depth;
     v.primary_tlas = 0;
     return ST_OK;
-}
-
-// The device address of a page-locked (pinned or registered) host buffer, or null for pageable
-// memory, which the device cannot write.
-static void *device_view_of_host(const void *p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
 static SceneDev scene_view(SceneSlot &S, const Scene *scene) {
@@ -1928,7 +1935,7 @@ int new_scene_version(st_ctx *ctx, int slot) {
         m = S->spare.back();
         S->spare.pop_back();
     }
-    for (int k = 0; k < 7; k++) {
+    for (int k = 0; k < 6; k++) {
         DevBuf *mine;
         DevBuf *copy = motion_field(*S, m, k, &mine);
         if (!mine->ptr) continue;
@@ -1939,7 +1946,7 @@ int new_scene_version(st_ctx *ctx, int slot) {
         }
         ST_CUDA(cudaMemcpyAsync(copy->ptr, mine->ptr, mine->bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    for (int k = 0; k < 7; k++) {
+    for (int k = 0; k < 6; k++) {
         DevBuf *mine;
         DevBuf *copy = motion_field(*S, m, k, &mine);
         std::swap(*mine, *copy);
@@ -2200,7 +2207,7 @@ int st_serve_start(st_ctx *ctx, const st_serve_config *cfg) {
         if (!S.allocated || !S.tlas_valid) continue;
         while ((int)S.spare.size() < V.cfg.max_in_flight) {
             MotionBufs m;
-            for (int k = 0; k < 7; k++) {
+            for (int k = 0; k < 6; k++) {
                 DevBuf *mine;
                 DevBuf *copy = motion_field(S, m, k, &mine);
                 if (mine->ptr) ST_TRY(reserve(ctx, *copy, mine->bytes));

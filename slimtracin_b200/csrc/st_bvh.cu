@@ -36,10 +36,7 @@ __device__ __forceinline__ v3 prim_to_world(v3 pos, const Primitive &p) {   // c
     return pos;
 }
 
-__global__ void prim_aabbs_kernel(const Primitive *prims, const MeshDev *meshes, u32t n, float *aabbs) {
-    u32t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const Primitive p = prims[i];
+__device__ __forceinline__ void prim_box(const Primitive &p, const MeshDev *meshes, float *o) {
     float lo[3], hi[3];
     if (p.type == PrimitiveType_Mesh) {
         const MeshDev &m = meshes[p.id];
@@ -60,8 +57,11 @@ __global__ void prim_aabbs_kernel(const Primitive *prims, const MeshDev *meshes,
         if (q.y < y) y = q.y;
         if (q.z < z) z = q.z;
     }
-    float *o = aabbs + 6 * (size_t)i;
     o[0] = x; o[1] = y; o[2] = z; o[3] = X; o[4] = Y; o[5] = Z;
+}
+__global__ void prim_aabbs_kernel(const Primitive *prims, const MeshDev *meshes, u32t n, float *aabbs) {
+    u32t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) prim_box(prims[i], meshes, aabbs + 6 * (size_t)i);
 }
 
 __global__ void tri_aabbs_kernel(const vec3 *pos, const uint32_t *idx, u32t n, float *aabbs) {
@@ -124,11 +124,8 @@ __device__ __forceinline__ u32t quantize(float c, float lo, float scale) {
     if (t >= 1023.0f) return 1023;
     return (u32t)t;
 }
-__global__ void morton_kernel(const float *aabbs, u32t n, const unsigned *b, u32t *codes, u32t *order) {
-    u32t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__device__ __forceinline__ u32t morton_code(const float *a, const unsigned *b) {
     u32t q[3];
-    const float *a = aabbs + 6 * (size_t)i;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         float lo = from_ord(b[k]), hi = from_ord(b[3 + k]);
@@ -137,7 +134,12 @@ __global__ void morton_kernel(const float *aabbs, u32t n, const unsigned *b, u32
         float c = (a[k] + a[3 + k]) * 0.5f;
         q[k] = quantize(c, lo, scale);
     }
-    codes[i] = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
+    return (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
+}
+__global__ void morton_kernel(const float *aabbs, u32t n, const unsigned *b, u32t *codes, u32t *order) {
+    u32t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    codes[i] = morton_code(aabbs + 6 * (size_t)i, b);
     order[i] = i;
 }
 
@@ -271,16 +273,17 @@ int radix_sort_pairs(u32t *k0, u32t *v0, u32t *k1, u32t *v1, u32t n, int passes,
 }
 
 // ---- Karras topology ------------------------------------------------------------------------------
-__device__ __forceinline__ int delta(const u32t *codes, const u32t *order, u32t n, int i, int j) {
+template <class Order>
+__device__ __forceinline__ int delta(const u32t *codes, const Order *order, u32t n, int i, int j) {
     if (j < 0 || j >= (int)n) return -1;
     unsigned long long a = ((unsigned long long)codes[i] << 32) | order[i];
     unsigned long long b = ((unsigned long long)codes[j] << 32) | order[j];
     return __clzll(a ^ b);
 }
-__global__ void karras_kernel(const u32t *codes, const u32t *order, u32t n, u32t *first, u32t *last, u32t *lchild,
-                              u32t *rchild, u32t *parent, u32t *leaf_parent) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int)n - 1) return;
+// Internal node i: the leaves it covers and its children (leaves marked with the storage's top bit).
+struct KarrasNode { u32t first, last, split; bool left_leaf, right_leaf; };
+template <class Order>
+__device__ __forceinline__ KarrasNode karras_node(const u32t *codes, const Order *order, u32t n, int i) {
     int d = (delta(codes, order, n, i, i + 1) - delta(codes, order, n, i, i - 1)) > 0 ? 1 : -1;
     int dmin = delta(codes, order, n, i, i - d);
     int lmax = 2;
@@ -296,15 +299,25 @@ __global__ void karras_kernel(const u32t *codes, const u32t *order, u32t n, u32t
         if (t == 1) break;
     }
     int g = i + s * d + (d < 0 ? -1 : 0);
-    int lo = min(i, j), hi = max(i, j);
-    first[i] = lo;
-    last[i] = hi;
-    u32t lc = (lo == g) ? (0x80000000u | (u32t)g) : (u32t)g;
-    u32t rc = (hi == g + 1) ? (0x80000000u | (u32t)(g + 1)) : (u32t)(g + 1);
-    lchild[i] = lc;
-    rchild[i] = rc;
-    if (lc & 0x80000000u) leaf_parent[lc & 0x7FFFFFFFu] = i; else parent[lc] = i;
-    if (rc & 0x80000000u) leaf_parent[rc & 0x7FFFFFFFu] = i; else parent[rc] = i;
+    KarrasNode k;
+    k.first = min(i, j);
+    k.last = max(i, j);
+    k.split = g;
+    k.left_leaf = (int)k.first == g;
+    k.right_leaf = (int)k.last == g + 1;
+    return k;
+}
+__global__ void karras_kernel(const u32t *codes, const u32t *order, u32t n, u32t *first, u32t *last, u32t *lchild,
+                              u32t *rchild, u32t *parent, u32t *leaf_parent) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (int)n - 1) return;
+    const KarrasNode k = karras_node(codes, order, n, i);
+    first[i] = k.first;
+    last[i] = k.last;
+    lchild[i] = k.split | (k.left_leaf ? 0x80000000u : 0u);
+    rchild[i] = (k.split + 1) | (k.right_leaf ? 0x80000000u : 0u);
+    (k.left_leaf ? leaf_parent : parent)[k.split] = i;
+    (k.right_leaf ? leaf_parent : parent)[k.split + 1] = i;
     if (i == 0) parent[0] = 0xFFFFFFFFu;
 }
 __global__ void keep_flags_kernel(const u32t *first, const u32t *last, u32t ni, u32t max_leaf, u32t *flags) {
@@ -374,7 +387,7 @@ __global__ void layout_kernel(const float *aabbs, const u32t *order, u32t ni, co
     }
     atomicMax(height, dep + 1);
 }
-__global__ void single_leaf_kernel(const float *aabbs, const u32t *order, u32t n, BVHNode *out) {
+__global__ void single_leaf_kernel(const float *aabbs, const u32t *order, u32t n, BVHNode *out, u32t *info) {
     unsigned b[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0, 0, 0};
     for (u32t i = 0; i < n; i++) {
         unsigned c[6];
@@ -382,6 +395,197 @@ __global__ void single_leaf_kernel(const float *aabbs, const u32t *order, u32t n
         for (int k = 0; k < 3; k++) { b[k] = min(b[k], c[k]); b[3 + k] = max(b[3 + k], c[3 + k]); }
     }
     write_node(out[0], b, 0, n, 0);
+    info[1] = 1;
+    info[2] = 0;
+}
+
+// ---- small builds: the whole LBVH30 by one block ----------------------------------------------------
+// The same steps as the kernels above, at most kBlockItems items, codes, order and topology in shared
+// memory (the boxes of internal nodes stay in kbox, read and written through L2).  A small build is
+// launches and their gaps, thirty of them: 173 us for 100 primitives, 218 for 1000, 257 for 4096 as
+// st_update_scene_bvh sees it, against 41, 70 and 168 with one (and tlas_finish_kernel below); above
+// 4096 items the shared arrays no longer fit and many blocks are faster than one.
+constexpr u32t kBlockItems = 4096;
+constexpr int kBlockThreads = 1024, kBlockWarps = kBlockThreads / 32;
+struct LbvhShared {
+    u32t code[2][kBlockItems];
+    u32t count[kBlockWarps][256];      // a pass' digit counts per warp; afterwards the nodes' arrivals
+    uint16_t item[2][kBlockItems];
+    uint16_t left[kBlockItems], right[kBlockItems], parent[kBlockItems], leaf_parent[kBlockItems];   // leaves: top bit
+    uint16_t first[kBlockItems], last[kBlockItems], rank[kBlockItems];
+    unsigned bounds[6];
+    u32t sums[kBlockWarps], height;
+};
+static_assert(sizeof(LbvhShared) <= 227 * 1024 && kBlockItems <= 0x8000 && kBlockItems <= kBlockWarps * 256, "");
+// The sum of the values of the threads before this one, and of all.
+__device__ __forceinline__ u32t block_exclusive_1024(u32t v, u32t *sums, u32t &total) {
+    const u32t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u32t x = v;
+    for (int off = 1; off < 32; off <<= 1) {
+        const u32t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+        if (lane >= (u32t)off) x += y;
+    }
+    if (lane == 31) sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        u32t w = sums[lane];
+        for (int off = 1; off < 32; off <<= 1) {
+            const u32t y = __shfl_up_sync(0xFFFFFFFFu, w, off);
+            if (lane >= (u32t)off) w += y;
+        }
+        sums[lane] = w;
+    }
+    __syncthreads();
+    total = sums[kBlockWarps - 1];
+    const u32t r = (warp ? sums[warp - 1] : 0) + x - v;
+    __syncthreads();
+    return r;
+}
+__global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const float *aabbs, u32t n, u32t max_leaf, u32t *codes,
+                                                                      u32t *order, u32t *out_order, unsigned *kbox,
+                                                                      BVHNode *out, u32t *info) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    LbvhShared &S = *reinterpret_cast<LbvhShared *>(raw);
+    const u32t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // bounds and codes
+    if (tid < 6) S.bounds[tid] = tid < 3 ? 0xFFFFFFFFu : 0u;
+    if (tid == 0) S.height = 0;
+    __syncthreads();
+    unsigned lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0, 0, 0};
+    for (u32t i = tid; i < n; i += kBlockThreads)
+        for (int k = 0; k < 3; k++) {
+            lo[k] = min(lo[k], ord_bits(aabbs[6 * i + k]));
+            hi[k] = max(hi[k], ord_bits(aabbs[6 * i + 3 + k]));
+        }
+    for (int k = 0; k < 3; k++) {
+        lo[k] = __reduce_min_sync(0xFFFFFFFFu, lo[k]);
+        hi[k] = __reduce_max_sync(0xFFFFFFFFu, hi[k]);
+        if (lane == 0) { atomicMin(S.bounds + k, lo[k]); atomicMax(S.bounds + 3 + k, hi[k]); }
+    }
+    __syncthreads();
+    for (u32t i = tid; i < n; i += kBlockThreads) {
+        S.code[0][i] = morton_code(aabbs + 6 * i, S.bounds);
+        S.item[0][i] = (uint16_t)i;
+    }
+    // stable radix sort, four passes of 8 bits: a warp takes consecutive keys, 32 at a time
+    const u32t per_warp = ((n + kBlockWarps - 1) / kBlockWarps + 31) & ~31u;
+    const u32t k0 = min(warp * per_warp, n), k1 = min(k0 + per_warp, n);
+    for (int pass = 0; pass < 4; pass++) {
+        const u32t *kin = S.code[pass & 1];
+        const uint16_t *vin = S.item[pass & 1];
+        for (u32t d = lane; d < 256; d += 32) S.count[warp][d] = 0;
+        __syncthreads();
+        for (u32t k = k0; k < k1; k += 32) {
+            const bool in = k + lane < k1;
+            const u32t d = in ? (kin[k + lane] >> (8 * pass)) & 255u : 256u;
+            const u32t peers = __match_any_sync(0xFFFFFFFFu, d);
+            if (in && lane == (u32t)__ffs(peers) - 1) S.count[warp][d] += __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        // counts -> where each warp's keys of each digit go
+        u32t run = 0, total;
+        if (tid < 256) for (int w = 0; w < kBlockWarps; w++) run += S.count[w][tid];
+        u32t at = block_exclusive_1024(tid < 256 ? run : 0, S.sums, total);
+        if (tid < 256) for (int w = 0; w < kBlockWarps; w++) { const u32t c = S.count[w][tid]; S.count[w][tid] = at; at += c; }
+        __syncthreads();
+        for (u32t k = k0; k < k1; k += 32) {
+            const bool in = k + lane < k1;
+            const u32t key = in ? kin[k + lane] : 0;
+            const u32t d = in ? (key >> (8 * pass)) & 255u : 256u;
+            const u32t peers = __match_any_sync(0xFFFFFFFFu, d);
+            u32t pos = 0;
+            if (in) pos = S.count[warp][d] + __popc(peers & ((1u << lane) - 1u));
+            __syncwarp();
+            if (in && lane == (u32t)__ffs(peers) - 1) S.count[warp][d] += __popc(peers);
+            if (in) { S.code[(pass + 1) & 1][pos] = key; S.item[(pass + 1) & 1][pos] = vin[k + lane]; }
+            __syncwarp();
+        }
+        __syncthreads();
+    }
+    const u32t *code = S.code[0];
+    const uint16_t *item = S.item[0];
+    for (u32t i = tid; i < n; i += kBlockThreads) {
+        codes[i] = code[i];
+        order[i] = out_order[i] = item[i];
+    }
+    auto leaf_box = [&](u32t place, unsigned b[6]) {
+        const float *a = aabbs + 6 * (u32t)item[place];
+        for (int k = 0; k < 6; k++) b[k] = ord_bits(a[k]);
+    };
+    if (n <= max_leaf) {                               // one leaf
+        if (warp == 0) {
+            unsigned b[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0, 0, 0};
+            for (u32t i = lane; i < n; i += 32) {
+                unsigned c[6];
+                leaf_box(i, c);
+                for (int k = 0; k < 3; k++) { b[k] = min(b[k], c[k]); b[3 + k] = max(b[3 + k], c[3 + k]); }
+            }
+            for (int k = 0; k < 3; k++) { b[k] = __reduce_min_sync(0xFFFFFFFFu, b[k]); b[3 + k] = __reduce_max_sync(0xFFFFFFFFu, b[3 + k]); }
+            if (lane == 0) { write_node(out[0], b, 0, n, 0); info[1] = 1; info[2] = 0; }
+        }
+        return;
+    }
+    // topology
+    const u32t ni = n - 1;
+    u32t *arrivals = &S.count[0][0];
+    for (u32t i = tid; i < ni; i += kBlockThreads) {
+        const KarrasNode k = karras_node(code, item, n, (int)i);
+        S.first[i] = (uint16_t)k.first;
+        S.last[i] = (uint16_t)k.last;
+        S.left[i] = (uint16_t)(k.split | (k.left_leaf ? 0x8000u : 0u));
+        S.right[i] = (uint16_t)((k.split + 1) | (k.right_leaf ? 0x8000u : 0u));
+        (k.left_leaf ? S.leaf_parent : S.parent)[k.split] = (uint16_t)i;
+        (k.right_leaf ? S.leaf_parent : S.parent)[k.split + 1] = (uint16_t)i;
+        if (i == 0) S.parent[0] = 0xFFFF;
+        arrivals[i] = 0;
+    }
+    __syncthreads();
+    // ranks of the kept nodes (those covering more than max_leaf items), in index order
+    u32t kept = 0, total;
+    const u32t per = (ni + kBlockThreads - 1) / kBlockThreads, r0 = min(tid * per, ni), r1 = min(r0 + per, ni);
+    auto keep = [&](u32t i) { return (u32t)(S.last[i] - S.first[i] + 1) > max_leaf; };
+    for (u32t i = r0; i < r1; i++) kept += keep(i);
+    u32t rank = block_exclusive_1024(kept, S.sums, total);
+    for (u32t i = r0; i < r1; i++) { S.rank[i] = (uint16_t)rank; rank += keep(i); }
+    // boxes, bottom-up: the first child to arrive at a node stops, the second combines
+    auto child_bits = [&](u32t ch, unsigned b[6]) {
+        if (ch & 0x8000u) leaf_box(ch & 0x7FFFu, b);
+        else for (int k = 0; k < 6; k++) b[k] = __ldcg(kbox + 6 * ch + k);
+    };
+    for (u32t j = tid; j < n; j += kBlockThreads)
+        for (u32t p = S.leaf_parent[j]; p != 0xFFFFu; p = S.parent[p]) {
+            __threadfence_block();
+            if (atomicAdd(arrivals + p, 1u) == 0) break;
+            __threadfence_block();
+            unsigned a[6], b[6];
+            child_bits(S.left[p], a);
+            child_bits(S.right[p], b);
+            for (int k = 0; k < 3; k++) { __stcg(kbox + 6 * p + k, min(a[k], b[k])); __stcg(kbox + 6 * p + 3 + k, max(a[3 + k], b[3 + k])); }
+        }
+    __threadfence_block();
+    __syncthreads();
+    for (u32t i = tid; i < ni; i += kBlockThreads) {
+        if (!keep(i)) continue;
+        u32t depth = 0;
+        for (u32t p = S.parent[i]; p != 0xFFFFu; p = S.parent[p]) depth++;
+        unsigned b[6];
+        if (i == 0) {
+            child_bits(0, b);
+            write_node(out[0], b, 1 + 2 * S.rank[0], 0, 0);
+        }
+        for (int c = 0; c < 2; c++) {
+            const u32t ch = c ? S.right[i] : S.left[i];
+            BVHNode &o = out[1 + 2 * S.rank[i] + c];
+            child_bits(ch, b);
+            if (ch & 0x8000u) write_node(o, b, ch & 0x7FFFu, 1, depth + 1);
+            else if (keep(ch)) write_node(o, b, 1 + 2 * S.rank[ch], 0, depth + 1);
+            else write_node(o, b, S.first[ch], S.last[ch] - S.first[ch] + 1, depth + 1);
+        }
+        atomicMax(&S.height, depth + 1);
+    }
+    __syncthreads();
+    if (tid == 0) { info[1] = S.height; info[2] = total; }
 }
 
 __global__ void codes_by_item_kernel(const u32t *sorted_codes, const u32t *order, u32t n, u32t *out) {
@@ -449,16 +653,23 @@ void lbvh_release(LbvhScratch &s) {
 cudaError_t lbvh_build(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t info[2],
                        cudaStream_t st) {
     if (n == 0) { info[0] = 0; info[1] = 0; return cudaSuccess; }
-    u32t h[3];
-    lbvh_enqueue(s, n, max_leaf, out_nodes, out_order, h, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    u32t h[3] = {0, 0, 0};
+    cudaError_t e = lbvh_enqueue(s, n, max_leaf, out_nodes, out_order, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, s.info, sizeof(h), cudaMemcpyDeviceToHost, st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);
     info[0] = 1 + 2 * h[2];
     info[1] = h[1];
-    return e;
+    return e != cudaSuccess ? e : e2;
 }
 
-void lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t *counts,
-                  cudaStream_t st) {
+cudaError_t lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, cudaStream_t st) {
+    if (n <= kBlockItems) {
+        const cudaError_t e = cudaFuncSetAttribute(lbvh_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LbvhShared));
+        if (e != cudaSuccess) return e;
+        lbvh_block_kernel<<<1, kBlockThreads, sizeof(LbvhShared), st>>>(s.aabbs, n, max_leaf, s.codes, s.order, out_order, s.kbox,
+                                                                        out_nodes, s.info);
+        return cudaGetLastError();
+    }
     const u32t T = 256;
     bounds_init_kernel<<<1, 32, 0, st>>>(s.bounds);
     bounds_kernel<<<min((n + T - 1) / T, 1184u), T, 0, st>>>(s.aabbs, n, s.bounds);
@@ -476,12 +687,8 @@ void lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32
     }
     // after an even number of passes kin/vin are codes/order again
     if (n <= max_leaf) {
-        single_leaf_kernel<<<1, 1, 0, st>>>(s.aabbs, s.order, n, out_nodes);
-        cudaMemcpyAsync(out_order, s.order, sizeof(u32t) * n, cudaMemcpyDeviceToDevice, st);
-        counts[0] = 0;                     // one node (1 + 2 * 0 kept internal nodes), height 1
-        counts[1] = 1;
-        counts[2] = 0;
-        return;
+        single_leaf_kernel<<<1, 1, 0, st>>>(s.aabbs, s.order, n, out_nodes, s.info);
+        return cudaMemcpyAsync(out_order, s.order, sizeof(u32t) * n, cudaMemcpyDeviceToDevice, st);
     }
     const u32t ni = n - 1;
     karras_kernel<<<(ni + T - 1) / T, T, 0, st>>>(s.codes, s.order, n, s.first, s.last, s.lchild, s.rchild, s.parent,
@@ -496,13 +703,14 @@ void lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32
     layout_kernel<<<(ni + T - 1) / T, T, 0, st>>>(s.aabbs, s.order, ni, s.first, s.last, s.lchild, s.rchild, s.parent,
                                                   s.flags, s.rank, s.kbox, out_nodes, s.info + 1);
     cudaMemcpyAsync(out_order, s.order, sizeof(u32t) * n, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(counts, s.info, sizeof(u32t) * 3, cudaMemcpyDeviceToHost, st);
+    return cudaGetLastError();
 }
 
 // ---- refit of a reference-layout BVH ------------------------------------------------------------
-__global__ void refit_parents_kernel(const BVHNode *nodes, u32t count, u32t *parent) {
+__global__ void refit_parents_kernel(const BVHNode *nodes, u32t count, u32t *parent, u32t *arrivals) {
     u32t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
+    arrivals[i] = 0;
     if (i == 0) parent[0] = 0xFFFFFFFFu;
     const BVHNode nd = nodes[i];
     if (!nd.child_count && nd.first_child_id + 1 < count) {
@@ -510,17 +718,18 @@ __global__ void refit_parents_kernel(const BVHNode *nodes, u32t count, u32t *par
         parent[nd.first_child_id + 1] = i;
     }
 }
-__global__ void refit_kernel(BVHNode *nodes, u32t count, const u32t *leaf_ids, const float *aabbs, const u32t *parent,
-                             u32t *arrivals, unsigned *box) {
+// A leaf's box from its primitives' boxes (as prim_aabbs_kernel gives them), then up the tree.
+__global__ void refit_kernel(BVHNode *nodes, u32t count, const u32t *leaf_ids, const Primitive *prims, const MeshDev *meshes,
+                             const u32t *parent, u32t *arrivals, unsigned *box) {
     u32t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     BVHNode nd = nodes[i];
     if (!nd.child_count) return;          // internal nodes are combined by their children's walk
     unsigned b[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0, 0, 0};
     for (u32t k = 0; k < nd.child_count; k++) {
-        unsigned c[6];
-        item_box(aabbs, leaf_ids[nd.first_child_id + k], c);
-        for (int q = 0; q < 3; q++) { b[q] = min(b[q], c[q]); b[3 + q] = max(b[3 + q], c[3 + q]); }
+        float f[6];
+        prim_box(prims[leaf_ids[nd.first_child_id + k]], meshes, f);
+        for (int q = 0; q < 3; q++) { b[q] = min(b[q], ord_bits(f[q])); b[3 + q] = max(b[3 + q], ord_bits(f[3 + q])); }
     }
     for (int q = 0; q < 6; q++) __stcg(box + 6 * (size_t)i + q, b[q]);
     write_node(nodes[i], b, nd.first_child_id, nd.child_count, nd.depth);
@@ -538,13 +747,12 @@ __global__ void refit_kernel(BVHNode *nodes, u32t count, const u32t *leaf_ids, c
         p = parent[p];
     }
 }
-cudaError_t refit_bvh(BVHNode *nodes, u32t node_count, const u32t *leaf_ids, const float *aabbs,
+cudaError_t refit_bvh(BVHNode *nodes, u32t node_count, const u32t *leaf_ids, const Primitive *prims, const MeshDev *meshes,
                       u32t *scratch_parent, u32t *scratch_flags, unsigned *scratch_box, cudaStream_t st) {
     if (!node_count) return cudaSuccess;
-    const u32t T = 256;
-    refit_parents_kernel<<<(node_count + T - 1) / T, T, 0, st>>>(nodes, node_count, scratch_parent);
-    cudaMemsetAsync(scratch_flags, 0, sizeof(u32t) * node_count, st);
-    refit_kernel<<<(node_count + T - 1) / T, T, 0, st>>>(nodes, node_count, leaf_ids, aabbs, scratch_parent,
+    const u32t T = 128;
+    refit_parents_kernel<<<(node_count + T - 1) / T, T, 0, st>>>(nodes, node_count, scratch_parent, scratch_flags);
+    refit_kernel<<<(node_count + T - 1) / T, T, 0, st>>>(nodes, node_count, leaf_ids, prims, meshes, scratch_parent,
                                                          scratch_flags, scratch_box);
     return cudaGetLastError();
 }
@@ -593,9 +801,7 @@ __global__ void tri_records_kernel(const vec3 *pos, const vec3 *nrm, const vec2 
 }
 
 // ---- conversions into the traversal layouts ---------------------------------------------------
-__global__ void make_pairs_kernel(const BVHNode *nodes, u32t node_count, NodePair *pairs) {
-    u32t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (2 + 2 * k >= node_count) return;
+__device__ __forceinline__ void make_pair(const BVHNode *nodes, u32t k, NodePair *pairs) {
     const BVHNode L = nodes[1 + 2 * k], R = nodes[2 + 2 * k];
     NodePair p;
     p.a = make_float4(L.aabb.min.x, L.aabb.min.y, L.aabb.max.x, L.aabb.max.y);
@@ -604,6 +810,56 @@ __global__ void make_pairs_kernel(const BVHNode *nodes, u32t node_count, NodePai
     p.d = make_uint4(L.child_count ? L.first_child_id : (L.first_child_id - 1) >> 1, L.child_count,
                      R.child_count ? R.first_child_id : (R.first_child_id - 1) >> 1, R.child_count);
     pairs[k] = p;
+}
+__global__ void make_pairs_kernel(const BVHNode *nodes, u32t node_count, NodePair *pairs) {
+    u32t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (2 + 2 * k < node_count) make_pair(nodes, k, pairs);
+}
+
+// ---- the end of a TLAS update -------------------------------------------------------------------
+// The node pairs, and what the host wants of the tree written straight into its page-locked staging
+// (a copy is a command of its own behind the kernels: three of them and the pairs' launch after the
+// wait took 30 to 45 us of an update).  info: the build's {-, height, pairs} on the device, or null
+// for a tree of `count` nodes.  parent_of_pair[k]: the node that claims pair k (tlas_check_kernel).
+__global__ void tlas_finish_kernel(const BVHNode *nodes, const u32t *info, u32t count, const u32t *ids, u32t n, NodePair *pairs,
+                                   u32t *parent_of_pair, TlasStaging out) {
+    const u32t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (info) count = 1 + 2 * min(info[2], n - 1);
+    if (i == 0) {
+        if (info) { out.counts[1] = info[1]; out.counts[2] = info[2]; }
+        *out.root = nodes[0];
+    }
+    if (2 + 2 * i < count) make_pair(nodes, i, pairs);
+    if (i < count) {
+        const BVHNode nd = nodes[i];
+        if (parent_of_pair && !nd.child_count && nd.first_child_id && (nd.first_child_id - 1) / 2 < n)
+            parent_of_pair[(nd.first_child_id - 1) / 2] = i;
+        if (out.nodes) out.nodes[i] = nd;
+    }
+    if (i < n && out.ids) out.ids[i] = ids[i];
+}
+// What st_validate_bvh asks of a tree, of a newly built one before the walk first uses it: every
+// children pair lies inside the array and has one parent, every leaf range and leaf id is in range, and
+// every node reaches the root by at most kStack - 2 parents.  A node that fails sets out.counts[3].
+__global__ void tlas_check_kernel(const BVHNode *nodes, const u32t *info, const u32t *ids, u32t n, const u32t *parent_of_pair,
+                                  TlasStaging out) {
+    const u32t i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool ok = info[2] < n;
+    const u32t count = 1 + 2 * min(info[2], n - 1);
+    if (i < count) {
+        const BVHNode nd = nodes[i];
+        const u32t f = nd.first_child_id;
+        if (nd.child_count) ok = ok && (unsigned long long)f + nd.child_count <= n;
+        else ok = ok && (f & 1u) && f + 1 < count && f + 1 > f && parent_of_pair[(f - 1) / 2] == i;
+        u32t steps = 0;
+        for (u32t at = i; at && ok; steps++) {
+            const u32t pair = (at - 1) / 2, p = parent_of_pair[pair];
+            ok = steps + 2 < (u32t)kStack && p < count && !nodes[p].child_count && nodes[p].first_child_id == 1 + 2 * pair;
+            at = p;
+        }
+    }
+    if (i < n) ok = ok && ids[i] < n;
+    if (!ok) out.counts[3] = 1;
 }
 __global__ void make_trihot_kernel(const Triangle *tris, u32t n, TriHot *hot) {
     u32t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -654,6 +910,12 @@ void launch_tri_records(const vec3 *pos, const vec3 *nrm, const vec2 *uv, const 
 void launch_make_pairs(const BVHNode *nodes, u32t node_count, NodePair *pairs, cudaStream_t st) {
     u32t np = node_count > 1 ? (node_count - 1) / 2 : 0;
     if (np) make_pairs_kernel<<<(np + 255) / 256, 256, 0, st>>>(nodes, node_count, pairs);
+}
+void launch_tlas_finish(const BVHNode *nodes, const u32t *info, u32t count, const u32t *ids, u32t n, NodePair *pairs,
+                        u32t *parent_of_pair, const TlasStaging &out, cudaStream_t st) {
+    const u32t most = max(info ? 2 * n - 1 : count, out.ids ? n : 1u);
+    tlas_finish_kernel<<<(most + 127) / 128, 128, 0, st>>>(nodes, info, count, ids, n, pairs, parent_of_pair, out);
+    if (info) tlas_check_kernel<<<(2 * n + 127) / 128, 128, 0, st>>>(nodes, info, ids, n, parent_of_pair, out);
 }
 void launch_make_trihot(const Triangle *tris, u32t n, TriHot *hot, cudaStream_t st) {
     if (n) make_trihot_kernel<<<(n + 255) / 256, 256, 0, st>>>(tris, n, hot);

@@ -158,10 +158,9 @@ void lbvh_carve(LbvhScratch &s, void *base, u32t cap);
 // out_nodes must hold 2n nodes; out_order n ids.  info (host) receives node_count, height.
 cudaError_t lbvh_build(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order,
                        u32t info[2], cudaStream_t st);
-// The same build (n > 0) without waiting: counts[3] (page-locked host memory, filled once `st`
-// reaches it) receive the words from which node_count = 1 + 2 * counts[2] and height = counts[1].
-void lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t *counts,
-                  cudaStream_t st);
+// The same build (n > 0) without waiting: s.info[1] = height and s.info[2] = pairs (node_count =
+// 1 + 2 * pairs) once `st` reaches it.
+cudaError_t lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, cudaStream_t st);
 // Binned SAH over n device boxes (st_sah.cu): reference-layout nodes (2n capacity) + leaf order.
 // scratch (optional, sah_scratch_bytes(n) bytes): used instead of a stream-ordered allocation
 cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t info[2],
@@ -169,9 +168,9 @@ cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_no
 size_t sah_scratch_bytes(u32t n);
 // Whether sah_enqueue makes the build without waiting for the device on the way.
 bool sah_without_wait(u32t n, u32t max_leaf);
-// The build with sah_scratch_bytes(n) bytes of scratch; counts as lbvh_enqueue's.
+// The build with sah_scratch_bytes(n) bytes of scratch; *info: three device words as lbvh_enqueue's.
 cudaError_t sah_enqueue(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, void *scratch,
-                        u32t *counts, cudaStream_t st);
+                        u32t **info, cudaStream_t st);
 // After lbvh_build: the Morton code of every item, by item index.
 void launch_codes_by_item(const LbvhScratch &s, u32t n, u32t *out, cudaStream_t st);
 // World boxes of primitives as updateSceneBVH computes them (builder_top_down.h:370-377).
@@ -182,10 +181,22 @@ void launch_tri_aabbs(const vec3 *pos, const uint32_t *idx, u32t n, float *aabbs
 void launch_tri_records(const vec3 *pos, const vec3 *nrm, const vec2 *uv, const uint32_t *pidx, const uint32_t *nidx,
                         const uint32_t *uidx, int has_uvs, const u32t *order, u32t n, Triangle *out,
                         u32t *inverse, cudaStream_t st);
-// Refit: recompute every node box of a reference-layout BVH whose items' boxes are `aabbs`
-// (leaf ranges index `leaf_ids`), bottom-up.
-cudaError_t refit_bvh(BVHNode *nodes, u32t node_count, const u32t *leaf_ids, const float *aabbs,
+// Refit: recompute every node box of a reference-layout TLAS over the primitives (leaf ranges index
+// `leaf_ids`), bottom-up.
+cudaError_t refit_bvh(BVHNode *nodes, u32t node_count, const u32t *leaf_ids, const Primitive *prims, const MeshDev *meshes,
                       u32t *scratch_parent, u32t *scratch_flags, unsigned *scratch_box, cudaStream_t st);
+// What the host reads of a TLAS update, in page-locked memory the device writes: counts[1] = height,
+// counts[2] = pairs, counts[3] set when a built tree is not one the walk may use; the root; and, when
+// not null, the nodes and the leaf ids.
+struct TlasStaging {
+    u32t *counts;
+    BVHNode *root, *nodes;
+    u32t *ids;
+};
+// Node pairs and staging of the TLAS `nodes`: a built one (info on the device; it is checked, with n
+// words of parent_of_pair scratch) or one of `count` nodes whose topology was checked before.
+void launch_tlas_finish(const BVHNode *nodes, const u32t *info, u32t count, const u32t *ids, u32t n, NodePair *pairs,
+                        u32t *parent_of_pair, const TlasStaging &out, cudaStream_t st);
 // Reference-layout BVHNode array -> child-pair array (pair k = nodes 1+2k, 2+2k).
 void launch_make_pairs(const BVHNode *nodes, u32t node_count, NodePair *pairs, cudaStream_t st);
 // Triangle -> TriHot

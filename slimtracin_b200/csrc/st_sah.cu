@@ -892,9 +892,9 @@ size_t sah_scratch_bytes(u32t n) { return sah_layout(n).bytes; }
 
 bool sah_without_wait(u32t n, u32t max_leaf) { return n <= kCap || n <= max_leaf; }
 
-// The build on `st`; scratch: sah_scratch_bytes(n) bytes; *info: where the device leaves {-, height, pairs}.
-static cudaError_t sah_launch(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, char *base,
-                              u32t **info, cudaStream_t st) {
+cudaError_t sah_enqueue(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, void *scratch,
+                        u32t **info, cudaStream_t st) {
+    char *base = static_cast<char *>(scratch);
     const SahLayout Lo = sah_layout(n);
     SahCounts *C = (SahCounts *)(base + Lo.counts);
     *info = C->info;
@@ -954,13 +954,6 @@ static cudaError_t sah_launch(const float *aabbs, u32t n, u32t max_leaf, BVHNode
     return cudaGetLastError();
 }
 
-cudaError_t sah_enqueue(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, void *scratch,
-                        u32t *counts, cudaStream_t st) {
-    u32t *info;
-    const cudaError_t e = sah_launch(aabbs, n, max_leaf, out_nodes, out_order, static_cast<char *>(scratch), &info, st);
-    return e != cudaSuccess ? e : cudaMemcpyAsync(counts, info, sizeof(u32t) * 3, cudaMemcpyDeviceToHost, st);
-}
-
 cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t info[2],
                       cudaStream_t st, void *scratch, size_t scratch_bytes) {
     if (n == 0) { info[0] = info[1] = 0; return cudaSuccess; }
@@ -971,8 +964,9 @@ cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_no
     cudaError_t e = cudaSuccess;
     if (own) e = cudaMallocAsync(&base, bytes, st);
     if (e != cudaSuccess) return e;
-    u32t got[3] = {0, 0, 0};
-    e = sah_enqueue(aabbs, n, max_leaf, out_nodes, out_order, base, got, st);
+    u32t got[3] = {0, 0, 0}, *dev_info = nullptr;
+    e = sah_enqueue(aabbs, n, max_leaf, out_nodes, out_order, base, &dev_info, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(got, dev_info, sizeof(got), cudaMemcpyDeviceToHost, st);
     if (own) cudaFreeAsync(base, st);
     const cudaError_t e2 = cudaStreamSynchronize(st);
     info[0] = 1 + 2 * got[2];
