@@ -400,23 +400,25 @@ __global__ void single_leaf_kernel(const float *aabbs, const u32t *order, u32t n
 }
 
 // ---- small builds: the whole LBVH30 by one block ----------------------------------------------------
-// The same steps as the kernels above, at most kBlockItems items, codes, order and topology in shared
-// memory (the boxes of internal nodes stay in kbox, read and written through L2).  A small build is
+// The same steps as the kernels above, at most kBlockItems items, everything between in shared memory.
+// A small build is
 // launches and their gaps, thirty of them: 173 us for 100 primitives, 218 for 1000, 257 for 4096 as
-// st_update_scene_bvh sees it, against 41, 70 and 168 with one (and tlas_finish_kernel below); above
+// st_update_scene_bvh sees it, against 42, 66 and 148 with one (and tlas_finish_kernel below); above
 // 4096 items the shared arrays no longer fit and many blocks are faster than one.
 constexpr u32t kBlockItems = 4096;
 constexpr int kBlockThreads = 1024, kBlockWarps = kBlockThreads / 32;
 struct LbvhShared {
+    unsigned box[6][kBlockItems];      // the internal nodes' boxes, ordered bits
     u32t code[2][kBlockItems];
-    u32t count[kBlockWarps][256];      // a pass' digit counts per warp; afterwards the nodes' arrivals
+    u32t arrived[kBlockItems / 32];    // a bit per internal node: its first child is there
+    uint16_t count[kBlockWarps][256];  // a pass' digit counts per warp
     uint16_t item[2][kBlockItems];
     uint16_t left[kBlockItems], right[kBlockItems], parent[kBlockItems], leaf_parent[kBlockItems];   // leaves: top bit
     uint16_t first[kBlockItems], last[kBlockItems], rank[kBlockItems];
     unsigned bounds[6];
     u32t sums[kBlockWarps], height;
 };
-static_assert(sizeof(LbvhShared) <= 227 * 1024 && kBlockItems <= 0x8000 && kBlockItems <= kBlockWarps * 256, "");
+static_assert(sizeof(LbvhShared) <= 227 * 1024 && kBlockItems <= 0x8000, "one block's shared memory, 15-bit nodes");
 // The sum of the values of the threads before this one, and of all.
 __device__ __forceinline__ u32t block_exclusive_1024(u32t v, u32t *sums, u32t &total) {
     const u32t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -442,8 +444,8 @@ __device__ __forceinline__ u32t block_exclusive_1024(u32t v, u32t *sums, u32t &t
     return r;
 }
 __global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const float *aabbs, u32t n, u32t max_leaf, u32t *codes,
-                                                                      u32t *order, u32t *out_order, unsigned *kbox,
-                                                                      BVHNode *out, u32t *info) {
+                                                                      u32t *order, u32t *out_order, BVHNode *out,
+                                                                      u32t *info) {
     extern __shared__ __align__(16) unsigned char raw[];
     LbvhShared &S = *reinterpret_cast<LbvhShared *>(raw);
     const u32t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -479,7 +481,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const floa
             const bool in = k + lane < k1;
             const u32t d = in ? (kin[k + lane] >> (8 * pass)) & 255u : 256u;
             const u32t peers = __match_any_sync(0xFFFFFFFFu, d);
-            if (in && lane == (u32t)__ffs(peers) - 1) S.count[warp][d] += __popc(peers);
+            if (in && lane == (u32t)__ffs(peers) - 1) S.count[warp][d] += (uint16_t)__popc(peers);
             __syncwarp();
         }
         __syncthreads();
@@ -487,7 +489,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const floa
         u32t run = 0, total;
         if (tid < 256) for (int w = 0; w < kBlockWarps; w++) run += S.count[w][tid];
         u32t at = block_exclusive_1024(tid < 256 ? run : 0, S.sums, total);
-        if (tid < 256) for (int w = 0; w < kBlockWarps; w++) { const u32t c = S.count[w][tid]; S.count[w][tid] = at; at += c; }
+        if (tid < 256) for (int w = 0; w < kBlockWarps; w++) { const u32t c = S.count[w][tid]; S.count[w][tid] = (uint16_t)at; at += c; }
         __syncthreads();
         for (u32t k = k0; k < k1; k += 32) {
             const bool in = k + lane < k1;
@@ -497,7 +499,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const floa
             u32t pos = 0;
             if (in) pos = S.count[warp][d] + __popc(peers & ((1u << lane) - 1u));
             __syncwarp();
-            if (in && lane == (u32t)__ffs(peers) - 1) S.count[warp][d] += __popc(peers);
+            if (in && lane == (u32t)__ffs(peers) - 1) S.count[warp][d] += (uint16_t)__popc(peers);
             if (in) { S.code[(pass + 1) & 1][pos] = key; S.item[(pass + 1) & 1][pos] = vin[k + lane]; }
             __syncwarp();
         }
@@ -528,7 +530,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const floa
     }
     // topology
     const u32t ni = n - 1;
-    u32t *arrivals = &S.count[0][0];
+    for (u32t i = tid; i < kBlockItems / 32; i += kBlockThreads) S.arrived[i] = 0;
     for (u32t i = tid; i < ni; i += kBlockThreads) {
         const KarrasNode k = karras_node(code, item, n, (int)i);
         S.first[i] = (uint16_t)k.first;
@@ -538,7 +540,6 @@ __global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const floa
         (k.left_leaf ? S.leaf_parent : S.parent)[k.split] = (uint16_t)i;
         (k.right_leaf ? S.leaf_parent : S.parent)[k.split + 1] = (uint16_t)i;
         if (i == 0) S.parent[0] = 0xFFFF;
-        arrivals[i] = 0;
     }
     __syncthreads();
     // ranks of the kept nodes (those covering more than max_leaf items), in index order
@@ -551,19 +552,18 @@ __global__ void __launch_bounds__(kBlockThreads, 1) lbvh_block_kernel(const floa
     // boxes, bottom-up: the first child to arrive at a node stops, the second combines
     auto child_bits = [&](u32t ch, unsigned b[6]) {
         if (ch & 0x8000u) leaf_box(ch & 0x7FFFu, b);
-        else for (int k = 0; k < 6; k++) b[k] = __ldcg(kbox + 6 * ch + k);
+        else for (int k = 0; k < 6; k++) b[k] = *const_cast<volatile unsigned *>(&S.box[k][ch]);
     };
     for (u32t j = tid; j < n; j += kBlockThreads)
         for (u32t p = S.leaf_parent[j]; p != 0xFFFFu; p = S.parent[p]) {
             __threadfence_block();
-            if (atomicAdd(arrivals + p, 1u) == 0) break;
+            if (!(atomicOr(&S.arrived[p / 32], 1u << (p % 32)) >> (p % 32) & 1u)) break;
             __threadfence_block();
             unsigned a[6], b[6];
             child_bits(S.left[p], a);
             child_bits(S.right[p], b);
-            for (int k = 0; k < 3; k++) { __stcg(kbox + 6 * p + k, min(a[k], b[k])); __stcg(kbox + 6 * p + 3 + k, max(a[3 + k], b[3 + k])); }
+            for (int k = 0; k < 3; k++) { S.box[k][p] = min(a[k], b[k]); S.box[3 + k][p] = max(a[3 + k], b[3 + k]); }
         }
-    __threadfence_block();
     __syncthreads();
     for (u32t i = tid; i < ni; i += kBlockThreads) {
         if (!keep(i)) continue;
@@ -666,7 +666,7 @@ cudaError_t lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nod
     if (n <= kBlockItems) {
         const cudaError_t e = cudaFuncSetAttribute(lbvh_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LbvhShared));
         if (e != cudaSuccess) return e;
-        lbvh_block_kernel<<<1, kBlockThreads, sizeof(LbvhShared), st>>>(s.aabbs, n, max_leaf, s.codes, s.order, out_order, s.kbox,
+        lbvh_block_kernel<<<1, kBlockThreads, sizeof(LbvhShared), st>>>(s.aabbs, n, max_leaf, s.codes, s.order, out_order,
                                                                         out_nodes, s.info);
         return cudaGetLastError();
     }

@@ -28,9 +28,9 @@ namespace st {
 
 constexpr int kBins = 32;
 constexpr u32t kCap = 4096;            // items one block splits in shared memory
-constexpr u32t kSub = 512;             // items a block builds to the leaves (a warp splits them in about 8 us)
+constexpr u32t kSub = 256;             // items a block builds to the leaves
 constexpr u32t kTiny = 10;             // items up to which a range is split without bins (3 axes x 10 lanes)
-constexpr int kMidThreads = 1024, kMidWarps = kMidThreads / 32;
+constexpr int kMidThreads = 1024, kMidWarps = kMidThreads / 32, kMidGroups = 8;
 constexpr int kThreads = 256, kWarps = kThreads / 32;
 constexpr u32t kPer = (kSub + kThreads - 1) / kThreads;
 constexpr u32t kChunk = 2048;          // items per block when binning / partitioning a large range
@@ -169,13 +169,12 @@ struct SubtreeShared {
 constexpr u32t kMidTasks = kCap / kSub;    // ranges above kSub items of one block: fewer than this
 struct MidShared {
     unsigned box[6][kCap];
-    unsigned bins[kWarpBins];
     uint16_t order[2][kCap];
     SahTask task[2][kMidTasks];        // begin and end within the block's range
     u32t tasks[2];
-    unsigned red[12];
-    Split axis_split[3];
-    u32t warp_sum[kMidWarps], child[2], self;
+    unsigned bins[kMidGroups][kWarpBins], red[kMidGroups][12];
+    Split axis_split[kMidGroups][3];
+    u32t child[kMidGroups][2], warp_sum[kMidWarps];
 };
 
 template <class Shared>
@@ -280,9 +279,16 @@ __device__ __forceinline__ u32t block_exclusive(u32t v, u32t *sums, u32t &total)
     return (warp ? sums[warp - 1] : 0) + x - v;
 }
 
-// Ranges of kSub to kCap items, a block each: split level after level by the whole block; children of
-// at most kSub items (or a leaf's) are left to sah_subtree_kernel.  The ranges are mids[0, C->mids), or
-// with mids == null the whole build, [0, n).
+// A barrier of one group of warps (1 <= id <= kMidGroups).
+__device__ __forceinline__ void group_sync(u32t id, u32t threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Ranges of kSub to kCap items, a block each: split level after level, a level's ranges side by side,
+// each by its share of the block's warps (a split is a chain of steps, some 10 us with 32 warps or with
+// four: one after another, and down to 512 items only, they took 80 us of a 4096-box build, side by side
+// down to 256 60 to 75, and the subtrees 75 instead of 140); children of at most kSub items (or a leaf's) are left to sah_subtree_kernel.  The ranges are mids[0, C->mids), or with
+// mids == null the whole build, [0, n), of items in their own order.
 __global__ void __launch_bounds__(kMidThreads, 1) sah_mid_kernel(const float *aabbs, SahCounts *C, const SahTask *mids, u32t n,
                                                                  u32t max_leaf, u32t *ids0, u32t *ids1, LargeNode *nodes,
                                                                  SahTask *subtrees) {
@@ -307,75 +313,93 @@ __global__ void __launch_bounds__(kMidThreads, 1) sah_mid_kernel(const float *aa
         for (int cur = 0; S.tasks[cur]; cur ^= 1) {
             const uint16_t *ord = S.order[cur];
             uint16_t *ord_next = S.order[cur ^ 1];
-            for (u32t t = 0; t < S.tasks[cur]; t++) {
+            const u32t nt = S.tasks[cur];
+            u32t groups = 1;
+            while (groups < nt && groups < (u32t)kMidGroups) groups *= 2;
+            const u32t warps = kMidWarps / groups, threads = 32 * warps;
+            const u32t g = warp / warps, gw = warp % warps, gt = tid % threads;
+            unsigned *bins = S.bins[g], *red = S.red[g];
+            for (u32t t = g; t < nt; t += groups) {
                 const SahTask K = S.task[cur][t];
                 const u32t b = K.begin, e = K.end, c = e - b;
                 unsigned bx[6], cb[6];
                 empty6(bx);
                 empty6(cb);
-                if (tid < 12) S.red[tid] = tid % 6 < 3 ? 0xFFFFFFFFu : 0u;
-                clear_bins(S.bins, tid, kMidThreads);
-                __syncthreads();
-                for (u32t k = b + tid; k < e; k += kMidThreads) {
+                if (gt < 12) red[gt] = gt % 6 < 3 ? 0xFFFFFFFFu : 0u;
+                clear_bins(bins, gt, threads);
+                group_sync(1 + g, threads);
+                for (u32t k = b + gt; k < e; k += threads) {
                     unsigned it[6], ct[6];
                     item_bits(S, ord[k], it);
                     for (int q = 0; q < 3; q++) ct[q] = ct[3 + q] = ob((fo(it[q]) + fo(it[3 + q])) * 0.5f);
                     grow6(bx, it);
                     grow6(cb, ct);
                 }
+                __syncwarp();
                 warp_grow6(bx);
                 warp_grow6(cb);
-                if (lane == 0) { atomic_grow6(S.red, bx); atomic_grow6(S.red + 6, cb); }
-                __syncthreads();
-                const Axes A = axes_of(S.red + 6);
-                for (u32t k = b + tid; k < e; k += kMidThreads) bin_item(S.bins, A, S, ord[k]);
-                __syncthreads();
-                if (warp < 3) {
-                    const Split s = sweep_bins(S.bins, A, (int)warp, (int)lane);
-                    if (lane == 0) S.axis_split[warp] = s;
+                if (lane == 0) { atomic_grow6(red, bx); atomic_grow6(red + 6, cb); }
+                group_sync(1 + g, threads);
+                const Axes A = axes_of(red + 6);
+                for (u32t k = b + gt; k < e; k += threads) bin_item(bins, A, S, ord[k]);
+                group_sync(1 + g, threads);
+                if (gw < 3) {
+                    const Split s = sweep_bins(bins, A, (int)gw, (int)lane);
+                    if (lane == 0) S.axis_split[g][gw] = s;
                 }
-                __syncthreads();
-                Split s = better(better(S.axis_split[0], S.axis_split[1]), S.axis_split[2]);
+                group_sync(1 + g, threads);
+                Split s = better(better(S.axis_split[g][0], S.axis_split[g][1]), S.axis_split[g][2]);
                 if (s.key == kNoSplit) s.nleft = c / 2;
-                // stable partition: a thread takes consecutive places
-                const u32t per = (c + kMidThreads - 1) / kMidThreads;
-                const u32t k0 = b + min(tid * per, c), k1 = b + min((tid + 1) * per, c);
-                u32t left = 0, total;
+                // stable partition: a thread takes consecutive places, its warp's and then the group's
+                // prefix sums give the left items before them
+                const u32t per = (c + threads - 1) / threads;
+                const u32t k0 = b + min(gt * per, c), k1 = b + min((gt + 1) * per, c);
+                u32t left = 0;
                 for (u32t k = k0; k < k1; k++) left += goes_left(S, A, s, ord[k], k - b);
-                u32t before = block_exclusive<kMidWarps>(left, S.warp_sum, total);
+                __syncwarp();
+                u32t x = left;
+                for (int off = 1; off < 32; off <<= 1) {
+                    const u32t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+                    if (lane >= (u32t)off) x += y;
+                }
+                if (lane == 31) S.warp_sum[warp] = x;
+                group_sync(1 + g, threads);
+                u32t before = x - left;
+                for (u32t w = 0; w < gw; w++) before += S.warp_sum[warp - gw + w];
                 for (u32t k = k0; k < k1; k++) {
                     const uint16_t it = ord[k];
                     const bool l = goes_left(S, A, s, it, k - b);
                     ord_next[l ? b + before : b + s.nleft + (k - b - before)] = it;
                     before += l;
                 }
-                if (tid == 0) {
+                if (gt == 0) {
                     const u32t self = atomicAdd(&C->nodes, 1u);
                     LargeNode &o = nodes[self];
-                    for (int q = 0; q < 6; q++) o.box[q] = S.red[q];
+                    for (int q = 0; q < 6; q++) o.box[q] = red[q];
                     o.begin = base + b; o.level = K.level; o.parent = K.parent; o.side = K.side;
                     for (u32t side = 0; side < 2; side++) {
                         SahTask N{side ? b + s.nleft : b, side ? e : b + s.nleft, K.level + 1, T.source ? 0u : 1u, self, side};
                         const u32t nc = N.end - N.begin;
-                        S.child[side] = nc <= kSub || nc <= max_leaf;
-                        if (S.child[side]) {
+                        S.child[g][side] = nc <= kSub || nc <= max_leaf;
+                        if (S.child[g][side]) {
                             N.begin += base;
                             N.end += base;
                             subtrees[atomicAdd(&C->subtrees, 1u)] = N;
                         } else {
-                            S.task[cur ^ 1][S.tasks[cur ^ 1]++] = N;
+                            S.task[cur ^ 1][atomicAdd(&S.tasks[cur ^ 1], 1u)] = N;
                         }
                     }
                 }
-                __syncthreads();
+                group_sync(1 + g, threads);
                 // a child that leaves takes its items, in their order, with it
-                for (u32t k = b + tid; k < e; k += kMidThreads) {
-                    if (!S.child[k - b < s.nleft ? 0 : 1]) continue;
+                for (u32t k = b + gt; k < e; k += threads) {
+                    if (!S.child[g][k - b < s.nleft ? 0 : 1]) continue;
                     const u32t it = base + ord_next[k];
                     parted[base + k] = ids ? ids[it] : it;
                 }
-                __syncthreads();
+                group_sync(1 + g, threads);
             }
+            __syncthreads();
             if (tid == 0) S.tasks[cur] = 0;
             __syncthreads();
         }
