@@ -193,9 +193,9 @@ struct st_ctx {
     char *bvh_pinned = nullptr;          // a TLAS build's counts, nodes and leaf order, read back at once
     size_t bvh_pinned_cap = 0;
     size_t upd_pinned_cap = 0;
-    // page-locked landing place of a render's status words and work counters, so that reading them
-    // back is an asynchronous copy rather than a staged one
-    unsigned long long *readback = nullptr;
+    // page-locked landing place of a render's work counters and of what kernels write to the host
+    // themselves: a render's status word (at word 16) and a pick's result (from word 20)
+    unsigned long long *readback = nullptr, *readback_dev = nullptr;   // host and device view
     // renders into host memory, traced in column strips: one stream per strip (so that the strips
     // run as one grid does, and each strip's copy follows its own trace), a stream for the strips'
     // resolves, and the events that order them (created on first use)
@@ -410,10 +410,11 @@ int st_init(st_ctx **out, const st_config *cfg) {
     }
     int s = reserve(ctx, ctx->status, 16);
     if (s == ST_OK) s = reserve(ctx, ctx->counters, sizeof(unsigned long long) * 16);
-    if (s == ST_OK && cudaMallocHost((void **)&ctx->readback, sizeof(unsigned long long) * 20) != cudaSuccess) {
+    if (s == ST_OK && cudaMallocHost((void **)&ctx->readback, sizeof(unsigned long long) * 32) != cudaSuccess) {
         ctx->readback = nullptr;
         s = ST_ERR_OUT_OF_MEMORY;
     }
+    if (s == ST_OK && cudaHostGetDevicePointer((void **)&ctx->readback_dev, ctx->readback, 0) != cudaSuccess) s = ST_ERR_CUDA;
     if (s != ST_OK) {
         st_shutdown(ctx);
         return s;
@@ -1182,11 +1183,13 @@ int st_render_ex(st_ctx *ctx, int slot, const Scene *scene, const Viewport *view
         }
     }
     SceneDev sd = scene_view(*S, scene);
-    ST_CUDA(cudaMemsetAsync(ctx->status.ptr, 0, 16, st));
+    // the trace writes its status word to the host itself, and only when there is something to say
+    volatile unsigned *status = reinterpret_cast<unsigned *>(ctx->readback + 16);
+    unsigned *dev_status = reinterpret_cast<unsigned *>(ctx->readback_dev + 16);
+    *status = 0;
     if (o->count_work) ST_CUDA(cudaMemsetAsync(ctx->counters.ptr, 0, sizeof(unsigned long long) * 16, st));
     ST_CUDA(cudaEventRecord(ctx->ev[0], st));
-    launch_ssb(sd, v, P<int4>(ctx->ssb), st);
-    launch_ray_rows(v, P<float>(ctx->dirs), st);
+    launch_frame_setup(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), st);
     // Host outputs.  A page-locked frame (pinned or registered) is written by the resolve kernel
     // itself; a page-locked float grid is traced in column strips, one stream per strip, and each
     // strip's columns are copied to the host by a 2-D DMA copy on its own stream, and its pixels
@@ -1219,7 +1222,7 @@ int st_render_ex(st_ctx *ctx, int slot, const Scene *scene, const Viewport *view
             strip_cols(k, gx0, gx1);
             cudaStream_t ts = ctx->strip_trace[k];
             ST_CUDA(cudaStreamWaitEvent(ts, fork, 0));
-            launch_trace(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), dev_float, dev_ids, P<unsigned>(ctx->status),
+            launch_trace(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), dev_float, dev_ids, dev_status,
                          P<unsigned long long>(ctx->counters), o->count_work != 0, ts, gx0 / 8, (gx1 - gx0 + 7) / 8);
             ST_CUDA(cudaGetLastError());
             ST_CUDA(cudaEventRecord(done[k], ts));
@@ -1250,7 +1253,7 @@ int st_render_ex(st_ctx *ctx, int slot, const Scene *scene, const Viewport *view
             ST_CUDA(cudaStreamWaitEvent(st, resolved_ev, 0));
         }
     } else {
-        launch_trace(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), dev_float, dev_ids, P<unsigned>(ctx->status),
+        launch_trace(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), dev_float, dev_ids, dev_status,
                      P<unsigned long long>(ctx->counters), o->count_work != 0, st);
         ST_CUDA(cudaGetLastError());
         ST_CUDA(cudaEventRecord(ctx->ev[2], st));
@@ -1266,16 +1269,14 @@ int st_render_ex(st_ctx *ctx, int slot, const Scene *scene, const Viewport *view
         if (o->out_prim_id)
             ST_CUDA(cudaMemcpyAsync(o->out_prim_id, dev_ids, sizeof(u32t) * grid, cudaMemcpyDeviceToHost, st));
     }
-    unsigned *status = reinterpret_cast<unsigned *>(ctx->readback + 16);
     unsigned long long *c = ctx->readback;
-    ST_CUDA(cudaMemcpyAsync(status, ctx->status.ptr, 16, cudaMemcpyDeviceToHost, st));
     if (o->count_work) ST_CUDA(cudaMemcpyAsync(c, ctx->counters.ptr, sizeof(unsigned long long) * 16, cudaMemcpyDeviceToHost, st));
     ST_CUDA(cudaStreamSynchronize(st));
     if (o->count_work)
         for (int k = 0; k < 16; k++) o->counters[k] = k < C_COUNT ? c[k] : 0;
     cudaEventElapsedTime(&o->trace_ms, ctx->ev[1], ctx->ev[2]);
     cudaEventElapsedTime(&o->total_ms, ctx->ev[0], ctx->ev[3]);
-    if (status[0] & S_STACK_OVERFLOW) return ST_ERR_STACK_OVERFLOW;
+    if (*status & S_STACK_OVERFLOW) return ST_ERR_STACK_OVERFLOW;
     return ST_OK;
 }
 
@@ -1668,18 +1669,13 @@ int st_pick(st_ctx *ctx, int slot, const Scene *scene, const Viewport *viewport,
     cudaSetDevice(ctx->device);
     ViewDev v;
     ST_TRY(make_view(viewport, v));
-    ST_TRY(reserve(ctx, ctx->ssb, sizeof(int4) * std::max(S->n_prims, 1u)));
-    ST_TRY(reserve(ctx, ctx->counters, sizeof(unsigned long long) * 16));
+    static_assert(sizeof(PickDev) <= sizeof(unsigned long long) * 12, "the readback's room for a pick");
     SceneDev sd = scene_view(*S, scene);
     cudaStream_t st = ctx->stream;
-    launch_ssb(sd, v, P<int4>(ctx->ssb), st);
-    PickDev *d = reinterpret_cast<PickDev *>(ctx->counters.ptr);     // 128 bytes of scratch
-    launch_pick(sd, v, P<int4>(ctx->ssb), x, y, d, st);
+    launch_pick(sd, v, x, y, reinterpret_cast<PickDev *>(ctx->readback_dev + 20), st);
     ST_CUDA(cudaGetLastError());
-    PickDev h;
-    ST_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, st));
     ST_CUDA(cudaStreamSynchronize(st));
-    memcpy(result, &h, sizeof(h));
+    memcpy(result, ctx->readback + 20, sizeof(PickDev));
     return ST_OK;
 }
 

@@ -89,7 +89,6 @@ struct ParkQueue {
 };
 constexpr u32t kParkCapacity = 1u << 20;   // parked rays per launch group at most (96 MB)
 
-void launch_ssb(const SceneDev &S, const ViewDev &v, int4 *ssb, cudaStream_t st);
 int launch_batch(const BatchView *views, u32t n_views, u32t total_tiles, int variant, u32t chunk, u32t grid_blocks,
                  u32t *tile_counter, unsigned *status, unsigned long long *counters, bool count, cudaStream_t st,
                  const ParkQueue &park);
@@ -98,9 +97,9 @@ int launch_drain(const BatchView *views, const ParkQueue &park, int variant, u32
                  unsigned long long *counters, bool count, cudaStream_t st);
 void tile_dims(int variant, u32t &tw, u32t &th);
 int batch_blocks_per_sm(int variant);
-// Row-segment starts of the view's ray directions: ceil(grid_w / kSegment) x grid_h float3,
-// segment-major.
-void launch_ray_rows(const ViewDev &v, float *dirs, cudaStream_t st);
+// The primitives' screen bounds and the row-segment starts of the view's ray directions:
+// ceil(grid_w / kSegment) x grid_h float3, segment-major.
+void launch_frame_setup(const SceneDev &S, const ViewDev &v, int4 *ssb, float *dirs, cudaStream_t st);
 inline size_t ray_rows_floats(const ViewDev &v) { return (size_t)v.grid_h * ((v.grid_w + kSegment - 1) / kSegment) * 3; }
 // Block columns [bx_first, bx_first + bx_count) of the grid (8 grid points wide each; bx_count 0:
 // to the last column).
@@ -114,7 +113,7 @@ struct PickDev {
     float position[3];
     float distance, object_distance;
 };
-void launch_pick(const SceneDev &S, const ViewDev &v, const int4 *ssb, int x, int y, PickDev *out, cudaStream_t st);
+void launch_pick(const SceneDev &S, const ViewDev &v, int x, int y, PickDev *out, cudaStream_t st);
 // Pixel columns [x0, x1) of the QCAA resolve (all of them by default).
 void launch_resolve(const FloatPixel *in, u32t grid_w, u32t width, u32t height, uint32_t *out, cudaStream_t st,
                     u32t x0 = 0, u32t x1 = 0xFFFFFFFFu);
