@@ -54,6 +54,7 @@ struct SceneSlot {
     DevBuf textures, mips, quads;
     DevBuf emissive, occluders;
     u32t n_emissive = 0, n_occluders = 0;
+    bool bounces = false;                  // some material reflects or refracts
     vec3 ambient{};
     bool lights_present = false;
     std::vector<Primitive> prims_host;    // host copy for the emissive/occluder lists
@@ -330,6 +331,8 @@ int refresh_lists(st_ctx *ctx, SceneSlot &S) {
             em.push_back(i);
         if (p.type == PrimitiveType_Sphere || p.type == PrimitiveType_Quad) oc.push_back(i);
     }
+    S.bounces = false;
+    for (const Material &m : S.materials_host) S.bounces = S.bounces || (m.is & (REFLECTIVE | REFRACTIVE));
     S.n_emissive = (u32t)em.size();
     S.n_occluders = (u32t)oc.size();
     if (!em.empty()) ST_CUDA(cudaMemcpyAsync(S.emissive.ptr, em.data(), em.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
@@ -1223,7 +1226,7 @@ int st_render_ex(st_ctx *ctx, int slot, const Scene *scene, const Viewport *view
             cudaStream_t ts = ctx->strip_trace[k];
             ST_CUDA(cudaStreamWaitEvent(ts, fork, 0));
             launch_trace(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), dev_float, dev_ids, dev_status,
-                         P<unsigned long long>(ctx->counters), o->count_work != 0, ts, gx0 / 8, (gx1 - gx0 + 7) / 8);
+                         P<unsigned long long>(ctx->counters), o->count_work != 0, ts, false, gx0 / 8, (gx1 - gx0 + 7) / 8);
             ST_CUDA(cudaGetLastError());
             ST_CUDA(cudaEventRecord(done[k], ts));
         }
@@ -1254,7 +1257,7 @@ int st_render_ex(st_ctx *ctx, int slot, const Scene *scene, const Viewport *view
         }
     } else {
         launch_trace(sd, v, P<int4>(ctx->ssb), P<float>(ctx->dirs), dev_float, dev_ids, dev_status,
-                     P<unsigned long long>(ctx->counters), o->count_work != 0, st);
+                     P<unsigned long long>(ctx->counters), o->count_work != 0, st, !S->bounces);
         ST_CUDA(cudaGetLastError());
         ST_CUDA(cudaEventRecord(ctx->ev[2], st));
         if (overlays) ST_TRY(draw_overlays(ctx, *S, viewport, v, o->overlays, dev_float, nullptr, st));

@@ -102,10 +102,10 @@ int batch_blocks_per_sm(int variant);
 void launch_frame_setup(const SceneDev &S, const ViewDev &v, int4 *ssb, float *dirs, cudaStream_t st);
 inline size_t ray_rows_floats(const ViewDev &v) { return (size_t)v.grid_h * ((v.grid_w + kSegment - 1) / kSegment) * 3; }
 // Block columns [bx_first, bx_first + bx_count) of the grid (8 grid points wide each; bx_count 0:
-// to the last column).
+// to the last column).  from_middle: for a launch that runs alone and whose paths do not bounce.
 void launch_trace(const SceneDev &S, const ViewDev &v, const int4 *ssb, const float *dirs, FloatPixel *out,
                   u32t *prim_ids, unsigned *status, unsigned long long *counters, bool count, cudaStream_t st,
-                  u32t bx_first = 0, u32t bx_count = 0);
+                  bool from_middle = false, u32t bx_first = 0, u32t bx_count = 0);
 // The result of a pick (layout of st_pick_result)
 struct PickDev {
     int found, object_type;
