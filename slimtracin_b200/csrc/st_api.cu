@@ -176,6 +176,7 @@ struct Server {
 // holding strip k back until strip k - 2 is done spreads their ends over the frame, but costs more
 // in the trace than it gains in the copies.
 constexpr int kRenderStrips = 8;
+constexpr uint64_t kTransientKept = (uint64_t)512 << 20;
 
 struct st_ctx {
     int device = 0;
@@ -203,6 +204,11 @@ struct st_ctx {
     cudaStream_t strip_trace[kRenderStrips] = {}, strip_resolve = nullptr;
     cudaEvent_t strip_ev[2 * kRenderStrips + 2] = {};
     LbvhScratch lbvh;
+    // what a call allocates for its own time comes from a pool that keeps up to kTransientKept bytes of
+    // it for the next call (mapping and unmapping it took 14 ms of a 327,680-triangle BLAS build, 1 ms
+    // of a 1024x1024 texture); given back when an allocation that stays needs the room, and at shutdown
+    cudaMemPool_t pool = nullptr;
+    Stage stage;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::string cuda_error;
 };
@@ -235,6 +241,22 @@ void release(st_ctx *ctx, DevBuf &b) {
     }
     b = DevBuf();
 }
+// Device memory for one call, freed with cudaFreeAsync on the same stream.
+cudaError_t transient(st_ctx *ctx, void **p, size_t bytes, cudaStream_t st) {
+    if (!ctx->pool) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
+        if (e != cudaSuccess) { ctx->pool = nullptr; return e; }
+        uint64_t keep = kTransientKept;
+        e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+}
 // Grow `b` to at least `bytes` (contents are not kept).  Refuses past the context's budget.
 int reserve(st_ctx *ctx, DevBuf &b, size_t bytes) {
     if (bytes <= b.bytes && b.ptr) return ST_OK;
@@ -242,7 +264,16 @@ int reserve(st_ctx *ctx, DevBuf &b, size_t bytes) {
     size_t add = bytes - (b.ptr ? b.bytes : 0);
     if (ctx->in_use + add > ctx->budget) return ST_ERR_BUDGET;
     release(ctx, b);
+    uint64_t kept = 0;
+    if (ctx->pool && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &kept) == cudaSuccess &&
+        ctx->in_use + bytes + kept > ctx->budget)
+        cudaMemPoolTrimTo(ctx->pool, 0);
     cudaError_t e = cudaMalloc(&b.ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && kept) {
+        cudaGetLastError();
+        cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMalloc(&b.ptr, bytes);
+    }
     if (e != cudaSuccess) return fail_cuda(ctx, e);
     b.bytes = bytes;
     ctx->in_use += bytes;
@@ -384,7 +415,7 @@ int st_init(st_ctx **out, const st_config *cfg) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess || prop.major != 10) return ST_ERR_NO_DEVICE;
     st_ctx *ctx = new st_ctx();
-    ctx->device = device;
+    ctx->device = ctx->stage.device = device;
     ctx->budget = (cfg && cfg->memory_budget) ? cfg->memory_budget : (uint64_t)120 << 30;
     ctx->slots.resize((cfg && cfg->max_scenes > 0) ? cfg->max_scenes : 16);
     cudaError_t e = cudaSetDevice(device);
@@ -442,6 +473,8 @@ void st_shutdown(st_ctx *ctx) {
     for (cudaStream_t t : ctx->strip_trace) if (t) cudaStreamDestroy(t);
     if (ctx->strip_resolve) cudaStreamDestroy(ctx->strip_resolve);
     lbvh_release(ctx->lbvh);
+    stage_release(ctx->stage);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     for (DevBuf *b : {&ctx->batch.table, &ctx->batch.ssb, &ctx->batch.seg, &ctx->batch.out_float, &ctx->batch.out_u8,
                       &ctx->batch.counter, &ctx->batch.park})
         release(ctx, *b);
@@ -682,7 +715,7 @@ int st_upload_mesh_bvhs(st_ctx *ctx, int slot, const Scene *scene) {
         if (M.bvh.node_count > 1) {
             // stage the nodes through the TLAS AABB scratch-free path: a temporary device copy
             BVHNode *tmp = nullptr;
-            ST_CUDA(cudaMallocAsync((void **)&tmp, sizeof(BVHNode) * M.bvh.node_count, ctx->stream));
+            ST_CUDA(transient(ctx, (void **)&tmp, sizeof(BVHNode) * M.bvh.node_count, ctx->stream));
             ST_CUDA(cudaMemcpyAsync(tmp, M.bvh.nodes, sizeof(BVHNode) * M.bvh.node_count, cudaMemcpyHostToDevice, ctx->stream));
             launch_make_pairs(tmp, M.bvh.node_count, P<NodePair>(S->mesh_pairs) + pair_off, ctx->stream);
             ST_CUDA(cudaFreeAsync(tmp, ctx->stream));
@@ -867,7 +900,7 @@ static int update_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode) {
         u32t info[2];
         ST_TRY(reserve(ctx, ctx->sah_scratch, sah_scratch_bytes(n)));
         cudaError_t e = sah_build(ctx->lbvh.aabbs, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes),
-                                  P<u32t>(S->tlas_leaf_ids), info, ctx->stream, ctx->sah_scratch.ptr, ctx->sah_scratch.bytes);
+                                  P<u32t>(S->tlas_leaf_ids), info, ctx->stream, ctx->sah_scratch.ptr);
         if (e != cudaSuccess) return fail_cuda(ctx, e);
         S->tlas_node_count = info[0];
         S->tlas_height = info[1];
@@ -914,19 +947,14 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
     cudaSetDevice(ctx->device);
     const u32t n = mesh->triangle_count;
     if (!n) return ST_ERR_BAD_SCENE;
-    for (u32t i = 0; i < 3 * n; i++) {
-        if (((const uint32_t *)mesh->vertex_position_indices)[i] >= mesh->vertex_count) return ST_ERR_BAD_SCENE;
-        if (((const uint32_t *)mesh->vertex_normal_indices)[i] >= mesh->normals_count) return ST_ERR_BAD_SCENE;
-        if (mesh->uvs_count && ((const uint32_t *)mesh->vertex_uvs_indices)[i] >= mesh->uvs_count) return ST_ERR_BAD_SCENE;
-    }
     if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
     cudaStream_t st = ctx->stream;
     size_t bytes = sizeof(vec3) * (mesh->vertex_count + mesh->normals_count) + sizeof(vec2) * (mesh->uvs_count + 1) +
                    sizeof(uint32_t) * 9 * (size_t)n + sizeof(BVHNode) * 2 * (size_t)n + sizeof(u32t) * 2 * (size_t)n +
-                   sizeof(Triangle) * (size_t)n + 256 * 8;
+                   sizeof(Triangle) * (size_t)n + 256 * 11;
     if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
     char *base = nullptr;
-    ST_CUDA(cudaMallocAsync((void **)&base, bytes, st));
+    ST_CUDA(transient(ctx, (void **)&base, bytes, st));
     char *cur = base;
     auto take = [&](size_t b) { char *p = cur; cur += (b + 255) & ~(size_t)255; return p; };
     vec3 *pos = (vec3 *)take(sizeof(vec3) * mesh->vertex_count);
@@ -939,32 +967,44 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
     u32t *order = (u32t *)take(sizeof(u32t) * n);
     u32t *inverse = (u32t *)take(sizeof(u32t) * n);
     Triangle *tris = (Triangle *)take(sizeof(Triangle) * n);
-    cudaMemcpyAsync(pos, mesh->vertex_positions, sizeof(vec3) * mesh->vertex_count, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(nrm, mesh->vertex_normals, sizeof(vec3) * mesh->normals_count, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(pidx, mesh->vertex_position_indices, sizeof(uint32_t) * 3 * n, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(nidx, mesh->vertex_normal_indices, sizeof(uint32_t) * 3 * n, cudaMemcpyHostToDevice, st);
-    if (mesh->uvs_count) {
-        cudaMemcpyAsync(uv, mesh->vertex_uvs, sizeof(vec2) * mesh->uvs_count, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(uidx, mesh->vertex_uvs_indices, sizeof(uint32_t) * 3 * n, cudaMemcpyHostToDevice, st);
-    }
-    launch_tri_aabbs(pos, pidx, n, ctx->lbvh.aabbs, st);
-    u32t info[2];
-    cudaError_t e = mode == ST_BVH_LBVH30
-        ? lbvh_build(ctx->lbvh, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st)
-        : sah_build(ctx->lbvh.aabbs, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st,
-                    ctx->sah_scratch.ptr, ctx->sah_scratch.bytes);
+    const size_t uvs = mesh->uvs_count, index_bytes = sizeof(uint32_t) * 3 * (size_t)n;
+    cudaError_t e = stage_copy(ctx->stage, {{mesh->vertex_positions, pos, sizeof(vec3) * mesh->vertex_count},
+                                            {mesh->vertex_normals, nrm, sizeof(vec3) * mesh->normals_count},
+                                            {mesh->vertex_position_indices, pidx, index_bytes},
+                                            {mesh->vertex_normal_indices, nidx, index_bytes},
+                                            {mesh->vertex_uvs, uv, sizeof(vec2) * uvs},
+                                            {mesh->vertex_uvs_indices, uidx, uvs ? index_bytes : 0}}, false, st);
+    // indices out of range are refused before anything is read through them
+    volatile unsigned *bad = reinterpret_cast<unsigned *>(ctx->readback + 18);
+    *bad = 0;
     if (e == cudaSuccess) {
-        launch_tri_records(pos, nrm, uv, pidx, nidx, uidx, mesh->uvs_count ? 1 : 0, order, n, tris, inverse, st);
-        cudaMemcpyAsync(mesh->bvh.nodes, nodes, sizeof(BVHNode) * info[0], cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(mesh->bvh.leaf_ids, inverse, sizeof(u32t) * n, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(mesh->triangles, tris, sizeof(Triangle) * n, cudaMemcpyDeviceToHost, st);
-        cudaFreeAsync(base, st);
+        launch_check_indices(pidx, nidx, uidx, 3 * n, mesh->vertex_count, mesh->normals_count, mesh->uvs_count,
+                             reinterpret_cast<unsigned *>(ctx->readback_dev + 18), st);
         e = cudaStreamSynchronize(st);
-    } else {
-        cudaFreeAsync(base, st);
-        cudaStreamSynchronize(st);
     }
+    u32t info[2];
+    void *scratch = nullptr;
+    if (e == cudaSuccess && !*bad) {
+        launch_tri_aabbs(pos, pidx, n, ctx->lbvh.aabbs, st);
+        if (mode == ST_BVH_LBVH30) {
+            e = lbvh_build(ctx->lbvh, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st);
+        } else {
+            e = transient(ctx, &scratch, sah_scratch_bytes(n), st);
+            if (e == cudaSuccess) e = sah_build(ctx->lbvh.aabbs, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st, scratch);
+        }
+        if (e == cudaSuccess) {
+            launch_tri_records(pos, nrm, uv, pidx, nidx, uidx, uvs ? 1 : 0, order, n, tris, inverse, st);
+            e = stage_copy(ctx->stage, {{mesh->triangles, tris, sizeof(Triangle) * (size_t)n},
+                                        {mesh->bvh.nodes, nodes, sizeof(BVHNode) * (size_t)info[0]},
+                                        {mesh->bvh.leaf_ids, inverse, sizeof(u32t) * (size_t)n}}, true, st);
+        }
+    }
+    if (scratch) cudaFreeAsync(scratch, st);
+    cudaFreeAsync(base, st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return fail_cuda(ctx, e);
+    if (*bad) return ST_ERR_BAD_SCENE;
     mesh->bvh.node_count = info[0];
     mesh->bvh.height = info[1];
     return ST_OK;
@@ -981,16 +1021,18 @@ int st_build_bvh(st_ctx *ctx, int mode, const float *aabbs, uint32_t n, uint32_t
     char *base = nullptr;
     const size_t bytes = sizeof(BVHNode) * 2 * (size_t)n + sizeof(u32t) * 2 * (size_t)n + 512;
     if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
-    ST_CUDA(cudaMallocAsync((void **)&base, bytes, st));
+    ST_CUDA(transient(ctx, (void **)&base, bytes, st));
     BVHNode *d_nodes = (BVHNode *)base;
     u32t *d_order = (u32t *)(base + ((sizeof(BVHNode) * 2 * (size_t)n + 255) & ~(size_t)255));
     u32t *d_codes = d_order + n;
     cudaMemcpyAsync(ctx->lbvh.aabbs, aabbs, sizeof(float) * 6 * (size_t)n, cudaMemcpyHostToDevice, st);
     u32t inf[2];
-    cudaError_t e = mode == ST_BVH_LBVH30     ? lbvh_build(ctx->lbvh, n, max_leaf, d_nodes, d_order, inf, st)
+    void *scratch = nullptr;
+    cudaError_t e = mode == ST_BVH_BINNED_SAH ? transient(ctx, &scratch, sah_scratch_bytes(n), st) : cudaSuccess;
+    if (e == cudaSuccess)
+        e = mode == ST_BVH_LBVH30     ? lbvh_build(ctx->lbvh, n, max_leaf, d_nodes, d_order, inf, st)
                     : mode == ST_BVH_REF_SAH ? refsah_build(ctx->lbvh.aabbs, n, max_leaf, d_nodes, d_order, inf, st)
-                                             : sah_build(ctx->lbvh.aabbs, n, max_leaf, d_nodes, d_order, inf, st,
-                                                         ctx->sah_scratch.ptr, ctx->sah_scratch.bytes);
+                                             : sah_build(ctx->lbvh.aabbs, n, max_leaf, d_nodes, d_order, inf, st, scratch);
     if (e == cudaSuccess) {
         if (mode == ST_BVH_LBVH30) launch_codes_by_item(ctx->lbvh, n, d_codes, st);
         else codes = nullptr;
@@ -999,6 +1041,7 @@ int st_build_bvh(st_ctx *ctx, int mode, const float *aabbs, uint32_t n, uint32_t
         if (codes) cudaMemcpyAsync(codes, d_codes, sizeof(u32t) * n, cudaMemcpyDeviceToHost, st);
         e = cudaStreamSynchronize(st);
     }
+    if (scratch) cudaFreeAsync(scratch, st);
     cudaFreeAsync(base, st);
     cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail_cuda(ctx, e);
@@ -1710,15 +1753,14 @@ int st_bake_texture(st_ctx *ctx, const uint8_t *components, uint16_t width, uint
     const size_t bytes = ((image + 255) & ~(size_t)255) + texture_scratch_bytes(width, height) + sizeof(TexelQuad) * quads + 512;
     if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
     char *base = nullptr;
-    ST_CUDA(cudaMallocAsync((void **)&base, bytes, st));
+    ST_CUDA(transient(ctx, (void **)&base, bytes, st));
     uint8_t *dev_image = reinterpret_cast<uint8_t *>(base);
     char *scratch = base + ((image + 255) & ~(size_t)255);
     TexelQuad *dev_quads = reinterpret_cast<TexelQuad *>(scratch + ((texture_scratch_bytes(width, height) + 255) & ~(size_t)255));
-    cudaError_t e = cudaMemcpyAsync(dev_image, components, image, cudaMemcpyHostToDevice, st);
+    cudaError_t e = stage_copy(ctx->stage, {{const_cast<uint8_t *>(components), dev_image, image}}, false, st);
     if (e == cudaSuccess) e = bake_texture(dev_image, width, height, bit_count, wrap != 0, mipmap != 0, scratch, dev_quads, st);
     char *host = static_cast<char *>(memory);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(host + table, dev_quads, sizeof(TexelQuad) * quads, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = stage_copy(ctx->stage, {{host + table, dev_quads, sizeof(TexelQuad) * quads}}, true, st);
     cudaFreeAsync(base, st);
     const cudaError_t e2 = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = e2;
@@ -1843,7 +1885,7 @@ int st_obj_to_mesh(st_ctx *ctx, const char *obj_path, int invert_winding_order, 
                          unique_edges_scratch_bytes(m.triangle_count);
     if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
     char *dev = nullptr;
-    ST_CUDA(cudaMallocAsync((void **)&dev, bytes, st));
+    ST_CUDA(transient(ctx, (void **)&dev, bytes, st));
     uint32_t *dev_ids = reinterpret_cast<uint32_t *>(dev);
     EdgeVertexIndices *dev_edges = reinterpret_cast<EdgeVertexIndices *>(dev + ((ids_bytes + 255) & ~(size_t)255));
     void *scratch = dev + ((ids_bytes + 255) & ~(size_t)255) + ((edges_bytes + 255) & ~(size_t)255);

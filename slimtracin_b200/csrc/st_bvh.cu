@@ -800,6 +800,19 @@ __global__ void tri_records_kernel(const vec3 *pos, const vec3 *nrm, const vec2 
     out[i] = r;
 }
 
+__global__ void check_indices_kernel(const uint32_t *pidx, const uint32_t *nidx, const uint32_t *uidx, u32t n, u32t n_positions,
+                                     u32t n_normals, u32t n_uvs, unsigned *flag) {
+    bool bad = false;
+    for (u32t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        bad |= pidx[i] >= n_positions || nidx[i] >= n_normals || (n_uvs && uidx[i] >= n_uvs);
+    if (bad) *flag = 1;
+}
+void launch_check_indices(const uint32_t *pidx, const uint32_t *nidx, const uint32_t *uidx, u32t n_indices, u32t n_positions,
+                          u32t n_normals, u32t n_uvs, unsigned *flag, cudaStream_t st) {
+    check_indices_kernel<<<min((n_indices + 255) / 256, 1184u), 256, 0, st>>>(pidx, nidx, uidx, n_indices, n_positions, n_normals,
+                                                                             n_uvs, flag);
+}
+
 // ---- conversions into the traversal layouts ---------------------------------------------------
 __device__ __forceinline__ void make_pair(const BVHNode *nodes, u32t k, NodePair *pairs) {
     const BVHNode L = nodes[1 + 2 * k], R = nodes[2 + 2 * k];

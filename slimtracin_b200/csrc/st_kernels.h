@@ -1,6 +1,7 @@
 // st_kernels.h — host-visible kernel launchers and the per-view parameter block.
 #pragma once
 #include <cstdint>
+#include <initializer_list>
 #include <cuda_runtime.h>
 #include "st_device.cuh"
 
@@ -161,9 +162,9 @@ cudaError_t lbvh_build(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes
 // 1 + 2 * pairs) once `st` reaches it.
 cudaError_t lbvh_enqueue(LbvhScratch &s, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, cudaStream_t st);
 // Binned SAH over n device boxes (st_sah.cu): reference-layout nodes (2n capacity) + leaf order.
-// scratch (optional, sah_scratch_bytes(n) bytes): used instead of a stream-ordered allocation
+// scratch: sah_scratch_bytes(n) bytes.  Waits for the build.
 cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t info[2],
-                      cudaStream_t st, void *scratch = nullptr, size_t scratch_bytes = 0);
+                      cudaStream_t st, void *scratch);
 size_t sah_scratch_bytes(u32t n);
 // Whether sah_enqueue makes the build without waiting for the device on the way.
 bool sah_without_wait(u32t n, u32t max_leaf);
@@ -231,6 +232,25 @@ int obj_parse(const char *path, bool invert_winding, const ObjCounts &expect, ve
 size_t unique_edges_scratch_bytes(u32t n_triangles);
 cudaError_t unique_edges(const uint32_t *dev_ids, u32t n_triangles, u32t n_vertices, void *scratch,
                          EdgeVertexIndices *dev_edges, u32t *n_edges, cudaStream_t st);
+
+// ---- copies from and to pageable host memory (st_stage.cu) ----
+constexpr int kStageThreads = 4;
+struct Stage {                     // a context's staging: page-locked slots, and a stream, per copying thread
+    int device = 0;
+    char *pinned = nullptr;
+    size_t copied = 0;             // bytes that large pageable copies have moved
+    cudaStream_t stream[kStageThreads] = {};
+    cudaEvent_t done[kStageThreads][2] = {}, ready = nullptr;
+};
+struct HostCopy { void *host, *dev; size_t bytes; };
+// The copies, after what is on `st`.  To the host: pageable destinations are filled when it returns,
+// page-locked ones once `st` gets there.  To the device: the sources may be reused when it returns
+// (page-locked ones once `st` gets there), and what is put on `st` afterwards sees the copies.
+cudaError_t stage_copy(Stage &s, std::initializer_list<HostCopy> copies, bool to_host, cudaStream_t st);
+void stage_release(Stage &s);
+// Whether any of a mesh's vertex indices is out of range: *flag (page-locked host memory) is set then.
+void launch_check_indices(const uint32_t *pidx, const uint32_t *nidx, const uint32_t *uidx, u32t n_indices, u32t n_positions,
+                          u32t n_normals, u32t n_uvs, unsigned *flag, cudaStream_t st);
 
 // ---- shared primitives (st_bvh.cu) ----
 // Exclusive scan of n u32 values (in place allowed); sums: (n/1024 + 1) words of scratch; total

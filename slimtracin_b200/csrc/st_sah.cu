@@ -979,19 +979,11 @@ cudaError_t sah_enqueue(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_
 }
 
 cudaError_t sah_build(const float *aabbs, u32t n, u32t max_leaf, BVHNode *out_nodes, u32t *out_order, u32t info[2],
-                      cudaStream_t st, void *scratch, size_t scratch_bytes) {
+                      cudaStream_t st, void *scratch) {
     if (n == 0) { info[0] = info[1] = 0; return cudaSuccess; }
-    const size_t bytes = sah_scratch_bytes(n);
-    // the caller's scratch when it is large enough, else a stream-ordered allocation
-    void *base = scratch;
-    const bool own = !(scratch && scratch_bytes >= bytes);
-    cudaError_t e = cudaSuccess;
-    if (own) e = cudaMallocAsync(&base, bytes, st);
-    if (e != cudaSuccess) return e;
     u32t got[3] = {0, 0, 0}, *dev_info = nullptr;
-    e = sah_enqueue(aabbs, n, max_leaf, out_nodes, out_order, base, &dev_info, st);
+    cudaError_t e = sah_enqueue(aabbs, n, max_leaf, out_nodes, out_order, scratch, &dev_info, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(got, dev_info, sizeof(got), cudaMemcpyDeviceToHost, st);
-    if (own) cudaFreeAsync(base, st);
     const cudaError_t e2 = cudaStreamSynchronize(st);
     info[0] = 1 + 2 * got[2];
     info[1] = got[1] < 1 ? 1 : got[1];
