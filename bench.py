@@ -656,7 +656,7 @@ def main():
             "config": bench_config(world, sd.meshes[0].triangle_count, grid),
             "e2e": {"value": e2e_value, "unit": "Mrays/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "api": "st_upload_primitives + st_render_scene, pinned host buffers"},
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": 3 * args.steps,  # set-up, trace, resolve
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
                          "kernel": "trace_kernel", "kernel_ms": trace_avg_ms,

@@ -214,8 +214,8 @@ typedef struct st_batch_options {
     float batch_ms;             /* out: CUDA-event time of the batch on the launch stream */
     uint64_t rays;              /* out: primary rays traced */
     int tile_shape_used, chunk_used, graph_replayed;   /* out; graph_replayed: an existing graph was updated */
-    int stack_placement;        /* -1: autotuned; 0: traversal stacks in local memory; 1: their first 16
-                                   entries in shared memory (the traversal is the same either way) */
+    int stack_placement;        /* -1: autotuned; 0: traversal stacks in local memory; 1: their first 32
+                                   words in shared memory (the traversal is the same either way) */
     int stack_placement_used;   /* out */
     int launch_mode;            /* st_launch_mode: ST_LAUNCH_AUTOTUNED (-1), ST_LAUNCH_PER_VIEW (0) or
                                    ST_LAUNCH_PERSISTENT (1); tile_shape, chunk and stack_placement apply to

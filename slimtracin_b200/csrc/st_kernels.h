@@ -9,7 +9,7 @@ namespace st {
 
 // One view: what rayTrace / renderSceneOnCPU read from the Viewport and its Camera
 // (raytracer.h:136-170) and what computeSSB reads from the frame buffer's Dimensions (SSB.h:5).
-constexpr int kSegment = 8;        // grid points per stored row-segment start (row_segments_kernel)
+constexpr int kSegment = 8;        // grid points per stored row-segment start (frame_setup_kernel)
 
 struct ViewDev {
     v3 cam_pos;
@@ -31,7 +31,7 @@ struct BatchView {
     SceneDev scene;
     ViewDev view;
     const int4 *ssb;
-    const float *dirs;             // row-segment starts (row_segments_kernel)
+    const float *dirs;             // row-segment starts (frame_setup_kernel)
     FloatPixel *out;
     u32t *prim_ids;
     uint32_t *out_u8;              // resolved frame (device), or null
@@ -51,7 +51,7 @@ struct BatchTable {
 static_assert(sizeof(BatchTable) + 64 <= 32764, "kernel parameters are limited to 32764 bytes");
 enum TileShape { TILE_8x4 = 0, TILE_16x2 = 1, TILE_32x1 = 2, TILE_4x8 = 3, TILE_SHAPES = 4 };
 // A batch kernel variant: tile shape + TILE_SHAPES * stack placement (0: traversal stacks in local
-// memory; 1: their first kSharedStackEntries entries in shared memory).
+// memory; 1: their first 2 * kSharedStackEntries words in shared memory).
 constexpr int kSharedStackEntries = 16;
 constexpr int STACK_PLACEMENTS = 2;
 constexpr int BATCH_VARIANTS = TILE_SHAPES * STACK_PLACEMENTS;

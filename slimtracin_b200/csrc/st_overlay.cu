@@ -426,7 +426,7 @@ __device__ void walk_edge(const OverlayParams &P, const BoxRec *boxes, u32t n_bo
     const u32t s = e - 12 * n_boxes, i = s >> 2;
     if (i >= P.n_prims) return;
     const int4 b = ssb[i];
-    if (b.x == 1 && b.y == 1 && b.z == 0 && b.w == 0) return;    // not visible (ssb_kernel's empty rect)
+    if (b.x == 1 && b.y == 1 && b.z == 0 && b.w == 0) return;    // not visible (ssb_of's empty rect)
     const Primitive &p = P.prims[i];
     const u32t color = p.type == PrimitiveType_Mesh ? 3u : type_color(p.type);
     if (!color) return;

@@ -43,7 +43,7 @@ def check(renderer, boxes, max_leaf):
 
 
 @pytest.mark.parametrize("kind", ["spread", "same", "peel", "clumps", "odd values"])
-@pytest.mark.parametrize("n", [1, 2, 3, 10, 11, 33, 512, 513, 1100, 4096, 4097, 9000])
+@pytest.mark.parametrize("n", [1, 2, 3, 10, 11, 33, 256, 257, 512, 513, 1100, 4096, 4097, 9000])
 def test_binned_sah_equals_specification(renderer, n, kind):
     for max_leaf in (1, 2, 4):
         check(renderer, item_boxes(kind, n), max_leaf)
