@@ -991,7 +991,8 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
     if (e == cudaSuccess) {
         launch_check_indices(pidx, nidx, uidx, 3 * n, mesh->vertex_count, mesh->normals_count, mesh->uvs_count,
                              reinterpret_cast<unsigned *>(ctx->readback_dev + 18), st);
-        e = cudaStreamSynchronize(st);
+        e = cudaGetLastError();              // (a refused launch leaves *bad as if every index were in range)
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
     u32t info[2];
     void *scratch = nullptr;
@@ -1005,10 +1006,12 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
         }
         if (e == cudaSuccess) {
             launch_tri_records(pos, nrm, uv, pidx, nidx, uidx, uvs ? 1 : 0, order, n, tris, inverse, st);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess)
             e = stage_copy(ctx->stage, {{mesh->triangles, tris, sizeof(Triangle) * (size_t)n},
                                         {mesh->bvh.nodes, nodes, sizeof(BVHNode) * (size_t)info[0]},
                                         {mesh->bvh.leaf_ids, inverse, sizeof(u32t) * (size_t)n}}, true, st);
-        }
     }
     if (scratch) cudaFreeAsync(scratch, st);
     cudaFreeAsync(base, st);

@@ -1,0 +1,63 @@
+// The mesh build (st_update_mesh_bvh) on the stand-in runtime; one scenario a process.
+#include <cstdio>
+#include <cstring>
+#include <vector>
+#include "runtime.h"
+#include "slimtracin_b200.h"
+
+namespace st {
+int batch_blocks_per_sm(int) { return 7; }       // (st_render.cu is not linked)
+}
+
+#define EXPECT(x) do { if (!(x)) { printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
+
+// A mesh of `n` triangles over four vertices, its arrays for the build's results.
+struct MeshArrays {
+    std::vector<vec3> positions, normals;
+    std::vector<TriangleVertexIndices> ids;
+    std::vector<Triangle> triangles;
+    std::vector<BVHNode> nodes;
+    std::vector<u32> leaf_ids;
+    Mesh mesh;
+    explicit MeshArrays(u32 n) : positions(4), normals(4), ids(n), triangles(n), nodes(2 * n), leaf_ids(n) {
+        memset(&mesh, 0, sizeof(mesh));
+        mesh.triangle_count = n;
+        mesh.vertex_count = mesh.normals_count = 4;
+        mesh.vertex_positions = positions.data();
+        mesh.vertex_normals = normals.data();
+        mesh.vertex_position_indices = mesh.vertex_normal_indices = ids.data();
+        mesh.triangles = triangles.data();
+        mesh.bvh.nodes = nodes.data();
+        mesh.bvh.leaf_ids = leaf_ids.data();
+        mesh.bvh.node_count = 77;
+    }
+};
+
+// A launch that is refused fails the build, and nothing after it reads what it should have made.
+static int refused_launch(st_ctx *ctx, const char *kernel, const char *must_not_follow) {
+    MeshArrays a(5000);
+    for (int mode : {ST_BVH_BINNED_SAH, ST_BVH_LBVH30}) {
+        fake.log.clear();
+        fake.refuse_kernel = kernel;
+        EXPECT(st_update_mesh_bvh(ctx, &a.mesh, mode) == ST_ERR_CUDA);
+        EXPECT(a.mesh.bvh.node_count == 77);
+        EXPECT(!*must_not_follow || fake.log.find(must_not_follow) == std::string::npos);
+        fake.refuse_kernel.clear();
+        EXPECT(st_update_mesh_bvh(ctx, &a.mesh, mode) == ST_OK);
+        a.mesh.bvh.node_count = 77;
+    }
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    st_ctx *ctx = nullptr;
+    if (what == "refused_launch") {
+        EXPECT(st_init(&ctx, nullptr) == ST_OK);
+        const int r = refused_launch(ctx, argv[2], argv[3]);
+        st_shutdown(ctx);
+        return r;
+    }
+    printf("no such scenario\n");
+    return 2;
+}

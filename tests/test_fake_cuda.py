@@ -1,0 +1,50 @@
+"""What the library does when a CUDA call is refused or memory is short, on a stand-in for the CUDA
+runtime (tests/fake_cuda) linked with the library's own host code: no GPU, and nothing on one, fails."""
+import os
+import subprocess
+from concurrent.futures import ThreadPoolExecutor
+
+import pytest
+
+from slimtracin_b200 import build
+
+HERE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "fake_cuda")
+LIBRARY = ["st_api", "st_bvh", "st_sah", "st_stage", "st_texture", "st_io", "st_obj"]
+DRIVERS = ["ingest"]
+
+
+@pytest.fixture(scope="module")
+def drivers(tmp_path_factory):
+    """The driver programs: the library's host code, one driver and the stand-in runtime each."""
+    out = tmp_path_factory.mktemp("fake_cuda")
+    flags = ["-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "--fmad=false", "-Xcompiler", "-fPIC"]
+    flags += sum([["-I", d] for d in build.INCLUDES + [HERE]], [])
+
+    def compile_one(src):
+        obj = str(out / (os.path.basename(src).rsplit(".", 1)[0] + ".o"))
+        subprocess.run([build._nvcc()] + flags + ["-c", src, "-o", obj], check=True)
+        return obj
+
+    sources = [os.path.join(build.CSRC, f + ".cu") for f in LIBRARY]
+    sources += [os.path.join(HERE, f + ".cpp") for f in ["runtime"] + DRIVERS]
+    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        objs = dict(zip([os.path.basename(s).rsplit(".", 1)[0] for s in sources], pool.map(compile_one, sources)))
+    # what the drivers never reach (rendering, graphs) is left out, and unresolved
+    subprocess.run(["g++", "-shared", "-o", str(out / "library.so"), objs["runtime"]] + [objs[f] for f in LIBRARY]
+                   + ["-lpthread", "-Wl,-z,lazy"], check=True)
+    for d in DRIVERS:
+        subprocess.run(["g++", "-o", str(out / d), objs[d], str(out / "library.so"), "-lpthread", "-rdynamic", "-Wl,-z,lazy",
+                        "-Wl,--allow-shlib-undefined"], check=True)
+    return out
+
+
+def run(drivers, name, *args):
+    p = subprocess.run([str(drivers / name), *args], capture_output=True, text=True, timeout=60)
+    assert p.returncode == 0, (p.returncode, p.stdout, p.stderr)
+
+
+@pytest.mark.parametrize("kernel,must_not_follow", [("check_indices_kernel", "tri_aabbs_kernel"), ("tri_aabbs_kernel", "tri_records_kernel"),
+                                                    ("tri_records_kernel", "")])
+def test_refused_launch_fails_the_mesh_build(drivers, kernel, must_not_follow):
+    """Above all that of the check on which the reads through the mesh's indices rely."""
+    run(drivers, "ingest", "refused_launch", kernel, must_not_follow)
