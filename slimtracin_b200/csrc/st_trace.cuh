@@ -112,10 +112,12 @@ __device__ __forceinline__ Slabs prepare(v3 org, v3 dir) {
 
 // hitAABB render/AABB.h:6, from the six plane distances of a box: the direction's sign picks each
 // axis' entry plane, as in the reference; the axes meet in three-operand minima and maxima instead of
-// its compare chain.  The values are the same unless a distance is NaN, which takes a NaN box bound (a
-// mesh with a NaN vertex): that axis is then left out, where the chain also drops a neighbouring one
-// and visits boxes that hold no point of the ray.  A walk step is bound by its dependent instructions, not by bandwidth: with the
-// planes of a pair multiplied and added two at a time (mul_add2) it takes about 65 instructions
+// its compare chain.  The values are the same unless a distance is NaN: a box bound that is (a mesh with
+// a NaN vertex), an origin that is (an instance with a zero scale), or a bound and an origin both beyond
+// 2^28 on an axis the ray does not move along.  That axis is then left out, where the chain also drops a
+// neighbouring one and visits boxes that hold no point of the ray.  `closest` must be a number: the chain
+// admits nothing where it is NaN.  A walk step is bound by its dependent instructions, not by bandwidth:
+// with the planes of a pair multiplied and added two at a time (mul_add2) it takes about 65 instructions
 // against 100; without the pairing the 4096-primitive moving scene traces in 1.08 ms instead of
 // 1.05, the mesh frames in 1 to 2 % more.
 __device__ __forceinline__ float min3(float a, float b, float c) {
