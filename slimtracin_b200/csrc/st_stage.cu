@@ -7,8 +7,8 @@
 // and a stream of its own, so that one slot is filled or emptied while the other is on the bus; a whole
 // updateMeshBVH of 327,680 triangles went from 6.5 to 4.7 ms with it, a bake from 1.9 to 1.5 (slots of
 // 1 MB: 3.6 and 1.5, of 64 KB 7.5 and 2.1).  Page-locking the slots costs 1 to 5 ms, 12 to 24 for 8 MB
-// of them, which takes some 60 MB of copies to earn back: a context's first kStageAfter bytes go the
-// plain way.  Page-locked host memory is copied directly, small copies as they are.
+// of them, which takes some 60 MB of copies to earn back: a context's first kStageAfter pageable bytes
+// go the plain way.  Page-locked host memory is copied directly and does not count, small copies as they are.
 #include <algorithm>
 #include <cstring>
 #include <system_error>
@@ -21,7 +21,7 @@ namespace st {
 namespace {
 
 constexpr size_t kSlotBytes = 256 << 10;
-constexpr size_t kStagedFrom = 2 << 20;        // less than this in one call is not worth the threads
+constexpr size_t kStagedFrom = 2 << 20;        // less pageable than this in one call is not worth the threads
 constexpr size_t kStageAfter = 64 << 20;
 
 struct Chunk { char *host, *dev; size_t bytes; };
@@ -94,8 +94,16 @@ void stage_release(Stage &s) {
 
 cudaError_t stage_copy(Stage &s, std::initializer_list<HostCopy> copies, bool to_host, cudaStream_t st) {
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
-    size_t total = 0;
-    for (const HostCopy &c : copies) total += c.bytes;
+    auto pageable = [](const HostCopy &c) {
+        cudaPointerAttributes a;
+        const bool locked = cudaPointerGetAttributes(&a, c.host) == cudaSuccess && a.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        return !locked;
+    };
+    size_t all = 0, total = 0;                         // of all, of the pageable ones
+    for (const HostCopy &c : copies) all += c.bytes;
+    if (all >= kStagedFrom)
+        for (const HostCopy &c : copies) total += c.bytes && pageable(c) ? c.bytes : 0;
     bool staged = false;
     if (total >= kStagedFrom) {
         staged = s.copied >= kStageAfter && stage_ready(s);
@@ -104,10 +112,7 @@ cudaError_t stage_copy(Stage &s, std::initializer_list<HostCopy> copies, bool to
     cudaError_t e = cudaSuccess;
     std::vector<Chunk> chunks;
     for (const HostCopy &c : copies) {
-        cudaPointerAttributes a;
-        const bool locked = staged && cudaPointerGetAttributes(&a, c.host) == cudaSuccess && a.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        if (!staged || locked) {
+        if (!staged || !pageable(c)) {
             if (c.bytes && e == cudaSuccess) e = cudaMemcpyAsync(to_host ? c.host : c.dev, to_host ? c.dev : c.host, c.bytes, kind, st);
             continue;
         }

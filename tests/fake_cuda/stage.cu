@@ -1,0 +1,55 @@
+// stage_copy (st_stage.cu) on the stand-in runtime; one scenario a process.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+#include "runtime.h"
+#include "st_kernels.h"
+
+#define EXPECT(x) do { if (!(x)) { printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
+
+using namespace st;
+
+constexpr size_t MB = (size_t)1 << 20;
+static cudaStream_t stream;
+
+struct Buffers {
+    std::vector<char> pageable;
+    char *locked = nullptr, *dev = nullptr;
+    cudaMemPool_t pool = nullptr;
+    explicit Buffers(size_t bytes) : pageable(bytes) {
+        cudaMallocHost((void **)&locked, bytes);
+        cudaMemPoolProps props = {};
+        cudaMemPoolCreate(&pool, &props);
+        cudaMallocFromPoolAsync((void **)&dev, bytes, pool, stream);
+        for (size_t i = 0; i < bytes; i++) pageable[i] = locked[i] = (char)(i * 7 + (i >> 12));
+    }
+};
+
+// Page-locked arrays are copied directly: they make no slots however many bytes have gone by, nor does a
+// call whose pageable part is small.  Pageable ones make them, after the first 64 MB.
+static int locked_only() {
+    Stage s;
+    Buffers b(8 * MB);
+    const int allocs = fake.host_allocs, streams = fake.streams;
+    for (int k = 0; k < 20; k++)
+        for (bool to_host : {false, true})
+            EXPECT(stage_copy(s, {{b.locked, b.dev, 7 * MB}, {b.pageable.data(), b.dev + 7 * MB, MB / 4}}, to_host, stream) == cudaSuccess);
+    EXPECT(!s.pinned && fake.host_allocs == allocs && fake.streams == streams);
+    for (int k = 0; k < 8; k++) {
+        EXPECT(stage_copy(s, {{b.pageable.data(), b.dev, 8 * MB}}, false, stream) == cudaSuccess);
+        EXPECT(!s.pinned);
+    }
+    EXPECT(stage_copy(s, {{b.pageable.data(), b.dev, 8 * MB}}, false, stream) == cudaSuccess);
+    EXPECT(s.pinned && !memcmp(b.dev, b.pageable.data(), 8 * MB));
+    stage_release(s);
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    cudaStreamCreateWithFlags(&stream, 0);
+    if (what == "locked_only") return locked_only();
+    printf("no such scenario\n");
+    return 2;
+}

@@ -10,7 +10,7 @@ from slimtracin_b200 import build
 
 HERE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "fake_cuda")
 LIBRARY = ["st_api", "st_bvh", "st_sah", "st_stage", "st_texture", "st_io", "st_obj"]
-DRIVERS = ["ingest"]
+DRIVERS = ["ingest.cpp", "stage.cu"]
 
 
 @pytest.fixture(scope="module")
@@ -26,13 +26,13 @@ def drivers(tmp_path_factory):
         return obj
 
     sources = [os.path.join(build.CSRC, f + ".cu") for f in LIBRARY]
-    sources += [os.path.join(HERE, f + ".cpp") for f in ["runtime"] + DRIVERS]
+    sources += [os.path.join(HERE, f) for f in ["runtime.cpp"] + DRIVERS]
     with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
         objs = dict(zip([os.path.basename(s).rsplit(".", 1)[0] for s in sources], pool.map(compile_one, sources)))
     # what the drivers never reach (rendering, graphs) is left out, and unresolved
     subprocess.run(["g++", "-shared", "-o", str(out / "library.so"), objs["runtime"]] + [objs[f] for f in LIBRARY]
                    + ["-lpthread", "-Wl,-z,lazy"], check=True)
-    for d in DRIVERS:
+    for d in [f.split(".")[0] for f in DRIVERS]:
         subprocess.run(["g++", "-o", str(out / d), objs[d], str(out / "library.so"), "-lpthread", "-rdynamic", "-Wl,-z,lazy",
                         "-Wl,--allow-shlib-undefined"], check=True)
     return out
@@ -48,3 +48,7 @@ def run(drivers, name, *args):
 def test_refused_launch_fails_the_mesh_build(drivers, kernel, must_not_follow):
     """Above all that of the check on which the reads through the mesh's indices rely."""
     run(drivers, "ingest", "refused_launch", kernel, must_not_follow)
+
+
+def test_page_locked_copies_make_no_slots(drivers):
+    run(drivers, "stage", "locked_only")
