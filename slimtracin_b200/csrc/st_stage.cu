@@ -96,9 +96,9 @@ cudaError_t stage_copy(Stage &s, std::initializer_list<HostCopy> copies, bool to
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
     auto pageable = [](const HostCopy &c) {
         cudaPointerAttributes a;
-        const bool locked = cudaPointerGetAttributes(&a, c.host) == cudaSuccess && a.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        return !locked;
+        if (cudaPointerGetAttributes(&a, c.host) == cudaSuccess) return a.type != cudaMemoryTypeHost;
+        cudaGetLastError();                            // (of this call alone: an earlier error is the caller's)
+        return true;
     };
     size_t all = 0, total = 0;                         // of all, of the pageable ones
     for (const HostCopy &c : copies) all += c.bytes;

@@ -46,10 +46,26 @@ static int locked_only() {
     return 0;
 }
 
+// An error that something before left for the caller to see is still there afterwards.
+static int keeps_errors() {
+    Stage s;
+    s.copied = 64 * MB;
+    Buffers b(4 * MB);
+    void *p;
+    fake.device_bytes = 0;
+    EXPECT(cudaMalloc(&p, 1) == cudaErrorMemoryAllocation);
+    fake.device_bytes = (size_t)1 << 40;
+    for (bool to_host : {false, true})
+        EXPECT(stage_copy(s, {{b.pageable.data(), b.dev, 3 * MB}, {b.locked, b.dev, MB}}, to_host, stream) == cudaSuccess);
+    EXPECT(s.pinned && cudaGetLastError() == cudaErrorMemoryAllocation);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     cudaStreamCreateWithFlags(&stream, 0);
     if (what == "locked_only") return locked_only();
+    if (what == "keeps_errors") return keeps_errors();
     printf("no such scenario\n");
     return 2;
 }

@@ -52,3 +52,7 @@ def test_refused_launch_fails_the_mesh_build(drivers, kernel, must_not_follow):
 
 def test_page_locked_copies_make_no_slots(drivers):
     run(drivers, "stage", "locked_only")
+
+
+def test_copies_keep_an_earlier_error(drivers):
+    run(drivers, "stage", "keeps_errors")
