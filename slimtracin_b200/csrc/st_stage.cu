@@ -137,6 +137,8 @@ cudaError_t stage_copy(Stage &s, std::initializer_list<HostCopy> copies, bool to
         // what follows on `st` comes after the copies
         for (int k = 0; k < 2 && !to_host && e == cudaSuccess; k++) e = cudaStreamWaitEvent(st, s.done[t][k], 0);
     }
+    // where one failed the others are not left on the bus: the caller gives up the memory they use
+    for (int t = 0; t < kStageThreads && e != cudaSuccess; t++) cudaStreamSynchronize(s.stream[t]);
     return e;
 }
 

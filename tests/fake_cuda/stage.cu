@@ -61,11 +61,45 @@ static int keeps_errors() {
     return 0;
 }
 
+// Whichever of a call's copies is refused, the others are over, or before what the stream does next, when
+// the call returns with the error: the caller gives the device memory back then.
+static int refused_copies(bool to_host) {
+    Stage s;
+    s.copied = 64 * MB;
+    Buffers b(5 * MB + 12345);
+    auto copy = [&] {
+        return stage_copy(s, {{b.pageable.data(), b.dev, 3 * MB}, {b.pageable.data() + 3 * MB, b.dev + 3 * MB, 2 * MB + 12345}},
+                          to_host, stream);
+    };
+    EXPECT(copy() == cudaSuccess);
+    int refused = 0;
+    for (int k = 1; k <= 24; k++) {
+        cudaStreamSynchronize(stream);
+        fake.fail_copy = k;
+        const cudaError_t e = copy();
+        refused += e != cudaSuccess;
+        EXPECT(fake.fail_copy ? e == cudaSuccess : e == cudaErrorInvalidValue);
+        fake.fail_copy = 0;
+        cudaGetLastError();
+        cudaFreeAsync(b.dev, stream);
+        EXPECT(fake.unordered_frees == 0);
+        EXPECT(!to_host || fake.in_flight() == 0);
+        cudaMallocFromPoolAsync((void **)&b.dev, 5 * MB + 12345, b.pool, stream);
+        // and the slots are fit for the next call
+        for (size_t i = 0; i < 5 * MB + 12345; i++) (to_host ? b.dev : b.pageable.data())[i] = (char)(i * k);
+        EXPECT(stage_copy(s, {{b.pageable.data(), b.dev, 5 * MB + 12345}}, to_host, stream) == cudaSuccess);
+        EXPECT(!memcmp(b.pageable.data(), b.dev, 5 * MB + 12345));
+    }
+    EXPECT(refused == 21);                             // 256 KB at a time
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     cudaStreamCreateWithFlags(&stream, 0);
     if (what == "locked_only") return locked_only();
     if (what == "keeps_errors") return keeps_errors();
+    if (what == "refused_copies") return refused_copies(argv[2] == std::string("to_host"));
     printf("no such scenario\n");
     return 2;
 }

@@ -56,3 +56,8 @@ def test_page_locked_copies_make_no_slots(drivers):
 
 def test_copies_keep_an_earlier_error(drivers):
     run(drivers, "stage", "keeps_errors")
+
+
+@pytest.mark.parametrize("direction", ["to_host", "to_device"])
+def test_a_refused_copy_leaves_none_in_flight(drivers, direction):
+    run(drivers, "stage", "refused_copies", direction)
