@@ -11,9 +11,7 @@
 // go the plain way.  Page-locked host memory is copied directly and does not count, small copies as they are.
 #include <algorithm>
 #include <cstring>
-#include <system_error>
 #include <thread>
-#include <vector>
 #include "st_kernels.h"
 
 namespace st {
@@ -23,19 +21,40 @@ namespace {
 constexpr size_t kSlotBytes = 256 << 10;
 constexpr size_t kStagedFrom = 2 << 20;        // less pageable than this in one call is not worth the threads
 constexpr size_t kStageAfter = 64 << 20;
+constexpr int kStageArrays = 8;                // a call's arrays that can go through the slots (a mesh build's: 6)
 
 struct Chunk { char *host, *dev; size_t bytes; };
 
+// The copies that go through the slots, a slot's size at a time.  (No allocation: an exception must not
+// leave the C entry points above, nor a thread.)
+struct Chunks {
+    HostCopy copies[kStageArrays];
+    int arrays = 0;
+    size_t count = 0;
+    static size_t of(const HostCopy &c) { return (c.bytes + kSlotBytes - 1) / kSlotBytes; }
+    void add(const HostCopy &c) {
+        copies[arrays++] = c;
+        count += of(c);
+    }
+    Chunk at(size_t k) const {
+        const HostCopy *c = copies;
+        for (; k >= of(*c); c++) k -= of(*c);
+        const size_t at = k * kSlotBytes;
+        return {static_cast<char *>(c->host) + at, static_cast<char *>(c->dev) + at, std::min(kSlotBytes, c->bytes - at)};
+    }
+};
+
 // Thread t's chunks: t, t + kStageThreads, ...
-cudaError_t copy_share(Stage &s, int t, const std::vector<Chunk> &chunks, bool to_host) {
+cudaError_t copy_share(Stage &s, int t, const Chunks &chunks, bool to_host) {
     cudaError_t e = cudaSetDevice(s.device);
     cudaStream_t st = s.stream[t];
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, s.ready, 0);
-    const size_t count = chunks.size() > (size_t)t ? (chunks.size() - t - 1) / kStageThreads + 1 : 0;
-    auto chunk = [&](size_t j) -> const Chunk & { return chunks[t + j * kStageThreads]; };
+    const size_t count = chunks.count > (size_t)t ? (chunks.count - t - 1) / kStageThreads + 1 : 0;
+    auto chunk = [&](size_t j) { return chunks.at(t + j * kStageThreads); };
     auto slot = [&](size_t j) { return s.pinned + (2 * t + (j & 1)) * kSlotBytes; };
     auto fetch = [&](size_t j) {
-        cudaError_t r = cudaMemcpyAsync(slot(j), chunk(j).dev, chunk(j).bytes, cudaMemcpyDeviceToHost, st);
+        const Chunk c = chunk(j);
+        cudaError_t r = cudaMemcpyAsync(slot(j), c.dev, c.bytes, cudaMemcpyDeviceToHost, st);
         return r == cudaSuccess ? cudaEventRecord(s.done[t][j & 1], st) : r;
     };
     // (a slot may still be on the bus for the call before)
@@ -45,15 +64,17 @@ cudaError_t copy_share(Stage &s, int t, const std::vector<Chunk> &chunks, bool t
         for (size_t j = 0; j < count && e == cudaSuccess; j++) {
             e = cudaEventSynchronize(s.done[t][j & 1]);
             if (e != cudaSuccess) break;
-            memcpy(chunk(j).host, slot(j), chunk(j).bytes);
+            const Chunk c = chunk(j);
+            memcpy(c.host, slot(j), c.bytes);
             if (j + 2 < count) e = fetch(j + 2);
         }
     } else {
         for (size_t j = 0; j < count && e == cudaSuccess; j++) {
             e = cudaEventSynchronize(s.done[t][j & 1]);
             if (e != cudaSuccess) break;
-            memcpy(slot(j), chunk(j).host, chunk(j).bytes);
-            e = cudaMemcpyAsync(chunk(j).dev, slot(j), chunk(j).bytes, cudaMemcpyHostToDevice, st);
+            const Chunk c = chunk(j);
+            memcpy(slot(j), c.host, c.bytes);
+            e = cudaMemcpyAsync(c.dev, slot(j), c.bytes, cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess) e = cudaEventRecord(s.done[t][j & 1], st);
         }
     }
@@ -110,16 +131,12 @@ cudaError_t stage_copy(Stage &s, std::initializer_list<HostCopy> copies, bool to
         s.copied += total;
     }
     cudaError_t e = cudaSuccess;
-    std::vector<Chunk> chunks;
+    Chunks chunks;
     for (const HostCopy &c : copies) {
-        if (!staged || !pageable(c)) {
-            if (c.bytes && e == cudaSuccess) e = cudaMemcpyAsync(to_host ? c.host : c.dev, to_host ? c.dev : c.host, c.bytes, kind, st);
-            continue;
-        }
-        for (size_t at = 0; at < c.bytes; at += kSlotBytes)
-            chunks.push_back({static_cast<char *>(c.host) + at, static_cast<char *>(c.dev) + at, std::min(kSlotBytes, c.bytes - at)});
+        if (staged && chunks.arrays < kStageArrays && pageable(c)) chunks.add(c);
+        else if (c.bytes && e == cudaSuccess) e = cudaMemcpyAsync(to_host ? c.host : c.dev, to_host ? c.dev : c.host, c.bytes, kind, st);
     }
-    if (e != cudaSuccess || chunks.empty()) return e;
+    if (e != cudaSuccess || !chunks.count) return e;
     if ((e = cudaEventRecord(s.ready, st)) != cudaSuccess) return e;
     cudaError_t got[kStageThreads] = {};
     std::thread threads[kStageThreads];
@@ -127,7 +144,7 @@ cudaError_t stage_copy(Stage &s, std::initializer_list<HostCopy> copies, bool to
     try {
         for (; started < kStageThreads; started++)
             threads[started] = std::thread([&, t = started] { got[t] = copy_share(s, t, chunks, to_host); });
-    } catch (const std::system_error &) {              // no more threads: the caller takes the other shares
+    } catch (...) {                                    // no more threads, or memory: the caller takes the other shares
     }
     got[0] = copy_share(s, 0, chunks, to_host);
     for (int t = started; t < kStageThreads; t++) got[t] = copy_share(s, t, chunks, to_host);

@@ -4,14 +4,30 @@
 // every stream's copies, and the host learns of their end by waiting.  Linked with the library's own
 // objects in place of cudart.
 #include <cuda_runtime.h>
+#include <dlfcn.h>
+#include <pthread.h>
+#include <cerrno>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <vector>
 #include "runtime.h"
 
 FakeRuntime fake;
+static thread_local int fake_inside = 0;         // > 0 in the stand-in itself
+
+void *operator new(size_t bytes) {
+    if (!fake_inside && fake.fail_new > 0 && --fake.fail_new == 0) throw std::bad_alloc();
+    return malloc(bytes);
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
+extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *arg) {
+    static auto real = reinterpret_cast<decltype(&pthread_create)>(dlsym(RTLD_NEXT, "pthread_create"));
+    return fake.no_threads ? EAGAIN : real(t, a, f, arg);
+}
 
 namespace {
 typedef std::map<const void *, long> Clock;      // stream -> its copies that are known to come before
@@ -27,7 +43,11 @@ struct Pool { size_t reserved = 0, used = 0; uint64_t threshold = 0; std::map<ch
 std::map<char *, Pool *> pool_of;
 thread_local cudaError_t last = cudaSuccess;
 
-typedef std::lock_guard<std::recursive_mutex> Lock;
+struct Lock {
+    std::lock_guard<std::recursive_mutex> guard;
+    explicit Lock(std::recursive_mutex &mutex) : guard(mutex) { fake_inside++; }
+    ~Lock() { fake_inside--; }
+};
 cudaError_t fail(cudaError_t e) { return last = e; }
 void merge(Clock &into, const Clock &from) {
     for (auto &kv : from) if (into[kv.first] < kv.second) into[kv.first] = kv.second;

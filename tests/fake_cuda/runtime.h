@@ -1,5 +1,6 @@
 // What a test driver sets and reads of the stand-in CUDA runtime (runtime.cpp).
 #pragma once
+#include <atomic>
 #include <cstddef>
 #include <string>
 
@@ -8,6 +9,8 @@ struct FakeRuntime {
     size_t device_bytes = (size_t)1 << 40;   // cudaMalloc and pool growth fail beyond this
     int fail_copy = 0;                       // > 0: the n-th cudaMemcpyAsync from now fails
     std::string refuse_kernel;               // launches of kernels whose name contains this fail
+    std::atomic<int> fail_new{0};            // > 0: the n-th operator new from now throws (the stand-in's own excepted)
+    bool no_threads = false;                 // no further thread can be made
     // read by a driver
     size_t device_held = 0;                  // what cudaMalloc and the pools hold of it
     int host_allocs = 0, streams = 0, launches = 0, trims = 0;

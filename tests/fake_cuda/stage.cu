@@ -94,12 +94,32 @@ static int refused_copies(bool to_host) {
     return 0;
 }
 
+// Without memory for it, or without more threads, a copy is still made, and no exception leaves it.
+static int no_resources() {
+    Stage s;
+    s.copied = 64 * MB;
+    Buffers b(5 * MB);
+    for (bool to_host : {false, true}) {
+        for (int k = 0; k <= 12; k++) {
+            for (size_t i = 0; i < 5 * MB; i++) (to_host ? b.dev : b.pageable.data())[i] = (char)(i * 3 + k);
+            fake.fail_new = k;
+            fake.no_threads = k == 0;
+            const cudaError_t e = stage_copy(s, {{b.pageable.data(), b.dev, 5 * MB}}, to_host, stream);
+            fake.fail_new = 0;
+            fake.no_threads = false;
+            EXPECT(e == cudaSuccess && !memcmp(b.pageable.data(), b.dev, 5 * MB));
+        }
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     cudaStreamCreateWithFlags(&stream, 0);
     if (what == "locked_only") return locked_only();
     if (what == "keeps_errors") return keeps_errors();
     if (what == "refused_copies") return refused_copies(argv[2] == std::string("to_host"));
+    if (what == "no_resources") return no_resources();
     printf("no such scenario\n");
     return 2;
 }

@@ -61,3 +61,7 @@ def test_copies_keep_an_earlier_error(drivers):
 @pytest.mark.parametrize("direction", ["to_host", "to_device"])
 def test_a_refused_copy_leaves_none_in_flight(drivers, direction):
     run(drivers, "stage", "refused_copies", direction)
+
+
+def test_copies_without_memory_or_threads(drivers):
+    run(drivers, "stage", "no_resources")
