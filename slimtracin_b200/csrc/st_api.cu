@@ -217,6 +217,7 @@ struct st_ctx {
 namespace {
 
 int fail_cuda(st_ctx *ctx, cudaError_t e) {
+    cudaGetLastError();                  // reported here: not again by the next call that looks after its launches
     ctx->cuda_error = cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? ST_ERR_OUT_OF_MEMORY : ST_ERR_CUDA;
 }
@@ -279,6 +280,11 @@ int reserve(st_ctx *ctx, DevBuf &b, size_t bytes) {
     b.bytes = bytes;
     ctx->in_use += bytes;
     return ST_OK;
+}
+// The builders' scratch for n items.
+int builder_room(st_ctx *ctx, u32t n) {
+    const cudaError_t e = lbvh_reserve(ctx->lbvh, n);
+    return e == cudaSuccess ? ST_OK : fail_cuda(ctx, e);
 }
 #define ST_TRY(x)                    \
     do {                             \
@@ -852,7 +858,7 @@ static int tlas_staging(st_ctx *ctx, u32t n, TlasStaging &t) {
 static int update_scene_once(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode, cudaStream_t st) {
     const u32t n = S->n_prims;
     const bool refit = mode == ST_BVH_REFIT, host = scene && scene->bvh.nodes && scene->bvh.leaf_ids;
-    if (!refit && lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
+    if (!refit) ST_TRY(builder_room(ctx, n));
     TlasStaging t;
     ST_TRY(tlas_staging(ctx, n, t));
     if (!host) {
@@ -906,7 +912,7 @@ static int build_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode, cu
         (mode == ST_BVH_BINNED_SAH && sah_without_wait(n, MAX_OBJS_PER_SCENE_BVH_NODE)))
         return update_scene_once(ctx, S, scene, mode, st);
     if (mode == ST_BVH_BINNED_SAH) {
-        if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
+        ST_TRY(builder_room(ctx, n));
         launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, ctx->stream);
         u32t info[2];
         ST_TRY(reserve(ctx, ctx->sah_scratch, sah_scratch_bytes(n)));
@@ -917,7 +923,7 @@ static int build_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode, cu
         S->tlas_height = info[1];
         if (S->tlas_height + 2 > (u32t)kStack) return ST_ERR_BAD_SCENE;
     } else if (mode == ST_BVH_REF_SAH) {
-        if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
+        ST_TRY(builder_room(ctx, n));
         launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, ctx->stream);
         u32t info[2];
         cudaError_t e = refsah_build(ctx->lbvh.aabbs, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes),
@@ -958,7 +964,7 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
     cudaSetDevice(ctx->device);
     const u32t n = mesh->triangle_count;
     if (!n) return ST_ERR_BAD_SCENE;
-    if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
+    ST_TRY(builder_room(ctx, n));
     cudaStream_t st = ctx->stream;
     size_t bytes = sizeof(vec3) * (mesh->vertex_count + mesh->normals_count) + sizeof(vec2) * (mesh->uvs_count + 1) +
                    sizeof(uint32_t) * 9 * (size_t)n + sizeof(BVHNode) * 2 * (size_t)n + sizeof(u32t) * 2 * (size_t)n +
@@ -1030,7 +1036,7 @@ int st_build_bvh(st_ctx *ctx, int mode, const float *aabbs, uint32_t n, uint32_t
         (mode != ST_BVH_LBVH30 && mode != ST_BVH_BINNED_SAH && mode != ST_BVH_REF_SAH))
         return ST_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
-    if (lbvh_reserve(ctx->lbvh, n) != cudaSuccess) return ST_ERR_OUT_OF_MEMORY;
+    ST_TRY(builder_room(ctx, n));
     cudaStream_t st = ctx->stream;
     char *base = nullptr;
     const size_t bytes = sizeof(BVHNode) * 2 * (size_t)n + sizeof(u32t) * 2 * (size_t)n + 512;

@@ -49,15 +49,31 @@ static int refused_launch(st_ctx *ctx, const char *kernel, const char *must_not_
     return 0;
 }
 
+// An allocation that one call is refused, wherever it is, is that call's error and no later one's.
+static int refused_allocation(st_ctx *ctx) {
+    const size_t all = fake.device_bytes;
+    for (u32 n : {2000u, 5000u, 40000u}) {           // (larger each time, so that the builder's scratch grows)
+        MeshArrays a(n);
+        for (size_t room : {(size_t)1000, (size_t)40 * n, (size_t)300 * n, (size_t)1 << 20}) {
+            fake.device_bytes = fake.device_held + room;
+            const int r = st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_BINNED_SAH);
+            EXPECT(r == ST_OK || r == ST_ERR_OUT_OF_MEMORY);
+            fake.device_bytes = all;
+            if (r == ST_OK) break;
+        }
+        EXPECT(st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_LBVH30) == ST_OK);
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     st_ctx *ctx = nullptr;
-    if (what == "refused_launch") {
-        EXPECT(st_init(&ctx, nullptr) == ST_OK);
-        const int r = refused_launch(ctx, argv[2], argv[3]);
-        st_shutdown(ctx);
-        return r;
-    }
-    printf("no such scenario\n");
-    return 2;
+    int r = 2;
+    EXPECT(st_init(&ctx, nullptr) == ST_OK);
+    if (what == "refused_launch") r = refused_launch(ctx, argv[2], argv[3]);
+    else if (what == "refused_allocation") r = refused_allocation(ctx);
+    else printf("no such scenario\n");
+    st_shutdown(ctx);
+    return r;
 }

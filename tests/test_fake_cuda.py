@@ -65,3 +65,7 @@ def test_a_refused_copy_leaves_none_in_flight(drivers, direction):
 
 def test_copies_without_memory_or_threads(drivers):
     run(drivers, "stage", "no_resources")
+
+
+def test_a_refused_allocation_fails_no_later_call(drivers):
+    run(drivers, "ingest", "refused_allocation")
