@@ -676,7 +676,9 @@ int st_upload_scene_bvh(st_ctx *ctx, int slot, const Scene *scene) {
     cudaSetDevice(ctx->device);
     ST_TRY(ensure(ctx, *S, scene));
     const u32t n = scene->settings.primitives;
-    if (!check_bvh(scene->bvh.nodes, scene->bvh.node_count, n, scene->bvh.height)) return ST_ERR_BAD_SCENE;
+    // (nodes that no other leads to pass the check, and would run past the arrays made for n primitives)
+    if (!check_bvh(scene->bvh.nodes, scene->bvh.node_count, n, scene->bvh.height) || scene->bvh.node_count > 2 * (uint64_t)n)
+        return ST_ERR_BAD_SCENE;
     for (u32t i = 0; i < n; i++) if (scene->bvh.leaf_ids[i] >= n) return ST_ERR_BAD_SCENE;
     S->tlas_node_count = scene->bvh.node_count;
     S->tlas_height = scene->bvh.height;
@@ -701,7 +703,8 @@ int st_upload_mesh_bvhs(st_ctx *ctx, int slot, const Scene *scene) {
     u32t tri_off = 0, pair_off = 0;
     for (u32t m = 0; m < scene->settings.meshes; m++) {
         const Mesh &M = scene->meshes[m];
-        if (!M.triangles || !M.bvh.nodes || !check_bvh(M.bvh.nodes, M.bvh.node_count, M.triangle_count, M.bvh.height))
+        if (!M.triangles || !M.bvh.nodes || !check_bvh(M.bvh.nodes, M.bvh.node_count, M.triangle_count, M.bvh.height) ||
+            (M.bvh.node_count - 1) / 2 > M.triangle_count)       // (as in st_upload_scene_bvh: a pair per triangle)
             return ST_ERR_BAD_SCENE;
         MeshDev d;
         memset(&d, 0, sizeof(d));

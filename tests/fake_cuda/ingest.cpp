@@ -66,6 +66,54 @@ static int refused_allocation(st_ctx *ctx) {
     return 0;
 }
 
+// A scene of n boxes, their TLAS, and one mesh of n triangles, each tree one split and two leaves; `extra`
+// nodes more, which no other leads to.
+struct SceneArrays {
+    std::vector<Primitive> prims;
+    std::vector<Material> materials;
+    std::vector<BVHNode> nodes;
+    std::vector<u32> ids;
+    MeshArrays mesh;
+    Scene scene;
+    SceneArrays(u32 n, u32 extra) : prims(n), materials(1), nodes(3 + extra), ids(n), mesh(n) {
+        memset(&scene, 0, sizeof(scene));
+        for (u32 i = 0; i < n; i++) {
+            prims[i].type = PrimitiveType_Box;
+            ids[i] = i;
+        }
+        nodes[0].first_child_id = 1;
+        nodes[1].child_count = 1;
+        nodes[2].first_child_id = 1;
+        nodes[2].child_count = (u16)(n - 1);
+        for (u32 k = 3; k < 3 + extra; k++) nodes[k] = nodes[1];
+        mesh.mesh.bvh.nodes = scene.bvh.nodes = nodes.data();
+        mesh.mesh.bvh.node_count = scene.bvh.node_count = 3 + extra;
+        mesh.mesh.bvh.height = scene.bvh.height = 1;
+        mesh.mesh.bvh.leaf_ids = scene.bvh.leaf_ids = ids.data();
+        scene.primitives = prims.data();
+        scene.materials = materials.data();
+        scene.meshes = &mesh.mesh;
+        scene.settings.primitives = n;
+        scene.settings.materials = scene.settings.meshes = 1;
+    }
+};
+
+// A tree with more nodes than a tree over its items has, and the library has room for, is refused.
+static int oversized_trees(st_ctx *ctx) {
+    for (u32 n : {2u, 3u, 700u}) {
+        for (u32 extra : {0u, 2 * n - 3, 2 * n - 2, 2 * n, 40 * n}) {
+            SceneArrays a(n, extra);
+            const bool fits = 3 + extra <= 2 * n, pairs_fit = (2 + extra) / 2 <= n;
+            EXPECT(st_upload_scene(ctx, 0, &a.scene) == ST_OK);
+            EXPECT(st_upload_mesh_bvhs(ctx, 0, &a.scene) == (pairs_fit ? ST_OK : ST_ERR_BAD_SCENE));
+            EXPECT(st_upload_scene_bvh(ctx, 0, &a.scene) == (fits ? ST_OK : ST_ERR_BAD_SCENE));
+            EXPECT(fake.out_of_range == 0);
+            EXPECT(st_free_scene(ctx, 0) == ST_OK);
+        }
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     st_ctx *ctx = nullptr;
@@ -73,6 +121,7 @@ int main(int argc, char **argv) {
     EXPECT(st_init(&ctx, nullptr) == ST_OK);
     if (what == "refused_launch") r = refused_launch(ctx, argv[2], argv[3]);
     else if (what == "refused_allocation") r = refused_allocation(ctx);
+    else if (what == "oversized_trees") r = oversized_trees(ctx);
     else printf("no such scenario\n");
     st_shutdown(ctx);
     return r;

@@ -183,6 +183,13 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { Lock 
 cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind, cudaStream_t st) {
     Lock l(m);
     if (fake.fail_copy > 0 && --fake.fail_copy == 0) return fail(cudaErrorInvalidValue);
+    for (const void *p : {(const void *)dst, src})
+        for (auto *blocks : {&device_blocks, &pinned_blocks})
+            if (auto *b = block(*blocks, p))
+                if (static_cast<const char *>(p) + bytes > b->first + b->second) {
+                    fake.out_of_range++;
+                    return fail(cudaErrorInvalidValue);
+                }
     memcpy(dst, src, bytes);
     const long at = ++issued[st];
     clocks[st][st] = at;

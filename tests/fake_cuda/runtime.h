@@ -14,6 +14,7 @@ struct FakeRuntime {
     // read by a driver
     size_t device_held = 0;                  // what cudaMalloc and the pools hold of it
     int host_allocs = 0, streams = 0, launches = 0, trims = 0;
+    int out_of_range = 0;                    // copies past the end of a block (not made)
     int unordered_frees = 0;                 // cudaFreeAsync of memory that a copy elsewhere may still use
     std::string log;                         // the launched kernels' names, in order
     int in_flight();                         // copies that neither the host nor a later wait has seen the end of

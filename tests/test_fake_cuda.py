@@ -69,3 +69,8 @@ def test_copies_without_memory_or_threads(drivers):
 
 def test_a_refused_allocation_fails_no_later_call(drivers):
     run(drivers, "ingest", "refused_allocation")
+
+
+def test_trees_with_more_nodes_than_items_allow_are_refused(drivers):
+    """The arrays of a scene hold 2n nodes and n pairs of children for n primitives or triangles."""
+    run(drivers, "ingest", "oversized_trees")
