@@ -631,13 +631,15 @@ int st_upload_scene(st_ctx *ctx, int slot, const Scene *scene) {
 // against 15 for a 4096-primitive TLAS).  A near-first walk keeps at most one pending sibling per
 // level, so a tree whose deepest node is at depth d needs d stack entries; d + 2 <= kStack keeps
 // the reference's two entries of slack.
-static bool check_bvh(const BVHNode *nodes, u32t count, u32t items, u32t height) {
+// *reached (optional): which nodes were.
+static bool check_bvh(const BVHNode *nodes, u32t count, u32t items, u32t height, std::vector<uint8_t> *reached = nullptr) {
+    std::vector<uint8_t> own, &seen = reached ? *reached : own;
     if (!nodes || !count || height + 2 > (u32t)kStack) return false;
+    seen.assign(count, 0);
+    seen[0] = 1;
     if (nodes[0].child_count) return (uint64_t)nodes[0].first_child_id + nodes[0].child_count <= items;
-    std::vector<uint8_t> seen(count, 0);
     std::vector<std::pair<u32t, u32t>> stack;    // (node, its depth)
     stack.push_back({0u, 0u});
-    seen[0] = 1;
     while (!stack.empty()) {
         const u32t at = stack.back().first, depth = stack.back().second;
         stack.pop_back();
@@ -677,12 +679,27 @@ int st_upload_scene_bvh(st_ctx *ctx, int slot, const Scene *scene) {
     ST_TRY(ensure(ctx, *S, scene));
     const u32t n = scene->settings.primitives;
     // (nodes that no other leads to pass the check, and would run past the arrays made for n primitives)
-    if (!check_bvh(scene->bvh.nodes, scene->bvh.node_count, n, scene->bvh.height) || scene->bvh.node_count > 2 * (uint64_t)n)
+    std::vector<uint8_t> reached;
+    if (!check_bvh(scene->bvh.nodes, scene->bvh.node_count, n, scene->bvh.height, &reached) || scene->bvh.node_count > 2 * (uint64_t)n)
         return ST_ERR_BAD_SCENE;
     for (u32t i = 0; i < n; i++) if (scene->bvh.leaf_ids[i] >= n) return ST_ERR_BAD_SCENE;
     S->tlas_node_count = scene->bvh.node_count;
     S->tlas_height = scene->bvh.height;
-    cudaError_t e = cudaMemcpyAsync(S->tlas_nodes.ptr, scene->bvh.nodes, sizeof(BVHNode) * S->tlas_node_count,
+    // What was not reached was not checked, but a refit and the overlays go over the whole array: a node
+    // there claims no children, and a leaf that runs past the leaf ids is none.
+    const BVHNode *nodes = scene->bvh.nodes;
+    std::vector<BVHNode> made_safe;
+    if (std::count(reached.begin(), reached.end(), 0)) {
+        made_safe.assign(nodes, nodes + scene->bvh.node_count);
+        for (u32t k = 0; k < scene->bvh.node_count; k++) {
+            BVHNode &nd = made_safe[k];
+            if (reached[k] || (nd.child_count && (uint64_t)nd.first_child_id + nd.child_count <= n)) continue;
+            nd.child_count = 0;
+            nd.first_child_id = 0xFFFFFFFEu;
+        }
+        nodes = made_safe.data();
+    }
+    cudaError_t e = cudaMemcpyAsync(S->tlas_nodes.ptr, nodes, sizeof(BVHNode) * S->tlas_node_count,
                                     cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(S->tlas_leaf_ids.ptr, scene->bvh.leaf_ids, sizeof(u32t) * n, cudaMemcpyHostToDevice, ctx->stream);

@@ -734,6 +734,8 @@ __global__ void refit_kernel(BVHNode *nodes, u32t count, const u32t *leaf_ids, c
     for (int q = 0; q < 6; q++) __stcg(box + 6 * (size_t)i + q, b[q]);
     write_node(nodes[i], b, nd.first_child_id, nd.child_count, nd.depth);
     u32t p = parent[i];
+    // (a leaf of an uploaded array that no node leads to has no parent: the word is whatever was there)
+    if (i && (p >= count || nodes[p].child_count || nodes[p].first_child_id != 1 + 2 * ((i - 1) / 2))) return;
     while (p != 0xFFFFFFFFu) {
         __threadfence();
         if (atomicAdd(arrivals + p, 1u) == 0) return;
