@@ -116,6 +116,8 @@ ST_API void st_shutdown(st_ctx *ctx);
 ST_API const char *st_strerror(int status);
 ST_API const char *st_last_cuda_error(st_ctx *ctx);
 ST_API void *st_get_stream(st_ctx *ctx);                       /* the context's cudaStream_t */
+/* Device bytes the context holds: its scenes and workspaces, and what it keeps of the memory that
+ * builds, bakes and conversions took for their own time (at most 512 MB, within the budget). */
 ST_API uint64_t st_device_bytes_in_use(st_ctx *ctx);
 /* Size of a contract struct ("Primitive") or offset of a field ("Primitive.rotation") as this
  * library was compiled; -1 if the name is not in include/slimtracin_layout.h. */

@@ -207,7 +207,8 @@ struct st_ctx {
     LbvhScratch lbvh;
     // what a call allocates for its own time comes from a pool that keeps up to kTransientKept bytes of
     // it for the next call (mapping and unmapping it took 14 ms of a 327,680-triangle BLAS build, 1 ms
-    // of a 1024x1024 texture); given back when an allocation that stays needs the room, and at shutdown
+    // of a 1024x1024 texture), within the budget; given back when an allocation that stays needs the
+    // room, when serving starts, and at shutdown
     cudaMemPool_t pool = nullptr;
     Stage stage;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -243,8 +244,15 @@ void release(st_ctx *ctx, DevBuf &b) {
     }
     b = DevBuf();
 }
-// Device memory for one call, freed with cudaFreeAsync on the same stream.
-cudaError_t transient(st_ctx *ctx, void **p, size_t bytes, cudaStream_t st) {
+// Device bytes that the pool of transient memory holds, in use or kept.
+uint64_t pool_bytes(st_ctx *ctx) {
+    uint64_t held = 0;
+    if (ctx->pool && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) held = 0;
+    return held;
+}
+// Device memory for one call, freed with cudaFreeAsync on the same stream.  Refuses past the context's
+// budget; what the pool keeps beyond the room that is left goes back first.
+int transient(st_ctx *ctx, void **p, size_t bytes, cudaStream_t st) {
     if (!ctx->pool) {
         cudaMemPoolProps props;
         memset(&props, 0, sizeof(props));
@@ -252,12 +260,29 @@ cudaError_t transient(st_ctx *ctx, void **p, size_t bytes, cudaStream_t st) {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = ctx->device;
         cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
-        if (e != cudaSuccess) { ctx->pool = nullptr; return e; }
+        if (e != cudaSuccess) {
+            ctx->pool = nullptr;
+            return fail_cuda(ctx, e);
+        }
         uint64_t keep = kTransientKept;
         e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) return fail_cuda(ctx, e);
     }
-    return cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    uint64_t used = 0;
+    cudaError_t e = cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    if (e != cudaSuccess) return fail_cuda(ctx, e);
+    if (ctx->in_use + used + bytes > ctx->budget) return ST_ERR_BUDGET;
+    if (ctx->in_use + pool_bytes(ctx) + bytes > ctx->budget) cudaMemPoolTrimTo(ctx->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    return e == cudaSuccess ? ST_OK : fail_cuda(ctx, e);
+}
+// The end of a call that took it: waits for `st`, and leaves no more kept than the budget has room for
+// (the pool holds whole granules).
+cudaError_t end_transient(st_ctx *ctx, void *p, cudaStream_t st) {
+    cudaFreeAsync(p, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (ctx->in_use + pool_bytes(ctx) > ctx->budget) cudaMemPoolTrimTo(ctx->pool, 0);
+    return e;
 }
 // Grow `b` to at least `bytes` (contents are not kept).  Refuses past the context's budget.
 int reserve(st_ctx *ctx, DevBuf &b, size_t bytes) {
@@ -266,10 +291,8 @@ int reserve(st_ctx *ctx, DevBuf &b, size_t bytes) {
     size_t add = bytes - (b.ptr ? b.bytes : 0);
     if (ctx->in_use + add > ctx->budget) return ST_ERR_BUDGET;
     release(ctx, b);
-    uint64_t kept = 0;
-    if (ctx->pool && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &kept) == cudaSuccess &&
-        ctx->in_use + bytes + kept > ctx->budget)
-        cudaMemPoolTrimTo(ctx->pool, 0);
+    const uint64_t kept = pool_bytes(ctx);
+    if (kept && ctx->in_use + bytes + kept > ctx->budget) cudaMemPoolTrimTo(ctx->pool, 0);
     cudaError_t e = cudaMalloc(&b.ptr, bytes);
     if (e == cudaErrorMemoryAllocation && kept) {
         cudaGetLastError();
@@ -496,7 +519,7 @@ void st_shutdown(st_ctx *ctx) {
 
 const char *st_last_cuda_error(st_ctx *ctx) { return ctx ? ctx->cuda_error.c_str() : ""; }
 void *st_get_stream(st_ctx *ctx) { return ctx ? (void *)ctx->stream : nullptr; }
-uint64_t st_device_bytes_in_use(st_ctx *ctx) { return ctx ? ctx->in_use : 0; }
+uint64_t st_device_bytes_in_use(st_ctx *ctx) { return ctx ? ctx->in_use + pool_bytes(ctx) : 0; }
 
 int st_free_scene(st_ctx *ctx, int slot) {
     SceneSlot *S = slot_of(ctx, slot);
@@ -736,17 +759,16 @@ int st_upload_mesh_bvhs(st_ctx *ctx, int slot, const Scene *scene) {
         memcpy(d.aabb, &M.bvh.nodes[0].aabb, sizeof(d.aabb));
         memcpy(d.mesh_aabb, &M.aabb, sizeof(d.mesh_aabb));
         S->mesh_host.push_back(d);
-        ST_CUDA(cudaMemcpyAsync(P<Triangle>(S->tri_full) + tri_off, M.triangles, sizeof(Triangle) * M.triangle_count,
-                                cudaMemcpyHostToDevice, ctx->stream));
-        launch_make_trihot(P<Triangle>(S->tri_full) + tri_off, M.triangle_count, P<TriHot>(S->tri_hot) + tri_off, ctx->stream);
+        Triangle *tris = P<Triangle>(S->tri_full) + tri_off;
         if (M.bvh.node_count > 1) {
-            // stage the nodes through the TLAS AABB scratch-free path: a temporary device copy
-            BVHNode *tmp = nullptr;
-            ST_CUDA(transient(ctx, (void **)&tmp, sizeof(BVHNode) * M.bvh.node_count, ctx->stream));
-            ST_CUDA(cudaMemcpyAsync(tmp, M.bvh.nodes, sizeof(BVHNode) * M.bvh.node_count, cudaMemcpyHostToDevice, ctx->stream));
-            launch_make_pairs(tmp, M.bvh.node_count, P<NodePair>(S->mesh_pairs) + pair_off, ctx->stream);
-            ST_CUDA(cudaFreeAsync(tmp, ctx->stream));
+            // the nodes are only read for their pairs: they pass through the room of the mesh's triangles
+            static_assert(sizeof(BVHNode) * 4 <= sizeof(Triangle), "2n + 2 nodes in the room of n triangles");
+            BVHNode *nodes = reinterpret_cast<BVHNode *>(tris);
+            ST_CUDA(cudaMemcpyAsync(nodes, M.bvh.nodes, sizeof(BVHNode) * M.bvh.node_count, cudaMemcpyHostToDevice, ctx->stream));
+            launch_make_pairs(nodes, M.bvh.node_count, P<NodePair>(S->mesh_pairs) + pair_off, ctx->stream);
         }
+        ST_CUDA(cudaMemcpyAsync(tris, M.triangles, sizeof(Triangle) * M.triangle_count, cudaMemcpyHostToDevice, ctx->stream));
+        launch_make_trihot(tris, M.triangle_count, P<TriHot>(S->tri_hot) + tri_off, ctx->stream);
         // the nodes drawMeshAccelerationStructure (raytracer.h:33) outlines: depth <= 5, coloured
         // Magenta (leaf), Green (inner) or Blue (root)
         const u32t first_outline = (u32t)outlines.size();
@@ -988,10 +1010,9 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
     cudaStream_t st = ctx->stream;
     size_t bytes = sizeof(vec3) * (mesh->vertex_count + mesh->normals_count) + sizeof(vec2) * (mesh->uvs_count + 1) +
                    sizeof(uint32_t) * 9 * (size_t)n + sizeof(BVHNode) * 2 * (size_t)n + sizeof(u32t) * 2 * (size_t)n +
-                   sizeof(Triangle) * (size_t)n + 256 * 11;
-    if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
+                   sizeof(Triangle) * (size_t)n + (mode == ST_BVH_BINNED_SAH ? sah_scratch_bytes(n) : 0) + 256 * 11;
     char *base = nullptr;
-    ST_CUDA(transient(ctx, (void **)&base, bytes, st));
+    ST_TRY(transient(ctx, (void **)&base, bytes, st));
     char *cur = base;
     auto take = [&](size_t b) { char *p = cur; cur += (b + 255) & ~(size_t)255; return p; };
     vec3 *pos = (vec3 *)take(sizeof(vec3) * mesh->vertex_count);
@@ -1004,6 +1025,7 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
     u32t *order = (u32t *)take(sizeof(u32t) * n);
     u32t *inverse = (u32t *)take(sizeof(u32t) * n);
     Triangle *tris = (Triangle *)take(sizeof(Triangle) * n);
+    void *scratch = cur;
     const size_t uvs = mesh->uvs_count, index_bytes = sizeof(uint32_t) * 3 * (size_t)n;
     cudaError_t e = stage_copy(ctx->stage, {{mesh->vertex_positions, pos, sizeof(vec3) * mesh->vertex_count},
                                             {mesh->vertex_normals, nrm, sizeof(vec3) * mesh->normals_count},
@@ -1021,15 +1043,11 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
     u32t info[2];
-    void *scratch = nullptr;
     if (e == cudaSuccess && !*bad) {
         launch_tri_aabbs(pos, pidx, n, ctx->lbvh.aabbs, st);
-        if (mode == ST_BVH_LBVH30) {
-            e = lbvh_build(ctx->lbvh, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st);
-        } else {
-            e = transient(ctx, &scratch, sah_scratch_bytes(n), st);
-            if (e == cudaSuccess) e = sah_build(ctx->lbvh.aabbs, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st, scratch);
-        }
+        e = mode == ST_BVH_LBVH30
+            ? lbvh_build(ctx->lbvh, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st)
+            : sah_build(ctx->lbvh.aabbs, n, MAX_TRIANGLES_PER_MESH_BVH_NODE, nodes, order, info, st, scratch);
         if (e == cudaSuccess) {
             launch_tri_records(pos, nrm, uv, pidx, nidx, uidx, uvs ? 1 : 0, order, n, tris, inverse, st);
             e = cudaGetLastError();
@@ -1039,9 +1057,7 @@ int st_update_mesh_bvh(st_ctx *ctx, Mesh *mesh, int mode) {
                                         {mesh->bvh.nodes, nodes, sizeof(BVHNode) * (size_t)info[0]},
                                         {mesh->bvh.leaf_ids, inverse, sizeof(u32t) * (size_t)n}}, true, st);
     }
-    if (scratch) cudaFreeAsync(scratch, st);
-    cudaFreeAsync(base, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
+    const cudaError_t e2 = end_transient(ctx, base, st);
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return fail_cuda(ctx, e);
     if (*bad) return ST_ERR_BAD_SCENE;
@@ -1059,18 +1075,16 @@ int st_build_bvh(st_ctx *ctx, int mode, const float *aabbs, uint32_t n, uint32_t
     ST_TRY(builder_room(ctx, n));
     cudaStream_t st = ctx->stream;
     char *base = nullptr;
-    const size_t bytes = sizeof(BVHNode) * 2 * (size_t)n + sizeof(u32t) * 2 * (size_t)n + 512;
-    if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
-    ST_CUDA(transient(ctx, (void **)&base, bytes, st));
+    const size_t node_bytes = (sizeof(BVHNode) * 2 * (size_t)n + 255) & ~(size_t)255;
+    const size_t id_bytes = (sizeof(u32t) * 2 * (size_t)n + 255) & ~(size_t)255;
+    ST_TRY(transient(ctx, (void **)&base, node_bytes + id_bytes + (mode == ST_BVH_BINNED_SAH ? sah_scratch_bytes(n) : 0), st));
     BVHNode *d_nodes = (BVHNode *)base;
-    u32t *d_order = (u32t *)(base + ((sizeof(BVHNode) * 2 * (size_t)n + 255) & ~(size_t)255));
+    u32t *d_order = (u32t *)(base + node_bytes);
     u32t *d_codes = d_order + n;
+    void *scratch = base + node_bytes + id_bytes;
     cudaMemcpyAsync(ctx->lbvh.aabbs, aabbs, sizeof(float) * 6 * (size_t)n, cudaMemcpyHostToDevice, st);
     u32t inf[2];
-    void *scratch = nullptr;
-    cudaError_t e = mode == ST_BVH_BINNED_SAH ? transient(ctx, &scratch, sah_scratch_bytes(n), st) : cudaSuccess;
-    if (e == cudaSuccess)
-        e = mode == ST_BVH_LBVH30     ? lbvh_build(ctx->lbvh, n, max_leaf, d_nodes, d_order, inf, st)
+    cudaError_t e = mode == ST_BVH_LBVH30     ? lbvh_build(ctx->lbvh, n, max_leaf, d_nodes, d_order, inf, st)
                     : mode == ST_BVH_REF_SAH ? refsah_build(ctx->lbvh.aabbs, n, max_leaf, d_nodes, d_order, inf, st)
                                              : sah_build(ctx->lbvh.aabbs, n, max_leaf, d_nodes, d_order, inf, st, scratch);
     if (e == cudaSuccess) {
@@ -1081,9 +1095,7 @@ int st_build_bvh(st_ctx *ctx, int mode, const float *aabbs, uint32_t n, uint32_t
         if (codes) cudaMemcpyAsync(codes, d_codes, sizeof(u32t) * n, cudaMemcpyDeviceToHost, st);
         e = cudaStreamSynchronize(st);
     }
-    if (scratch) cudaFreeAsync(scratch, st);
-    cudaFreeAsync(base, st);
-    cudaStreamSynchronize(st);
+    end_transient(ctx, base, st);
     if (e != cudaSuccess) return fail_cuda(ctx, e);
     info[0] = inf[0];
     info[1] = inf[1];
@@ -1791,9 +1803,8 @@ int st_bake_texture(st_ctx *ctx, const uint8_t *components, uint16_t width, uint
     const size_t image = (size_t)width * height * (bit_count / 8);
     const size_t table = (sizeof(TextureMip) * mips + 15) & ~(size_t)15;
     const size_t bytes = ((image + 255) & ~(size_t)255) + texture_scratch_bytes(width, height) + sizeof(TexelQuad) * quads + 512;
-    if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
     char *base = nullptr;
-    ST_CUDA(transient(ctx, (void **)&base, bytes, st));
+    ST_TRY(transient(ctx, (void **)&base, bytes, st));
     uint8_t *dev_image = reinterpret_cast<uint8_t *>(base);
     char *scratch = base + ((image + 255) & ~(size_t)255);
     TexelQuad *dev_quads = reinterpret_cast<TexelQuad *>(scratch + ((texture_scratch_bytes(width, height) + 255) & ~(size_t)255));
@@ -1801,8 +1812,7 @@ int st_bake_texture(st_ctx *ctx, const uint8_t *components, uint16_t width, uint
     if (e == cudaSuccess) e = bake_texture(dev_image, width, height, bit_count, wrap != 0, mipmap != 0, scratch, dev_quads, st);
     char *host = static_cast<char *>(memory);
     if (e == cudaSuccess) e = stage_copy(ctx->stage, {{host + table, dev_quads, sizeof(TexelQuad) * quads}}, true, st);
-    cudaFreeAsync(base, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
+    const cudaError_t e2 = end_transient(ctx, base, st);
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return fail_cuda(ctx, e);
     TextureMip *mip = reinterpret_cast<TextureMip *>(host);
@@ -1923,9 +1933,8 @@ int st_obj_to_mesh(st_ctx *ctx, const char *obj_path, int invert_winding_order, 
     const size_t edges_bytes = sizeof(EdgeVertexIndices) * 3 * (size_t)m.triangle_count;
     const size_t bytes = ((ids_bytes + 255) & ~(size_t)255) + ((edges_bytes + 255) & ~(size_t)255) +
                          unique_edges_scratch_bytes(m.triangle_count);
-    if (ctx->in_use + bytes > ctx->budget) return ST_ERR_BUDGET;
     char *dev = nullptr;
-    ST_CUDA(transient(ctx, (void **)&dev, bytes, st));
+    ST_TRY(transient(ctx, (void **)&dev, bytes, st));
     uint32_t *dev_ids = reinterpret_cast<uint32_t *>(dev);
     EdgeVertexIndices *dev_edges = reinterpret_cast<EdgeVertexIndices *>(dev + ((ids_bytes + 255) & ~(size_t)255));
     void *scratch = dev + ((ids_bytes + 255) & ~(size_t)255) + ((edges_bytes + 255) & ~(size_t)255);
@@ -1934,8 +1943,7 @@ int st_obj_to_mesh(st_ctx *ctx, const char *obj_path, int invert_winding_order, 
     if (e == cudaSuccess) e = unique_edges(dev_ids, m.triangle_count, m.vertex_count, scratch, dev_edges, &n_edges, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m.edge_vertex_indices, dev_edges, sizeof(EdgeVertexIndices) * n_edges, cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(dev, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
+    const cudaError_t e2 = end_transient(ctx, dev, st);
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return fail_cuda(ctx, e);
     m.edge_count = n_edges;
@@ -2253,6 +2261,7 @@ int st_serve_start(st_ctx *ctx, const st_serve_config *cfg) {
     if (V.cfg.refit_fraction <= 0) V.cfg.refit_fraction = 0.25;
     if (!cfg) { V.cfg.tile_shape = -1; V.cfg.chunk = 0; }
     if (V.cfg.launch_mode != ST_LAUNCH_PER_VIEW && V.cfg.launch_mode != ST_LAUNCH_PERSISTENT) return ST_ERR_INVALID_ARG;
+    if (ctx->pool) cudaMemPoolTrimTo(ctx->pool, 0);     // (nothing takes transient memory while serving)
     V.frame_budget = V.cfg.frame_budget ? V.cfg.frame_budget
                                         : (ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : 0);
     // The blocks of a kernel wait for those of the kernels before it on the device: with the flights'

@@ -114,10 +114,53 @@ static int oversized_trees(st_ctx *ctx) {
     return 0;
 }
 
+// What a build takes for its own time is within the budget, the binned builder's scratch too, and so is
+// what is kept of it; it is reported, and given back for memory that stays and for serving.
+static int budget() {
+    const size_t MB = (size_t)1 << 20;
+    st_ctx *ctx = nullptr;
+    st_config cfg = {};
+    cfg.memory_budget = 30 * MB;
+    EXPECT(st_init(&ctx, &cfg) == ST_OK);
+    const uint64_t empty = st_device_bytes_in_use(ctx);
+    MeshArrays a(100000);                              // 23 MB, and 18 of scratch
+    EXPECT(st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_BINNED_SAH) == ST_ERR_BUDGET);
+    EXPECT(a.mesh.bvh.node_count == 77);
+    std::vector<float> boxes(6 * 200000);
+    std::vector<u32> order(200000);
+    std::vector<BVHNode> nodes(400000);
+    u32 info[2];
+    EXPECT(st_build_bvh(ctx, ST_BVH_BINNED_SAH, boxes.data(), 200000, 2, nullptr, order.data(), nodes.data(), info) == ST_ERR_BUDGET);
+    EXPECT(st_build_bvh(ctx, ST_BVH_LBVH30, boxes.data(), 200000, 2, nullptr, order.data(), nodes.data(), info) == ST_OK);
+    EXPECT(st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_LBVH30) == ST_OK);
+    EXPECT(st_device_bytes_in_use(ctx) > empty + 20 * MB && st_device_bytes_in_use(ctx) <= 30 * MB);
+    // a scene takes the room that was kept, and leaves the builds what it does not need
+    SceneArrays s(20000, 0);                           // 12 MB with its mesh of as many triangles
+    EXPECT(st_upload_scene(ctx, 0, &s.scene) == ST_OK);
+    EXPECT(st_upload_mesh_bvhs(ctx, 0, &s.scene) == ST_OK);
+    EXPECT(st_upload_scene_bvh(ctx, 0, &s.scene) == ST_OK);
+    EXPECT(st_device_bytes_in_use(ctx) <= 30 * MB);
+    EXPECT(st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_LBVH30) == ST_ERR_BUDGET);
+    EXPECT(st_update_mesh_bvh(ctx, &s.mesh.mesh, ST_BVH_LBVH30) == ST_OK);
+    EXPECT(st_device_bytes_in_use(ctx) <= 30 * MB);
+    EXPECT(st_free_scene(ctx, 0) == ST_OK);
+    EXPECT(st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_LBVH30) == ST_OK);
+    // serving has what no scene holds for its frames
+    st_serve_config serve = {};
+    serve.frame_budget = 2 * MB;
+    EXPECT(st_serve_start(ctx, &serve) == ST_OK);
+    EXPECT(st_device_bytes_in_use(ctx) < 3 * MB);
+    EXPECT(st_serve_stop(ctx) == ST_OK);
+    st_shutdown(ctx);
+    EXPECT(fake.device_held == 0);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     st_ctx *ctx = nullptr;
     int r = 2;
+    if (what == "budget") return budget();
     EXPECT(st_init(&ctx, nullptr) == ST_OK);
     if (what == "refused_launch") r = refused_launch(ctx, argv[2], argv[3]);
     else if (what == "refused_allocation") r = refused_allocation(ctx);

@@ -74,3 +74,7 @@ def test_a_refused_allocation_fails_no_later_call(drivers):
 def test_trees_with_more_nodes_than_items_allow_are_refused(drivers):
     """The arrays of a scene hold 2n nodes and n pairs of children for n primitives or triangles."""
     run(drivers, "ingest", "oversized_trees")
+
+
+def test_transient_memory_is_within_the_budget(drivers):
+    run(drivers, "ingest", "budget")
