@@ -250,6 +250,12 @@ uint64_t pool_bytes(st_ctx *ctx) {
     if (ctx->pool && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) held = 0;
     return held;
 }
+// Whether an allocation that failed with `e` is worth another try: memory the pool only kept was given back.
+bool gave_back(st_ctx *ctx, cudaError_t e) {
+    if (e != cudaErrorMemoryAllocation || !pool_bytes(ctx)) return false;
+    cudaGetLastError();
+    return cudaMemPoolTrimTo(ctx->pool, 0) == cudaSuccess;
+}
 // Device memory for one call, freed with cudaFreeAsync on the same stream.  Refuses past the context's
 // budget; what the pool keeps beyond the room that is left goes back first.
 int transient(st_ctx *ctx, void **p, size_t bytes, cudaStream_t st) {
@@ -274,6 +280,7 @@ int transient(st_ctx *ctx, void **p, size_t bytes, cudaStream_t st) {
     if (ctx->in_use + used + bytes > ctx->budget) return ST_ERR_BUDGET;
     if (ctx->in_use + pool_bytes(ctx) + bytes > ctx->budget) cudaMemPoolTrimTo(ctx->pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    if (gave_back(ctx, e)) e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
     return e == cudaSuccess ? ST_OK : fail_cuda(ctx, e);
 }
 // The end of a call that took it: waits for `st`, and leaves no more kept than the budget has room for
@@ -294,11 +301,7 @@ int reserve(st_ctx *ctx, DevBuf &b, size_t bytes) {
     const uint64_t kept = pool_bytes(ctx);
     if (kept && ctx->in_use + bytes + kept > ctx->budget) cudaMemPoolTrimTo(ctx->pool, 0);
     cudaError_t e = cudaMalloc(&b.ptr, bytes);
-    if (e == cudaErrorMemoryAllocation && kept) {
-        cudaGetLastError();
-        cudaMemPoolTrimTo(ctx->pool, 0);
-        e = cudaMalloc(&b.ptr, bytes);
-    }
+    if (gave_back(ctx, e)) e = cudaMalloc(&b.ptr, bytes);
     if (e != cudaSuccess) return fail_cuda(ctx, e);
     b.bytes = bytes;
     ctx->in_use += bytes;
@@ -306,8 +309,15 @@ int reserve(st_ctx *ctx, DevBuf &b, size_t bytes) {
 }
 // The builders' scratch for n items.
 int builder_room(st_ctx *ctx, u32t n) {
-    const cudaError_t e = lbvh_reserve(ctx->lbvh, n);
+    cudaError_t e = lbvh_reserve(ctx->lbvh, n);
+    if (gave_back(ctx, e)) e = lbvh_reserve(ctx->lbvh, n);
     return e == cudaSuccess ? ST_OK : fail_cuda(ctx, e);
+}
+// The reference's builder, which takes its scratch itself.
+cudaError_t refsah(st_ctx *ctx, u32t n, u32t max_leaf, BVHNode *nodes, u32t *leaf_ids, u32t info[2]) {
+    cudaError_t e = refsah_build(ctx->lbvh.aabbs, n, max_leaf, nodes, leaf_ids, info, ctx->stream);
+    if (gave_back(ctx, e)) e = refsah_build(ctx->lbvh.aabbs, n, max_leaf, nodes, leaf_ids, info, ctx->stream);
+    return e;
 }
 #define ST_TRY(x)                    \
     do {                             \
@@ -968,8 +978,7 @@ static int build_scene_bvh(st_ctx *ctx, SceneSlot *S, Scene *scene, int mode, cu
         ST_TRY(builder_room(ctx, n));
         launch_prim_aabbs(P<Primitive>(S->prims_raw), P<MeshDev>(S->meshes), n, ctx->lbvh.aabbs, ctx->stream);
         u32t info[2];
-        cudaError_t e = refsah_build(ctx->lbvh.aabbs, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes),
-                                     P<u32t>(S->tlas_leaf_ids), info, ctx->stream);
+        cudaError_t e = refsah(ctx, n, MAX_OBJS_PER_SCENE_BVH_NODE, P<BVHNode>(S->tlas_nodes), P<u32t>(S->tlas_leaf_ids), info);
         if (e != cudaSuccess) return fail_cuda(ctx, e);
         S->tlas_node_count = info[0];
         S->tlas_height = info[1];
@@ -1085,7 +1094,7 @@ int st_build_bvh(st_ctx *ctx, int mode, const float *aabbs, uint32_t n, uint32_t
     cudaMemcpyAsync(ctx->lbvh.aabbs, aabbs, sizeof(float) * 6 * (size_t)n, cudaMemcpyHostToDevice, st);
     u32t inf[2];
     cudaError_t e = mode == ST_BVH_LBVH30     ? lbvh_build(ctx->lbvh, n, max_leaf, d_nodes, d_order, inf, st)
-                    : mode == ST_BVH_REF_SAH ? refsah_build(ctx->lbvh.aabbs, n, max_leaf, d_nodes, d_order, inf, st)
+                    : mode == ST_BVH_REF_SAH ? refsah(ctx, n, max_leaf, d_nodes, d_order, inf)
                                              : sah_build(ctx->lbvh.aabbs, n, max_leaf, d_nodes, d_order, inf, st, scratch);
     if (e == cudaSuccess) {
         if (mode == ST_BVH_LBVH30) launch_codes_by_item(ctx->lbvh, n, d_codes, st);

@@ -156,6 +156,31 @@ static int budget() {
     return 0;
 }
 
+// Memory that is only kept is no reason to refuse a call: not the builders' scratch, nor a scene's arrays,
+// nor a transient block.
+static int kept_memory(st_ctx *ctx) {
+    MeshArrays a(100000), b(150000);
+    EXPECT(st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_BINNED_SAH) == ST_OK);     // 41 MB kept
+    const size_t all = fake.device_bytes, MB = (size_t)1 << 20;
+    fake.device_bytes = fake.device_held + 4 * MB;
+    std::vector<float> boxes(6 * 150000);
+    std::vector<u32> order(150000);
+    std::vector<BVHNode> nodes(300000);
+    u32 info[2];
+    EXPECT(st_build_bvh(ctx, ST_BVH_LBVH30, boxes.data(), 150000, 2, nullptr, order.data(), nodes.data(), info) == ST_OK);
+    fake.device_bytes = fake.device_held + 25 * MB;
+    EXPECT(st_update_mesh_bvh(ctx, &a.mesh, ST_BVH_LBVH30) == ST_OK);
+    fake.device_bytes = fake.device_held + 4 * MB;
+    SceneArrays s(20000, 0);                                                  // 12 MB
+    EXPECT(st_upload_scene(ctx, 0, &s.scene) == ST_OK);
+    // and what does not fit without it is refused as before
+    fake.device_bytes = fake.device_held + MB;
+    EXPECT(st_update_mesh_bvh(ctx, &b.mesh, ST_BVH_LBVH30) == ST_ERR_OUT_OF_MEMORY);
+    fake.device_bytes = all;
+    EXPECT(st_update_mesh_bvh(ctx, &b.mesh, ST_BVH_LBVH30) == ST_OK);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     st_ctx *ctx = nullptr;
@@ -165,6 +190,7 @@ int main(int argc, char **argv) {
     if (what == "refused_launch") r = refused_launch(ctx, argv[2], argv[3]);
     else if (what == "refused_allocation") r = refused_allocation(ctx);
     else if (what == "oversized_trees") r = oversized_trees(ctx);
+    else if (what == "kept_memory") r = kept_memory(ctx);
     else printf("no such scenario\n");
     st_shutdown(ctx);
     return r;

@@ -78,3 +78,7 @@ def test_trees_with_more_nodes_than_items_allow_are_refused(drivers):
 
 def test_transient_memory_is_within_the_budget(drivers):
     run(drivers, "ingest", "budget")
+
+
+def test_kept_memory_goes_back_before_a_call_is_refused(drivers):
+    run(drivers, "ingest", "kept_memory")
