@@ -17,6 +17,7 @@
 //              reference's BVHNode layout (root 0, sibling pairs, builder_top_down.h:172-174)
 #include <cstdio>
 #include "st_kernels.h"
+#include "st_treecheck.h"
 
 namespace st {
 
@@ -847,32 +848,20 @@ __global__ void tlas_finish_kernel(const BVHNode *nodes, const u32t *info, u32t 
     if (2 + 2 * i < count) make_pair(nodes, i, pairs);
     if (i < count) {
         const BVHNode nd = nodes[i];
-        if (parent_of_pair && !nd.child_count && nd.first_child_id && (nd.first_child_id - 1) / 2 < n)
-            parent_of_pair[(nd.first_child_id - 1) / 2] = i;
+        const u32t pair = parent_of_pair ? claimed_pair(nd, n) : kClaimsNone;
+        if (pair != kClaimsNone) parent_of_pair[pair] = i;
         if (out.nodes) out.nodes[i] = nd;
     }
     if (i < n && out.ids) out.ids[i] = ids[i];
 }
-// What st_validate_bvh asks of a tree, of a newly built one before the walk first uses it: every
-// children pair lies inside the array and has one parent, every leaf range and leaf id is in range, and
-// every node reaches the root by at most kStack - 2 parents.  A node that fails sets out.counts[3].
+// What st_validate_bvh asks of a tree, of a newly built one before the walk first uses it, and that every
+// node is reached: tree_node_ok of each, and every leaf id in range.  A node that fails sets out.counts[3].
 __global__ void tlas_check_kernel(const BVHNode *nodes, const u32t *info, const u32t *ids, u32t n, const u32t *parent_of_pair,
                                   TlasStaging out) {
     const u32t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool ok = info[2] < n;
     const u32t count = 1 + 2 * min(info[2], n - 1);
-    if (i < count) {
-        const BVHNode nd = nodes[i];
-        const u32t f = nd.first_child_id;
-        if (nd.child_count) ok = ok && (unsigned long long)f + nd.child_count <= n;
-        else ok = ok && (f & 1u) && f + 1 < count && f + 1 > f && parent_of_pair[(f - 1) / 2] == i;
-        u32t steps = 0;
-        for (u32t at = i; at && ok; steps++) {
-            const u32t pair = (at - 1) / 2, p = parent_of_pair[pair];
-            ok = steps + 2 < (u32t)kStack && p < count && !nodes[p].child_count && nodes[p].first_child_id == 1 + 2 * pair;
-            at = p;
-        }
-    }
+    if (i < count) ok = ok && tree_node_ok(nodes, count, n, parent_of_pair, (u32t)kStack, i);
     if (i < n) ok = ok && ids[i] < n;
     if (!ok) out.counts[3] = 1;
 }

@@ -69,3 +69,35 @@ def test_tlas_update_and_refit(renderer, n, mode):
     g = H.gpu_frame(renderer, 5, sd, cam, 64, 40, depth=1, mode=S.RM_NORMALS)
     o = H.oracle_frame(sd, cam, 64, 40, depth=1, mode=S.RM_NORMALS)
     assert g.float_pixels.tobytes() == o.float_pixels.tobytes()
+
+
+@pytest.mark.parametrize("n", [130, 300, 4096, 5000])
+def test_too_deep_a_tree_is_refused(n):
+    """Thin boxes at a small spacing whose unions all have the same area (2^40, the spacing rounds away): of
+    equal costs the first split wins, so a level loses its first bin only and the binned tree is deeper than
+    the 62 levels that a walk's stack holds.  The update refuses it, and leaves no TLAS until a build
+    succeeds."""
+    not_resident = 8
+    sd, cam = scenes.moving_scene(count=n)
+    sd.primitives["type"] = S.PT_BOX
+    sd.primitives["rotation"] = (0, 0, 0, 1)
+    sd.primitives["position"] = 0
+    sd.primitives["position"][:, 0] = np.linspace(0, 0.01, n)
+    sd.primitives["scale"] = (1e-9, 2.0 ** 19, 2.0 ** 19)
+    want = sd.copy()
+    H.tlas_binned(want)
+    assert want.tlas_height > 62
+    with api.Renderer(device=0) as r:
+        r.upload(0, sd, tlas=None)
+        r.build_tlas(0, sd, api.ST_BVH_LBVH30)
+        first = H.gpu_frame(r, 0, sd, cam, 64, 40, depth=1)
+        sc, keep = sd.to_ctypes()
+        nodes, ids = sd.tlas_nodes.tobytes(), sd.tlas_leaf_ids.tobytes()
+        assert r.L.st_update_scene_bvh(r.ctx, 0, C.byref(sc), api.ST_BVH_BINNED_SAH) == api.ST_ERR_BAD_SCENE
+        assert sd.tlas_nodes.tobytes() == nodes and sd.tlas_leaf_ids.tobytes() == ids
+        assert r.L.st_update_scene_bvh(r.ctx, 0, None, api.ST_BVH_REFIT) == not_resident
+        with pytest.raises(api.STError) as e:
+            H.gpu_frame(r, 0, sd, cam, 64, 40, depth=1)
+        assert e.value.status == not_resident
+        r.build_tlas(0, sd, api.ST_BVH_LBVH30)
+        assert H.gpu_frame(r, 0, sd, cam, 64, 40, depth=1).float_pixels.tobytes() == first.float_pixels.tobytes()
