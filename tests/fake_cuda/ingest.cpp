@@ -181,6 +181,27 @@ static int kept_memory(st_ctx *ctx) {
     return 0;
 }
 
+// What a TLAS update page-locks is what it writes there: not the tree's arrays where the host wants none,
+// or gets them by copies.
+static int update_staging(st_ctx *ctx) {
+    for (u32 n : {700u, 40000u}) {
+        SceneArrays a(n, 0);
+        EXPECT(st_upload_scene(ctx, 0, &a.scene) == ST_OK);
+        EXPECT(st_upload_scene_bvh(ctx, 0, &a.scene) == ST_OK);
+        size_t before = fake.host_bytes;
+        EXPECT(st_update_scene_bvh(ctx, 0, nullptr, ST_BVH_REFIT) == ST_OK);
+        EXPECT(st_update_scene_bvh(ctx, 0, nullptr, ST_BVH_LBVH30) == ST_OK);
+        EXPECT(fake.host_bytes - before <= 4096);
+        EXPECT(st_upload_scene_bvh(ctx, 0, &a.scene) == ST_OK);
+        before = fake.host_bytes;
+        EXPECT(st_update_scene_bvh(ctx, 0, &a.scene, ST_BVH_REFIT) == ST_OK);
+        EXPECT(n <= 16384 || fake.host_bytes - before <= 4096);
+        EXPECT(a.scene.bvh.node_count == 3);
+        EXPECT(st_free_scene(ctx, 0) == ST_OK);
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     st_ctx *ctx = nullptr;
@@ -191,6 +212,7 @@ int main(int argc, char **argv) {
     else if (what == "refused_allocation") r = refused_allocation(ctx);
     else if (what == "oversized_trees") r = oversized_trees(ctx);
     else if (what == "kept_memory") r = kept_memory(ctx);
+    else if (what == "update_staging") r = update_staging(ctx);
     else printf("no such scenario\n");
     st_shutdown(ctx);
     return r;

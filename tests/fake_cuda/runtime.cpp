@@ -77,6 +77,7 @@ cudaError_t host_alloc(void **p, size_t bytes) {
     *p = calloc(1, bytes);
     pinned_blocks[static_cast<char *>(*p)] = bytes;
     fake.host_allocs++;
+    fake.host_bytes += bytes;
     return cudaSuccess;
 }
 }  // namespace

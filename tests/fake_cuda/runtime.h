@@ -13,6 +13,7 @@ struct FakeRuntime {
     bool no_threads = false;                 // no further thread can be made
     // read by a driver
     size_t device_held = 0;                  // what cudaMalloc and the pools hold of it
+    size_t host_bytes = 0;                   // page-locked, all told
     int host_allocs = 0, streams = 0, launches = 0, trims = 0;
     int out_of_range = 0;                    // copies past the end of a block (not made)
     int unordered_frees = 0;                 // cudaFreeAsync of memory that a copy elsewhere may still use

@@ -82,3 +82,7 @@ def test_transient_memory_is_within_the_budget(drivers):
 
 def test_kept_memory_goes_back_before_a_call_is_refused(drivers):
     run(drivers, "ingest", "kept_memory")
+
+
+def test_tlas_updates_page_lock_what_they_use(drivers):
+    run(drivers, "ingest", "update_staging")
