@@ -2266,12 +2266,33 @@ void serve_loop(st_ctx *ctx) {
 
 }  // namespace
 
-extern "C" {
+namespace {
 
-int st_serve_start(st_ctx *ctx, const st_serve_config *cfg) {
-    if (!ctx) return ST_ERR_INVALID_ARG;
+// What serving holds beside the scenes: the flights, the updates' stream, the arenas' pool.
+void release_serving(st_ctx *ctx) {
     Server &V = ctx->server;
-    if (V.running) return ST_ERR_INVALID_ARG;
+    for (InFlight &F : V.flights) {
+        if (F.pinned) cudaFreeHost(F.pinned);
+        if (F.B.staging) cudaFreeHost(F.B.staging);
+        release_aux(F.B);
+        for (DevBuf *b : {&F.B.table, &F.B.counter, &F.status}) release(ctx, *b);
+        if (F.done_ev) cudaEventDestroy(F.done_ev);
+        if (F.stream) cudaStreamDestroy(F.stream);
+    }
+    V.flights.clear();
+    for (RetiredVersion &rv : V.retired) slot_of(ctx, rv.slot)->spare.push_back(rv.bufs);
+    V.retired.clear();
+    if (V.updates) cudaStreamDestroy(V.updates);
+    V.updates = nullptr;
+    if (V.pool) {
+        cudaDeviceSynchronize();
+        cudaMemPoolDestroy(V.pool);
+        V.pool = nullptr;
+    }
+}
+
+int serve_start(st_ctx *ctx, const st_serve_config *cfg) {
+    Server &V = ctx->server;
     cudaSetDevice(ctx->device);
     V.cfg = cfg ? *cfg : st_serve_config{};
     if (V.cfg.max_in_flight <= 0) V.cfg.max_in_flight = 3;
@@ -2325,19 +2346,36 @@ int st_serve_start(st_ctx *ctx, const st_serve_config *cfg) {
         if (!S.allocated || !S.tlas_valid) continue;
         while ((int)S.spare.size() < V.cfg.max_in_flight) {
             MotionBufs m;
-            for (int k = 0; k < 6; k++) {
+            int status = ST_OK;
+            for (int k = 0; k < 6 && status == ST_OK; k++) {
                 DevBuf *mine;
                 DevBuf *copy = motion_field(S, m, k, &mine);
-                if (mine->ptr) ST_TRY(reserve(ctx, *copy, mine->bytes));
+                if (mine->ptr) status = reserve(ctx, *copy, mine->bytes);
             }
-            S.spare.push_back(m);
+            S.spare.push_back(m);        // (what there is of it is the scene's either way)
+            ST_TRY(status);
         }
     }
     V.stop = false;
-    V.running = true;
     V.inflight_bytes = 0;
-    V.worker = std::thread(serve_loop, ctx);
+    try {
+        V.worker = std::thread(serve_loop, ctx);
+    } catch (...) {
+        return ST_ERR_OUT_OF_MEMORY;
+    }
+    V.running = true;
     return ST_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int st_serve_start(st_ctx *ctx, const st_serve_config *cfg) {
+    if (!ctx || ctx->server.running) return ST_ERR_INVALID_ARG;
+    const int s = serve_start(ctx, cfg);
+    if (s != ST_OK) release_serving(ctx);
+    return s;
 }
 
 int st_submit(st_ctx *ctx, const st_request *req, st_ticket *ticket) {
@@ -2421,24 +2459,7 @@ int st_serve_stop(st_ctx *ctx) {
         V.cv_work.notify_all();
     }
     V.worker.join();
-    for (InFlight &F : V.flights) {
-        if (F.pinned) cudaFreeHost(F.pinned);
-        if (F.B.staging) cudaFreeHost(F.B.staging);
-        release_aux(F.B);
-        for (DevBuf *b : {&F.B.table, &F.B.counter, &F.status}) release(ctx, *b);
-        if (F.done_ev) cudaEventDestroy(F.done_ev);
-        if (F.stream) cudaStreamDestroy(F.stream);
-    }
-    V.flights.clear();
-    for (RetiredVersion &rv : V.retired) slot_of(ctx, rv.slot)->spare.push_back(rv.bufs);
-    V.retired.clear();
-    if (V.updates) cudaStreamDestroy(V.updates);
-    V.updates = nullptr;
-    if (V.pool) {
-        cudaDeviceSynchronize();
-        cudaMemPoolDestroy(V.pool);
-        V.pool = nullptr;
-    }
+    release_serving(ctx);
     V.running = false;
     return ST_OK;
 }

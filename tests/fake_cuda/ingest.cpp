@@ -202,6 +202,33 @@ static int update_staging(st_ctx *ctx) {
     return 0;
 }
 
+// Serving that cannot start leaves nothing but its scene's spare arrays, which go with the scene, and starts
+// once there is room.
+static int refused_serving(st_ctx *ctx) {
+    const size_t all = fake.device_bytes, empty = fake.device_held, MB = (size_t)1 << 20;
+    const int streams = fake.streams;
+    for (size_t room : {0 * MB, 1 * MB, 3 * MB, 9 * MB, 19 * MB, 50 * MB}) {     // (three spares take 14 MB)
+        SceneArrays a(20000, 0);
+        EXPECT(st_upload_scene(ctx, 0, &a.scene) == ST_OK);
+        EXPECT(st_upload_scene_bvh(ctx, 0, &a.scene) == ST_OK);
+        st_serve_config cfg = {};
+        cfg.frame_budget = MB;
+        fake.device_bytes = fake.device_held + room;
+        fake.no_threads = room == 19 * MB;
+        EXPECT(st_serve_start(ctx, &cfg) == (room == 50 * MB ? ST_OK : ST_ERR_OUT_OF_MEMORY));
+        fake.device_bytes = all;
+        fake.no_threads = false;
+        if (room == 50 * MB) {
+            EXPECT(st_serve_start(ctx, &cfg) == ST_ERR_INVALID_ARG);
+            EXPECT(st_serve_stop(ctx) == ST_OK);
+        }
+        EXPECT(fake.streams == streams);
+        EXPECT(st_free_scene(ctx, 0) == ST_OK);
+        EXPECT(fake.device_held == empty);
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     st_ctx *ctx = nullptr;
@@ -213,6 +240,7 @@ int main(int argc, char **argv) {
     else if (what == "oversized_trees") r = oversized_trees(ctx);
     else if (what == "kept_memory") r = kept_memory(ctx);
     else if (what == "update_staging") r = update_staging(ctx);
+    else if (what == "refused_serving") r = refused_serving(ctx);
     else printf("no such scenario\n");
     st_shutdown(ctx);
     return r;

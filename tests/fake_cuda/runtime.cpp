@@ -170,7 +170,7 @@ cudaError_t cudaFreeAsync(void *p, cudaStream_t st) {
 static void *handle() { return calloc(1, 8); }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { Lock l(m); *s = static_cast<cudaStream_t>(handle()); fake.streams++; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned f, int) { return cudaStreamCreateWithFlags(s, f); }
-cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { Lock l(m); fake.streams--; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { Lock l(m); host_waits(s); return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { Lock l(m); copies.clear(); return cudaSuccess; }
 cudaError_t cudaDeviceGetStreamPriorityRange(int *least, int *greatest) { *least = 0; *greatest = -5; return cudaSuccess; }

@@ -86,3 +86,7 @@ def test_kept_memory_goes_back_before_a_call_is_refused(drivers):
 
 def test_tlas_updates_page_lock_what_they_use(drivers):
     run(drivers, "ingest", "update_staging")
+
+
+def test_serving_that_cannot_start_holds_nothing(drivers):
+    run(drivers, "ingest", "refused_serving")
