@@ -134,9 +134,11 @@ ST_API int st_upload_primitives(st_ctx *ctx, int slot, const Scene *scene);
 ST_API int st_upload_materials(st_ctx *ctx, int slot, const Scene *scene);
 /* uploadLights (core/init.h:80). */
 ST_API int st_upload_lights(st_ctx *ctx, int slot, const Scene *scene);
-/* uploadSceneBVH (core/init.h:106): the host-built TLAS (scene->bvh) as-is. */
+/* uploadSceneBVH (core/init.h:106): the host-built TLAS (scene->bvh) as-is; at most 2n nodes for n
+ * primitives (ST_ERR_BAD_SCENE). */
 ST_API int st_upload_scene_bvh(st_ctx *ctx, int slot, const Scene *scene);
-/* uploadMeshBVHs (core/init.h:111): every mesh's BLAS nodes and BVH-ordered Triangles as-is. */
+/* uploadMeshBVHs (core/init.h:111): every mesh's BLAS nodes and BVH-ordered Triangles as-is; at most n
+ * pairs of children for a mesh of n triangles (ST_ERR_BAD_SCENE). */
 ST_API int st_upload_mesh_bvhs(st_ctx *ctx, int slot, const Scene *scene);
 /* Primitives whose transform changed since the last upload: primitives[k] replaces primitive
  * ids[k]; the ids must be distinct and below the scene's primitive count (else ST_ERR_INVALID_ARG,
@@ -169,7 +171,8 @@ ST_API int st_build_bvh(st_ctx *ctx, int mode, const float *aabbs, uint32_t n, u
  * st_upload_mesh_bvhs), on the host, with no context: every children pair reached from the root
  * lies inside `nodes[node_count]` and is reached once, every leaf range lies inside `items`, and
  * both `height` and the depth the walk reaches leave room in the 64-entry traversal stacks (depth
- * + 2 <= 64).  ST_OK, ST_ERR_BAD_SCENE, or ST_ERR_INVALID_ARG for a null array.  No reference
+ * + 2 <= 64).  (The uploads also bound node_count, see there.)  ST_OK, ST_ERR_BAD_SCENE, or
+ * ST_ERR_INVALID_ARG for a null array.  No reference
  * counterpart: a host can check a loaded .mesh or .scene BVH before it uploads it. */
 ST_API int st_validate_bvh(const BVHNode *nodes, uint32_t node_count, uint32_t items, uint32_t height);
 

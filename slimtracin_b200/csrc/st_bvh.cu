@@ -402,10 +402,10 @@ __global__ void single_leaf_kernel(const float *aabbs, const u32t *order, u32t n
 
 // ---- small builds: the whole LBVH30 by one block ----------------------------------------------------
 // The same steps as the kernels above, at most kBlockItems items, everything between in shared memory.
-// A small build is
-// launches and their gaps, thirty of them: 173 us for 100 primitives, 218 for 1000, 257 for 4096 as
-// st_update_scene_bvh sees it, against 42, 66 and 148 with one (and tlas_finish_kernel below); above
-// 4096 items the shared arrays no longer fit and many blocks are faster than one.
+// A small build is launches and their gaps, some thirty of them: 142 us for 100 primitives, 192 for 1000,
+// 268 for 4096 as st_update_scene_bvh without host arrays sees it, against 39, 63 and 147 with one (and
+// tlas_finish_kernel below).  The line is where the shared arrays no longer fit: 4097 primitives take 198
+// us by the launches above, 10,000 take 202.
 constexpr u32t kBlockItems = 4096;
 constexpr int kBlockThreads = 1024, kBlockWarps = kBlockThreads / 32;
 struct LbvhShared {

@@ -88,7 +88,8 @@ struct ParkQueue {
     u32t *drained = nullptr;       // the batch's total of parked paths traced by the drain (all groups)
     u32t capacity = 0, threshold = 0;
 };
-constexpr u32t kParkCapacity = 1u << 20;   // parked rays per launch group at most (96 MB)
+constexpr u32t kParkCapacity = 1u << 20;   // parked rays per launch group at most (84 MB)
+static_assert(sizeof(ParkedRay) == 80, "the queue's size above");
 
 int launch_batch(const BatchView *views, u32t n_views, u32t total_tiles, int variant, u32t chunk, u32t grid_blocks,
                  u32t *tile_counter, unsigned *status, unsigned long long *counters, bool count, cudaStream_t st,
@@ -103,7 +104,7 @@ int batch_blocks_per_sm(int variant);
 void launch_frame_setup(const SceneDev &S, const ViewDev &v, int4 *ssb, float *dirs, cudaStream_t st);
 inline size_t ray_rows_floats(const ViewDev &v) { return (size_t)v.grid_h * ((v.grid_w + kSegment - 1) / kSegment) * 3; }
 // Block columns [bx_first, bx_first + bx_count) of the grid (8 grid points wide each; bx_count 0:
-// to the last column).  from_middle: for a launch that runs alone and whose paths do not bounce.
+// to the last column).  from_middle: for a launch that runs alone over a scene without bounces.
 void launch_trace(const SceneDev &S, const ViewDev &v, const int4 *ssb, const float *dirs, FloatPixel *out,
                   u32t *prim_ids, unsigned *status, unsigned long long *counters, bool count, cudaStream_t st,
                   bool from_middle = false, u32t bx_first = 0, u32t bx_count = 0);

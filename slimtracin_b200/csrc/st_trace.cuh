@@ -117,9 +117,8 @@ __device__ __forceinline__ Slabs prepare(v3 org, v3 dir) {
 // 2^28 on an axis the ray does not move along.  That axis is then left out, where the chain also drops a
 // neighbouring one and visits boxes that hold no point of the ray.  `closest` must be a number: the chain
 // admits nothing where it is NaN.  A walk step is bound by its dependent instructions, not by bandwidth:
-// with the planes of a pair multiplied and added two at a time (mul_add2) it takes about 65 instructions
-// against 100; without the pairing the 4096-primitive moving scene traces in 1.08 ms instead of
-// 1.05, the mesh frames in 1 to 2 % more.
+// hence the planes of a pair are multiplied and added two at a time (mul_add2); without the pairing the
+// 4096-primitive moving scene traces in 1.08 ms instead of 1.05, the mesh frames in 1 to 2 % more.
 __device__ __forceinline__ float min3(float a, float b, float c) {
     float r;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -143,9 +142,9 @@ __device__ __forceinline__ bool hit_box_slabs(const float *b, const Slabs &r, fl
                      b[2] * r.rcp.z + r.so.z, b[5] * r.rcp.z + r.so.z, r.rcp, closest, dist);
 }
 // v * m + a on two floats at once, each product and sum rounded by itself.  The product is a fused
-// v * m + -0, the same value, with a -0 that the compiler does not know (SceneDev::neg_zero): a packed
-// multiply and a packed add, both .rn, were contracted into one rounding on the way to machine code,
-// which moved entry distances by an ulp and changed the work of 54 of the 1080p frame's rays.
+// v * m + -0, the same value, with a -0 that the compiler does not know (SceneDev::neg_zero): written as
+// a packed multiply and a packed add, both .rn, the results were those of one rounding, an ulp off in some
+// entry distances, and the work of 54 of the 1080p frame's rays changed.
 __device__ __forceinline__ float2 mul_add2(float2 v, float2 m, float2 a, float nz) {
     float2 r;
     asm("{.reg .b64 v, m, a, z;\n\tmov.b64 v, {%2, %3};\n\tmov.b64 m, {%4, %5};\n\tmov.b64 a, {%6, %7};\n\t"
