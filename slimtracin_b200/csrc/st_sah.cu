@@ -38,8 +38,7 @@ constexpr int kBinWords = 13;          // large ranges: count + box(6) + centroi
 constexpr int kSweepWords = 7;         // in shared memory: count + box(6), [axis][word][bin]
 constexpr int kWarpBins = 3 * kSweepWords * kBins;
 
-// The move is opaque on purpose: written as __float_as_uint the bits of a NaN were not kept, and scenes
-// with NaN positions got other trees than the specification's (65 and 700 primitives, one in eight NaN).
+// The move is opaque on purpose: written as __float_as_uint the bits of a NaN were not kept.
 __device__ __forceinline__ unsigned ob(float f) {
     unsigned u;
     asm("mov.b32 %0, %1;" : "=r"(u) : "f"(f));
